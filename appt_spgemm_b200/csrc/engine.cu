@@ -40,7 +40,7 @@ struct spg_ctx {
   cudaMemPool_t pool = nullptr;
   spg_config cfg{};
   uint32_t* d_status = nullptr;   // device status word (+ scratch, 256 B)
-  int64_t* h_pin = nullptr;       // pinned readback area (512 B)
+  int64_t* h_pin = nullptr;       // pinned readback area (1 KB)
   // profiling: per-kernel events on the launching stream, resolved on read
   bool prof = false;
   std::vector<ProfEntry> pending;
@@ -194,6 +194,7 @@ struct spg_plan {
   // numeric one with tables of 2^small_log2 slots
   bool small = false;
   int small_log2 = 6;
+  int small_sort = 0;  // > 0: sorted rows of up to this many products instead
   int32_t* hqueue = nullptr;  // next row of the CTA-per-row kernels, one counter per bin
                               // (zeroed before each launch; bins may run at once)
   int window_bits = 1 << 20;  // heavy-path shape (heavy_shape)
@@ -581,6 +582,10 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   // row length (several rows per warp), 2048 a warp per row
   int lg = ceil_log2_64((int64_t)sv[2] * 100 / ctx->cfg.num_load_pct + 1);
   p->small_log2 = lg < kMinTableLog2 ? kMinTableLog2 : (lg > 11 ? 11 : lg);
+  // products that hardly merge: sorted rows, sized from the largest row
+  if ((int64_t)sv[0] >= kSortMinProducts * n && sorted_row((int64_t)sv[1], kSortMaxProducts, n) &&
+      2 * (int64_t)sv[0] <= kSortMaxMerge2 * p->nnz_c)
+    p->small_sort = (int)sv[1];
   if (ctx->cfg.lanes_per_row > 0) {
     p->G = ctx->cfg.lanes_per_row;
   } else {
@@ -693,7 +698,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
                  ctx->cfg.sym_load_pct,
                  numeric_heavy_min(num_lg, ctx->cfg.num_load_pct),
                  p->A.rowptr, split, short_lg,
-                 numeric_heavy_min(short_lg, ctx->cfg.num_load_pct), dense_lw};
+                 numeric_heavy_min(short_lg, ctx->cfg.num_load_pct), dense_lw, 0};
   // column blocks of the heavy rows: 1024 columns (windows are packed from
   // the counts; a block above the window cap, 675 columns at the default
   // load, is cut into fixed 512-column windows); wider when that many counts
@@ -793,7 +798,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     ProfScope ps(ctx, "sym/bin", bs, b);
     TRY_CUDA(launch_hash_bin(b, false, gram, r, ctx->num_sms, bs), "symbolic");
   }
-  for (int b = kDenseBin0; b < kNumBins; ++b) {
+  for (int b = kDenseBin0; b < kSortBin0; ++b) {
     if (sym_count[b] == 0) continue;
     RowArgs r = ra;
     r.rows = rows_sym + sym_start[b];
@@ -839,7 +844,8 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   // numeric binning by exact counts, stats; host sync #2 (nnz(C))
   TRY(palloc(p, &p->rows_num, n));
   BinSource bnum{1, n, p->f, p->lo, p->hi, p->rownnz, gram ? p->rowlow : nullptr, num_lg, force,
-                 ctx->cfg.num_load_pct, 0, p->A.rowptr, split, short_lg, 0, dense_lw};
+                 ctx->cfg.num_load_pct, 0, p->A.rowptr, split, short_lg, 0, dense_lw,
+                 gram ? 0 : 1};
   {
     ProfScope ps(ctx, "plan/bin_num", st);
     TRY_CUDA(launch_bin_rows(bnum, hist, counts + 2 * kNumBins, p->rows_num, st),
@@ -973,7 +979,8 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       const int bin = p->small_log2 - kMinTableLog2 + 1;
       r.G = hash_bin_lanes(bin, p->G);
       ProfScope ps(ctx, "num/small", st);
-      cudaError_t e = launch_hash_bin(bin, true, false, r, ctx->num_sms, st);
+      cudaError_t e = p->small_sort ? launch_sort_rows(p->small_sort, r, ctx->num_sms, st)
+                                    : launch_hash_bin(bin, true, false, r, ctx->num_sms, st);
       if (e != cudaSuccess) result = cuda_status(e, "numeric");
     }
     for (int b = 1; b <= kNumTableBins && result == SPG_OK; ++b) {
@@ -988,7 +995,18 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       cudaError_t e = launch_hash_bin(b, true, gram, r, ctx->num_sms, bs);
       if (e != cudaSuccess) result = cuda_status(e, "numeric");
     }
-    for (int b = kDenseBin0; b < kNumBins && result == SPG_OK; ++b) {
+    for (int b = kSortBin0; b < kNumBins && result == SPG_OK; ++b) {
+      if (p->num_count[b] == 0) continue;
+      RowArgs r = ra;
+      r.rows = p->rows_num + p->num_start[b];
+      r.nrows = (int32_t)p->num_count[b];
+      const int most = sort_bin_products(b - kSortBin0);
+      const cudaStream_t bs = fork.next();
+      ProfScope ps(ctx, "num/sort", bs, most);
+      cudaError_t e = launch_sort_rows(most, r, ctx->num_sms, bs);
+      if (e != cudaSuccess) result = cuda_status(e, "numeric");
+    }
+    for (int b = kDenseBin0; b < kSortBin0 && result == SPG_OK; ++b) {
       if (p->num_count[b] == 0) continue;
       RowArgs r = ra;
       r.rows = p->rows_num + p->num_start[b];
@@ -1129,7 +1147,7 @@ spg_status spg_create(spg_ctx** out, const spg_config* cfg) {
     cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &thr);
     if ((e = cudaMalloc(&ctx->d_status, 256)) != cudaSuccess) { st = cuda_status(e, "status"); break; }
     if ((e = cudaMemset(ctx->d_status, 0, 256)) != cudaSuccess) { st = cuda_status(e, "status"); break; }
-    if ((e = cudaMallocHost(&ctx->h_pin, 512)) != cudaSuccess) { st = cuda_status(e, "pinned"); break; }
+    if ((e = cudaMallocHost(&ctx->h_pin, 1024)) != cudaSuccess) { st = cuda_status(e, "pinned"); break; }
     if ((e = cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming)) != cudaSuccess) {
       st = cuda_status(e, "event");
       break;

@@ -37,7 +37,11 @@ constexpr int kHeavyBin = kNumTableBins + 1;  // 12
 constexpr int kDenseMinLog2W = 8;
 constexpr int kDenseMaxLog2W = 11;
 constexpr int kDenseBin0 = kHeavyBin + 1;     // 13
-constexpr int kNumBins = kDenseBin0 + kDenseMaxLog2W - kDenseMinLog2W + 1;  // 17
+// kSortBin0 + b = sorted row (numeric phase only) of up to sort_bin_products(b)
+// products.
+constexpr int kSortBins = 8;
+constexpr int kSortBin0 = kDenseBin0 + kDenseMaxLog2W - kDenseMinLog2W + 1;  // 17
+constexpr int kNumBins = kSortBin0 + kSortBins;                              // 25
 constexpr int kDenseVals = 256;  // entries of a bitmap-path row (numeric)
 
 }  // namespace spg

@@ -1,0 +1,83 @@
+"""GPU parity of the row kernels that the binning picks by structure, at the edges
+of their ranges, bit for bit against the CPU oracle; the kernels that ran are
+read from the engine's per-kernel profile."""
+import numpy as np
+import pytest
+
+import oracle
+from appt_spgemm_b200 import csr
+from parity import assert_same_csr
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module", params=["default", "binned"])
+def eng(request):
+    from appt_spgemm_b200.engine import Engine
+    e = Engine("cuda:0", **({} if request.param == "default" else {"small_max_nnz": -1}))
+    e.binned = request.param == "binned"
+    yield e
+    e.check_device_status()
+    e.close()
+
+
+def product(eng, A, task):
+    """The product twice from one plan (the second re-derives what depends on
+    A's values), compared both times; returns the kernel labels."""
+    from appt_spgemm_b200.engine import CsrDevice
+    eng.profile_enable(True)
+    eng.profile_reset()
+    p = eng.plan(CsrDevice.from_host(A, "cuda:0"), task)
+    ref = oracle.multiply(A, task)
+    for _ in range(2):
+        C = p.execute()
+        torch.cuda.synchronize()
+        assert_same_csr(C.to_host(), ref, task)
+    p.close()
+    labels = set(eng.profile_read()["kernels"])
+    eng.profile_enable(False)
+    eng.check_device_status()
+    return labels
+
+
+def from_rows(n, rows, seed):
+    """CSR of the given column lists (sorted here), values uniform(-1, 1)."""
+    rows = [np.unique(np.asarray(r, dtype=np.int64)) for r in rows]
+    rp = np.zeros(n + 1, dtype=np.int32)
+    rp[1:len(rows) + 1] = np.cumsum([len(r) for r in rows])
+    rp[len(rows) + 1:] = rp[len(rows)]
+    col = np.concatenate(rows).astype(np.int32)
+    return csr.CsrHost(n, rp, col, np.random.default_rng(seed).uniform(-1, 1, len(col)))
+
+
+# rows of exactly d·d products over 20,011 columns: either side of the kernel's
+# smallest row (48), of each row capacity and of the largest (4096)
+@pytest.mark.parametrize("d", [6, 7, 11, 12, 16, 17, 19, 20, 22, 23, 27, 28, 32, 33, 39, 45, 46, 55,
+                               64, 65])
+def test_sorted_rows(eng, d):
+    labels = product(eng, csr.uniform(20011, d, seed=d), "AA")
+    if eng.binned:
+        assert any(x.startswith("num/sort") for x in labels) == (7 <= d <= 64)
+
+
+def test_sorted_rows_uneven(eng):
+    # empty B rows between others, rows of very different lengths, repeated columns
+    rng = np.random.default_rng(5)
+    n = 6007
+    rows = [rng.integers(0, n, rng.choice([0, 0, 1, 2, 30, 70])) for _ in range(n)]
+    for task in ("AA", "AAt", "AAtS"):
+        product(eng, from_rows(n, rows, 6), task)
+
+
+@pytest.mark.parametrize("width", [1, 60, 700])
+def test_sorted_rows_clustered(eng, width):
+    # a row's products fall into a few columns at one end of a wide span, so one
+    # bucket holds them all
+    n = 50021
+    rng = np.random.default_rng(width)
+    rows = [np.concatenate([rng.integers(0, 40, 9), [n - 1 - i % 5]]) for i in range(400)]
+    rows += [[n - 1 - i % 3, i % width] for i in range(400, 3000)]
+    rows[:40] = [np.concatenate([rng.integers(1000, 1000 + width, 12), [n - 3]]) for _ in range(40)]
+    product(eng, from_rows(n, rows, 7), "AA")

@@ -197,6 +197,9 @@ struct spg_plan {
   int small_sort = 0;  // > 0: sorted rows of up to this many products instead
   int32_t* hqueue = nullptr;  // next row of the CTA-per-row kernels, one counter per bin
                               // (zeroed before each launch; bins may run at once)
+  int pan_log2 = 0;           // heavy rows in panels of 2^pan_log2 columns (0: none)
+  int npan = 0;
+  bool pan_table = false;     // their slice bounds are tabulated at each execute
   int window_bits = 1 << 20;  // heavy-path shape (heavy_shape)
   int heavy_threads = 1024;
 };
@@ -687,6 +690,8 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   const int64_t split = ctx->cfg.heavy_split > 0 ? (int64_t)ctx->cfg.heavy_split
                                                  : kHeavySplitDefault;
   const int short_lg = std::min(num_lg, 11);
+  // panels, unless the configuration shapes the heavy path itself
+  const int panels = ctx->cfg.heavy_split == 0 && ctx->cfg.heavy_vcap < 0;
   // bitmap bins (not for the Gram path): the largest bitmap the config allows
   int dense_lw = -1;
   if (!gram && ctx->cfg.dense_max_words >= (1 << kDenseMinLog2W)) {
@@ -698,7 +703,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
                  ctx->cfg.sym_load_pct,
                  numeric_heavy_min(num_lg, ctx->cfg.num_load_pct),
                  p->A.rowptr, split, short_lg,
-                 numeric_heavy_min(short_lg, ctx->cfg.num_load_pct), dense_lw, 0};
+                 numeric_heavy_min(short_lg, ctx->cfg.num_load_pct), dense_lw, 0, panels};
   // column blocks of the heavy rows: 1024 columns (windows are packed from
   // the counts; a block above the window cap, 675 columns at the default
   // load, is cut into fixed 512-column windows); wider when that many counts
@@ -750,17 +755,31 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     sym_count[b] = hp[b];
     sym_start[b] = hp[kNumBins + b];
   }
-  // Σ over heavy rows of ((hi − lo) >> b) + 1 is at most
-  // total_1024 / 2^(b−10) + rows, so the wider blocks need no second readback
+  // A row's blocks of 2^b columns are at most its blocks of 1024 columns times
+  // 2^(10−b), or for b > 10 divided by 2^(b−10) plus two, so other widths need
+  // no second readback
   int64_t total_blocks = hp[2 * kNumBins];
   const int64_t heavy_sym = sym_count[kHeavyBin];
   const int64_t budget = ctx->cfg.heavy_block_budget;
+  // panels of 1024 columns, narrower while they are too few to fill the GPU's
+  // warps twice over
+  if (heavy_sym > 0 && panels) {
+    p->pan_log2 = 10;
+    while (p->pan_log2 > 8 && (total_blocks << 1 >> (p->pan_log2 - 9)) < 4096) --p->pan_log2;
+    while (p->blk_log2 > p->pan_log2) {
+      --p->blk_log2;
+      total_blocks <<= 1;
+    }
+  }
   while (total_blocks > budget && p->blk_log2 < 20 &&
          p->window_bits % (2 << p->blk_log2) == 0) {
     ++p->blk_log2;
-    total_blocks = (hp[2 * kNumBins] >> (p->blk_log2 - 10)) + heavy_sym;
+    total_blocks = p->blk_log2 <= 10 ? hp[2 * kNumBins] << (10 - p->blk_log2)
+                                     : (hp[2 * kNumBins] >> (p->blk_log2 - 10)) + 2 * heavy_sym;
   }
-  if (p->blk_log2 > 10) {
+  if (p->pan_log2 > 0 && p->blk_log2 > p->pan_log2)
+    p->pan_log2 = p->blk_log2 <= 12 ? p->blk_log2 : 0;
+  if (p->blk_log2 != 10) {
     ProfScope ps(ctx, "plan/heavy_blocks", st);
     TRY_CUDA(launch_heavy_blocks(bsym, p->blk_log2, nblk, p->blk_off, btmp, st), "heavy blocks");
   }
@@ -845,7 +864,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   TRY(palloc(p, &p->rows_num, n));
   BinSource bnum{1, n, p->f, p->lo, p->hi, p->rownnz, gram ? p->rowlow : nullptr, num_lg, force,
                  ctx->cfg.num_load_pct, 0, p->A.rowptr, split, short_lg, 0, dense_lw,
-                 gram ? 0 : 1};
+                 gram ? 0 : 1, panels};
   {
     ProfScope ps(ctx, "plan/bin_num", st);
     TRY_CUDA(launch_bin_rows(bnum, hist, counts + 2 * kNumBins, p->rows_num, st),
@@ -886,8 +905,16 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   p->info.bins_used = bins_used;
   p->info.output_bytes = 8 * ((int64_t)n + 1) + 12 * p->nnz_c;
   p->info.workspace_bytes = p->ws_bytes;
-  p->info.exec_workspace_bytes = exec_workspace(n, gram, p->nnz_low) +
-                                 (p->heavy_windows ? 16 * Ad->nnz : 0);
+  // the panels' slice bounds (an int per row of B and panel) may take an eighth
+  // of C's size; beyond that the panels search for them
+  if (p->heavy_windows && p->pan_log2 > 0) {
+    p->npan = ((n - 1) >> p->pan_log2) + 1;
+    p->pan_table = 4 * (int64_t)n * (p->npan + 1) <=
+                   std::max<int64_t>((int64_t)64 << 20, p->info.output_bytes / 8);
+  }
+  p->info.exec_workspace_bytes =
+      exec_workspace(n, gram, p->nnz_low) + (p->heavy_windows ? 16 * Ad->nnz : 0) +
+      (p->npan > 0 ? panel_workspace(n, p->npan, p->num_count[kHeavyBin], p->pan_table) : 0);
   return SPG_OK;
 }
 
@@ -968,9 +995,14 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       if ((result = talloc(&hc, sizeof(int4) * (size_t)p->A.nnz)) != SPG_OK) break;
       hcur = (int4*)hc;
     }
+    void* panel_ws = nullptr;
+    if (p->npan > 0 &&
+        (result = talloc(&panel_ws, (size_t)panel_workspace(n, p->npan, p->num_count[kHeavyBin],
+                                                            p->pan_table))) != SPG_OK)
+      break;
     int launches = p->small && n > 0 ? 1 : 0;
     for (int b = 1; b < kNumBins; ++b)
-      if (p->num_count[b] > 0) launches += b == kHeavyBin && p->heavy_windows ? 2 : 1;
+      if (p->num_count[b] > 0) launches += b == kHeavyBin && p->heavy_windows ? 3 : 1;
     BinFork fork(ctx, st, launches);
     if (p->small && n > 0) {
       RowArgs r = ra;
@@ -1047,8 +1079,15 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       const int win_threads = ctx->cfg.heavy_threads > 512 ? 1024 : 512;
       h.vcap = ctx->cfg.heavy_vcap > 0 ? (int32_t)ctx->cfg.heavy_vcap : 8192;
       h.wcap_bits = win_threads > 512 ? (1 << 18) : (1 << 17);
+      h.pan_log2 = p->pan_log2;
+      h.npan = p->npan;
       cudaError_t e = cudaSuccess;
-      if (windows) {
+      if (p->npan > 0) {
+        const cudaStream_t bs = fork.next();
+        ProfScope ps(ctx, "num/panels", bs);
+        e = launch_panels(gram, h, panel_ws, p->pan_table, ctx->num_sms, bs);
+      }
+      if (e == cudaSuccess && windows) {
         const cudaStream_t bs = fork.next();
         ProfScope ps(ctx, "num/heavy_w32", bs);
         e = launch_heavy_w32(gram, h, ctx->num_sms, bs);

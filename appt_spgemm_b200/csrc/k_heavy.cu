@@ -108,7 +108,9 @@ __global__ void __launch_bounds__(1024, 2) k_heavy_sym(HeavyArgs h) {
     const int row = a.rows[r];
     const int lo = h.lo[row], hi = h.hi[row];
     long long c = 0, cl = 0;
-    for (long long w0 = lo; w0 <= hi; w0 += h.window_bits) {
+    // windows start on a column block's first column
+    const int lo_blk = lo >> h.blk_log2 << h.blk_log2;
+    for (long long w0 = lo_blk; w0 <= hi; w0 += h.window_bits) {
       const int nwords = (int)min((long long)nw_max, (hi - w0) / 32 + 1);
       for (int i = threadIdx.x; i < nwords; i += blockDim.x) bm[i] = 0u;
       __syncthreads();
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(1024, 2) k_heavy_sym(HeavyArgs h) {
       int lc = 0, lcl = 0;
       const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
       const int wpb = 1 << (h.blk_log2 - 5);
-      const long long blk0 = (w0 - lo) >> h.blk_log2;
+      const long long blk0 = (w0 - lo_blk) >> h.blk_log2;
       for (int blk = wid; blk * wpb < nwords; blk += nwarps) {
         int bc = 0;
         for (int i = blk * wpb + lane; i < min((blk + 1) * wpb, nwords); i += 32) {
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num(HeavyArgs h) {
     const int lo = GRAM ? max(h.lo[row], row) : h.lo[row];
     const int32_t low = GRAM ? a.low_in[row] : 0;
     const long long expect = (long long)a.cnt_in[row] - low;
-    if (heavy_row_windowed(h, row)) continue;  // the windowed warp kernel's row
+    if (heavy_row_paneled(h, row) || heavy_row_windowed(h, row)) continue;  // another kernel's row
     const int64_t base = a.rowptr[row] + low;
     const int cb = a.colbase ? a.colbase[row] : 0;
     long long written = 0;
@@ -344,7 +346,7 @@ __global__ void k_heavy_blocks(BinSource bsym, int blk_log2, int32_t* __restrict
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < bsym.n;
        i += (int64_t)gridDim.x * blockDim.x)
     nblk[i] = row_bin(bsym, (int)i) == kHeavyBin
-                  ? (int32_t)((((int64_t)bsym.hi[i] - bsym.lo[i]) >> blk_log2) + 1)
+                  ? (bsym.hi[i] >> blk_log2) - (bsym.lo[i] >> blk_log2) + 1
                   : 0;
 }
 

@@ -207,9 +207,10 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
       const int64_t b0 = h.blk_off[row];
       const int nb = (int)(h.blk_off[row + 1] - b0);
       const uint16_t* cnt = h.blk_cnt + b0;
-      int b = (lo_r - lo) >> h.blk_log2;
+      int b = (lo_r >> h.blk_log2) - (lo >> h.blk_log2);
+      const int lo_blk = lo >> h.blk_log2 << h.blk_log2;
       while (b < nb) {
-        const int bstart = lo + (b << h.blk_log2);
+        const int bstart = lo_blk + (b << h.blk_log2);
         if ((int)cnt[b] > h.cap) {
           // a dense block: fixed windows of sw columns
           const int bend = (int)min((int64_t)bstart + bw, (int64_t)hi + 1);
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
         } else {
           const int e = window_end(cnt, b, nb, h.cap, max_blocks);
           const int c0 = max(bstart, lo_r);
-          const int c1 = (int)min((int64_t)lo + ((int64_t)e << h.blk_log2), (int64_t)hi + 1);
+          const int c1 = (int)min((int64_t)lo_blk + ((int64_t)e << h.blk_log2), (int64_t)hi + 1);
           written += heavy_window<LOG2T, GRAM>(h, row, ps, pe, c0, c1, keys, vals, base + written,
                                                expect - written);
           b = e;

@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
     const int r = cta_item(h.queue, a.nrows, it, &s_next);
     if (r >= a.nrows) break;
     const int row = a.rows[r];
-    if (heavy_row_windowed(h, row)) continue;  // the windowed warp kernel's row
+    if (heavy_row_paneled(h, row) || heavy_row_windowed(h, row)) continue;  // the windowed warp kernel's row
     const int lo = h.lo[row], hi = h.hi[row];
     const int lo_r = GRAM ? max(lo, row) : lo;
     const int32_t low = GRAM ? a.low_in[row] : 0;
@@ -111,7 +111,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
       const int nb = (int)(h.blk_off[row + 1] - b0);
       const uint16_t* cnt = h.blk_cnt + b0;
       // window walk state (thread 0): next block, next column inside a cut block
-      int wb = (int)(((long long)lo_r - lo) >> bw_log2);
+      int wb = (lo_r >> bw_log2) - (lo >> bw_log2);
+      const int lo_blk = lo >> bw_log2 << bw_log2;
       long long wsub = -1;
       for (;;) {
         __syncthreads();  // cursors written; the previous window is finished
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
           int c0 = 0, c1 = 0;
           bool done = wb >= nb;
           if (!done) {
-            const long long bstart = (long long)lo + ((long long)wb << bw_log2);
+            const long long bstart = (long long)lo_blk + ((long long)wb << bw_log2);
             const long long bend = min(bstart + bwidth, (long long)hi + 1);
             if ((int)cnt[wb] > vcap || bwidth > wcap) {
               const long long s0 = wsub >= 0 ? wsub : max(bstart, (long long)lo_r);
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
                 ++e;
               }
               c0 = (int)max(bstart, (long long)lo_r);
-              c1 = (int)min((long long)lo + ((long long)e << bw_log2), (long long)hi + 1);
+              c1 = (int)min((long long)lo_blk + ((long long)e << bw_log2), (long long)hi + 1);
               wb = e;
             }
           }

@@ -33,6 +33,22 @@ constexpr int64_t kSortMinProducts = 48;
 constexpr int64_t kSortMaxProducts = 4096;
 constexpr int64_t kSortMaxMerge2 = 3;
 
+// Paneled rows: the fewest products, the narrowest span, the fewest products per
+// 1024 columns of it and, up to kWarpRowMaxProducts products, the fewest per
+// entry of A's row there (a slice of a B row) for rows within and beyond the
+// sorted rows' range.  Measured per call, 48-matrix batch (Erdős–Rényi rows of
+// 1,000 products, slices of 2 to 4) / R-MAT 2^16 / 2^13: slices of 2 for all
+// rows 10.70 / 5.97 / 0.88 ms, of 5 for all 8.63 / 6.56 / 0.88, as below
+// 8.62 / 5.97 / 0.88; tables and sorted rows up to 5,400 entries as before the
+// panels 8.58 / 6.51 / 1.62.
+constexpr int64_t kPanelMinRow = 256;
+constexpr int32_t kPanelMinSpan = 600;
+constexpr int64_t kPanelMinProducts = 64;
+constexpr int64_t kPanelMinSliceSmall = 5;
+constexpr int64_t kPanelMinSlice = 2;
+// one warp walks a windowed heavy row alone: a larger row would set its tail
+constexpr int64_t kWarpRowMaxProducts = (int64_t)1 << 17;
+
 // What a row's bin is computed from.
 struct BinSource {
   int mode;                 // 0: symbolic (from products and span), 1: numeric (from counts)
@@ -66,6 +82,8 @@ struct BinSource {
   // numeric, not Gram: rows of up to kSortMaxProducts products of which few
   // merge take the sorted-row kernels
   int sort_rows;
+  // rows for the panel kernel go heavy whatever their table (0: no such rule)
+  int panels;
 };
 
 __host__ __device__ __forceinline__ int ceil_log2_64(int64_t x) {
@@ -88,6 +106,18 @@ __host__ __device__ __forceinline__ bool sorted_row(int64_t f, int64_t m, int64_
          span <= ((int64_t)1 << (32 - ceil_log2_64(f < 128 ? 128 : f)));
 }
 
+// A row of f products from `len` entries of A over columns [lo, hi]: cut into
+// panels?  By its products and span alone, so that the symbolic and the numeric
+// binning agree.
+__host__ __device__ __forceinline__ bool paneled_row(int64_t f, int32_t len, int32_t lo,
+                                                     int32_t hi) {
+  if (f < kPanelMinRow || hi - lo < kPanelMinSpan) return false;
+  const int64_t panels = (hi >> 10) - (lo >> 10) + 1;
+  return f >= kPanelMinProducts * panels &&
+         (f > kWarpRowMaxProducts ||
+          f >= (f > kSortMaxProducts ? kPanelMinSlice : kPanelMinSliceSmall) * panels * len);
+}
+
 // Table size rule: symbolic tables hold keys only and are sized for the load
 // limit (default 75%) of min(products, span); numeric tables hold key+value
 // and are sized for the load limit (default 66%) of the exact row count.
@@ -105,7 +135,7 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
     size = m;
   }
   const int64_t want = size * 100 / s.load_pct + 1;
-  if (s.force_heavy) return kHeavyBin;
+  if (s.force_heavy || (s.panels && paneled_row(s.f[i], s.arowptr[i + 1] - s.arowptr[i], s.lo[i], s.hi[i]))) return kHeavyBin;
   if (s.mode == 1 && s.sort_rows && want <= ((int64_t)1 << s.max_log2) &&
       sorted_row(s.f[i], size, (int64_t)s.hi[i] - s.lo[i] + 1)) {
     int b = 0;
@@ -260,9 +290,9 @@ struct HeavyArgs {
   const int32_t* lo;        // output column span per row
   const int32_t* hi;
   int32_t window_bits;      // W (multiple of 32 * threads)
-  // column blocks: heavy row i's span [lo, hi] is cut into blocks of
-  // 2^blk_log2 columns from lo; blk_cnt[blk_off[i] + b] is the number of
-  // distinct output columns in block b (saturated at 65535), written by the
+  // column blocks: heavy row i's span [lo, hi] is cut at multiples of
+  // 2^blk_log2 columns; blk_cnt[blk_off[i] + b] is the number of distinct output
+  // columns in its b-th block (saturated at 65535), written by the
   // symbolic kernel when blk_cnt is set and read by the windowed numeric one
   const int64_t* blk_off;   // per row (n + 1), 0 blocks for rows not heavy
   uint16_t* blk_cnt;
@@ -282,13 +312,23 @@ struct HeavyArgs {
   // next row from this counter (launch_heavy zeroes it on the stream first),
   // so a CTA that drew hub rows does not hold the others back; required
   int32_t* queue;
+  // panel kernel (k_panel.cu): panels of 2^pan_log2 columns, npan of them over
+  // n columns; slice bounds (nullptr: searched for) and task counter set by
+  // launch_panels (npan 0: no row takes it)
+  int32_t pan_log2, npan;
+  const int32_t* ptr;
+  int64_t* task_queue;
 };
 
+__device__ __forceinline__ bool heavy_row_paneled(const HeavyArgs& h, int row) {
+  return h.npan > 0 && paneled_row(h.f[row], h.r.A.rowptr[row + 1] - h.r.A.rowptr[row],
+                                   h.lo[row], h.hi[row]);
+}
+
 // The heavy row goes to the windowed warp kernel: mean B-row length
-// f / nnz(A row) below split, and at most kWarpRowMaxProducts products (one
-// warp walks its row alone: a larger row would set the kernel's tail).
-constexpr int64_t kWarpRowMaxProducts = (int64_t)1 << 17;
+// f / nnz(A row) below split, and at most kWarpRowMaxProducts products.
 __device__ __forceinline__ bool heavy_row_windowed(const HeavyArgs& h, int row) {
+  if (heavy_row_paneled(h, row)) return false;
   if (h.split <= 0 || h.f[row] > kWarpRowMaxProducts) return false;
   const int64_t len = (int64_t)h.r.A.rowptr[row + 1] - h.r.A.rowptr[row];
   return h.f[row] < h.split * len;
@@ -311,6 +351,13 @@ size_t heavy_win_smem_bytes(int threads, int vcap, int wcap_bits);
 // Windowed numeric phase of heavy rows (k_heavy_w32.cu): a warp per row walks
 // the row's column blocks in windows of at most `cap` distinct columns.
 cudaError_t launch_heavy_w32(bool gram, const HeavyArgs& a, int num_sms, cudaStream_t s);
+// Numeric phase of the rows cut into panels (k_panel.cu), in `workspace` of
+// panel_workspace bytes (with or without the table of slice bounds); sets h.ptr
+// and h.task_queue.
+__host__ __device__ constexpr size_t panel_warp_bytes(int pan_log2) { return ((size_t)8 << pan_log2) + 512; }
+int64_t panel_workspace(int64_t n, int npan, int64_t nrows, bool table);
+cudaError_t launch_panels(bool gram, HeavyArgs& h, void* workspace, bool table, int num_sms,
+                          cudaStream_t s);
 constexpr int kHeavyTableLog2 = 10;  // its shared table: 1024 slots per warp
 
 // ---- transpose and segment sort (k_transpose.cu) ----------------------------

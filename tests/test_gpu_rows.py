@@ -81,3 +81,56 @@ def test_sorted_rows_clustered(eng, width):
     rows += [[n - 1 - i % 3, i % width] for i in range(400, 3000)]
     rows[:40] = [np.concatenate([rng.integers(1000, 1000 + width, 12), [n - 3]]) for _ in range(40)]
     product(eng, from_rows(n, rows, 7), "AA")
+
+
+def hub_rows(n, hubs, width, seed):
+    """`hubs` rows of `width` random columns each, the first of them 3·width, among
+    rows of 8 and empty rows; columns skewed to the low end."""
+    rng = np.random.default_rng(seed)
+    rows = []
+    for i in range(n):
+        if i % (n // hubs) == 1:
+            k = 3 * width if i == 1 else width
+        else:
+            k = 0 if i % 7 == 3 else 8
+        rows.append((n * rng.random(k) ** 2).astype(np.int64))
+    return from_rows(n, rows, seed)
+
+
+# spans below one panel, of a panel and a bit, ragged and many; panels of 256,
+# 512 and 1024 columns (few or many tasks)
+@pytest.mark.parametrize("n,hubs,width", [(601, 30, 90), (1025, 40, 200), (3001, 60, 300),
+                                          (16411, 300, 400)])
+@pytest.mark.parametrize("task", ["AA", "AAt", "AAtS"])
+def test_paneled_rows(eng, n, hubs, width, task):
+    labels = product(eng, hub_rows(n, hubs, width, seed=n), task)
+    assert "num/panels" in labels
+
+
+def test_paneled_rows_signed_zeros():
+    # products of −0.0, cancelled sums and underflow stay entries, with the
+    # oracle's signs; every row through panels that search for their slices or
+    # read them from the table
+    from appt_spgemm_b200.engine import Engine
+    A = hub_rows(2003, 50, 200, seed=9)
+    rng = np.random.default_rng(10)
+    A.val = rng.choice([0.0, -0.0, 1.0, -1.0, 1e-200, -1e-200], A.nnz)
+    with Engine("cuda:0", small_max_nnz=-1, force_heavy=1) as e:
+        e.binned = True
+        for task in ("AA", "AAt", "AAtS"):
+            assert "num/panels" in product(e, A, task)
+
+
+def test_paneled_rows_without_table():
+    # many columns and a small C: the slice bounds would take more memory than
+    # they may, so the panels search for them
+    from appt_spgemm_b200.engine import Engine
+    n, hubs = 262144, 280
+    rng = np.random.default_rng(11)
+    ids = rng.choice(n, hubs, replace=False)
+    rows = [[i] for i in range(n)]
+    for i in ids:
+        rows[i] = np.concatenate([ids, rng.integers(0, n, 240)])
+    with Engine("cuda:0", small_max_nnz=-1) as e:
+        e.binned = True
+        assert "num/panels" in product(e, from_rows(n, rows, 12), "AA")

@@ -193,6 +193,7 @@ struct spg_plan {
   // one-readback plan: every row in one warp-per-row launch per phase, the
   // numeric one with tables of 2^small_log2 slots
   bool small = false;
+  uint16_t* runlen = nullptr;  // runs of shifted rows (nullptr: none looked for)
   int small_log2 = 6;
   int small_sort = 0;  // > 0: sorted rows of up to this many products instead
   int32_t* hqueue = nullptr;  // next row of the CTA-per-row kernels, one counter per bin
@@ -423,6 +424,7 @@ int64_t plan_workspace_bound(const spg_config& cfg, spg_task task, int64_t n, in
          + scan + 4 * nz + 8 * nz + 4 * nn + 4;   // scan, staging copy, long list
   }
   b += 8 * nn + 4 * nn + 4 * nn + 4;                              // f, lo, hi, queue
+  b += 16 * nn + 8 * prepass_pieces(nz) + 8 + 7 * nn;                             // pre-pass, runs
   b += 4 * kNumBins * (nblocks > 0 ? nblocks : 1) + 8 * 4 * kNumBins + 4 * nn;  // binning
   b += 4 * nn + 8 * (nn + 1) + scan;                              // heavy block offsets
   const int64_t per_row_blocks = (nn + 1023) / 1024 + 1;
@@ -637,7 +639,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   p->symmetric = p->task != SPG_TASK_AA;  // until the check says otherwise
   p->B = p->task == SPG_TASK_AA ? p->A : MatView{n, Ad->nnz, Ad->rowptr, Ad->col, bx};
   auto build_transpose = [&]() -> spg_status {
-    int32_t *bp, *bi;
+    int32_t *bp = nullptr, *bi = nullptr;
     TRY(palloc(p, &bp, (int64_t)n + 1));
     TRY(palloc(p, &bi, Ad->nnz));
     TransposeWork w{};
@@ -699,11 +701,30 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     while (dense_lw < kDenseMaxLog2W && ((int64_t)2 << dense_lw) <= ctx->cfg.dense_max_words)
       ++dense_lw;
   }
+  // runs of shifted rows (not for the Gram path, nor where every row is forced
+  // onto the heavy path)
+  const bool runs = !gram && !force && n > 0;
+  PrepassArrays pre{};
+  pre.f = p->f;
+  pre.lo = p->lo;
+  pre.hi = p->hi;
+  TRY(palloc(p, &pre.info, n));
+  TRY(palloc(p, &pre.pieces, prepass_pieces(Ad->nnz)));
+  TRY(palloc(p, &pre.marks, 2));
+  TRY(palloc(p, &pre.flag_a, n));
+  TRY(palloc(p, &pre.need, n));
+  if (runs) {
+    if (p->task != SPG_TASK_AA) TRY(palloc(p, &pre.flag_b, n));
+    TRY(palloc(p, &pre.lead, n));
+    TRY(palloc(p, &pre.runlen, n));
+    p->runlen = pre.runlen;
+  }
   BinSource bsym{0, n, p->f, p->lo, p->hi, nullptr, nullptr, kMaxTableLog2, force,
                  ctx->cfg.sym_load_pct,
                  numeric_heavy_min(num_lg, ctx->cfg.num_load_pct),
                  p->A.rowptr, split, short_lg,
-                 numeric_heavy_min(short_lg, ctx->cfg.num_load_pct), dense_lw, 0, panels};
+                 numeric_heavy_min(short_lg, ctx->cfg.num_load_pct), dense_lw, 0, panels,
+                 pre.lead, pre.runlen, pre.need};
   // column blocks of the heavy rows: 1024 columns (windows are packed from
   // the counts; a block above the window cap, 675 columns at the default
   // load, is cut into fixed 512-column windows); wider when that many counts
@@ -719,9 +740,9 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   // pre-pass, binning and block offsets over the current B, then one readback
   // of the bin sizes, the heavy blocks' total and the two status words
   auto bin_pass = [&]() -> spg_status {
-    {  // the pre-pass also validates A (the verdict comes back below)
+    {  // A is validated in the same reads (the verdict comes back below)
       ProfScope ps(ctx, "plan/prepass", st);
-      TRY_CUDA(launch_prepass(p->A, p->B, p->f, p->lo, p->hi, st, ctx->d_status), "prepass");
+      TRY_CUDA(launch_prepass_rows(p->A, p->B, pre, ctx->num_sms, ctx->d_status, st), "prepass");
     }
     {
       ProfScope ps(ctx, "plan/bin_sym", st);
@@ -845,6 +866,11 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   }
   TRY_CUDA(fork.join(), "join");
 
+  if (runs) {
+    ProfScope ps(ctx, "plan/run_counts", st);
+    TRY_CUDA(launch_run_counts(pre.lead, n, p->rownnz, st), "run counts");
+  }
+
   // C row pointers (and lower-part offsets of the Gram mirror)
   void* scan_tmp;
   TRY(palloc(p, (char**)&scan_tmp, (int64_t)scan_tmp_bytes(n)));
@@ -864,7 +890,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   TRY(palloc(p, &p->rows_num, n));
   BinSource bnum{1, n, p->f, p->lo, p->hi, p->rownnz, gram ? p->rowlow : nullptr, num_lg, force,
                  ctx->cfg.num_load_pct, 0, p->A.rowptr, split, short_lg, 0, dense_lw,
-                 gram ? 0 : 1, panels};
+                 gram ? 0 : 1, panels, pre.lead, pre.runlen, pre.need};
   {
     ProfScope ps(ctx, "plan/bin_num", st);
     TRY_CUDA(launch_bin_rows(bnum, hist, counts + 2 * kNumBins, p->rows_num, st),
@@ -1027,7 +1053,18 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       cudaError_t e = launch_hash_bin(b, true, gram, r, ctx->num_sms, bs);
       if (e != cudaSuccess) result = cuda_status(e, "numeric");
     }
-    for (int b = kSortBin0; b < kNumBins && result == SPG_OK; ++b) {
+    ra.runlen = p->runlen;
+    for (int b = kRunBin0; b < kNumBins && result == SPG_OK; ++b) {
+      if (p->num_count[b] == 0) continue;
+      RowArgs r = ra;
+      r.rows = p->rows_num + p->num_start[b];
+      r.nrows = (int32_t)p->num_count[b];
+      const cudaStream_t bs = fork.next();
+      ProfScope ps(ctx, "num/runs", bs, 1 << (b - kRunBin0));
+      cudaError_t e = launch_runs(b - kRunBin0, r, ctx->num_sms, bs);
+      if (e != cudaSuccess) result = cuda_status(e, "numeric");
+    }
+    for (int b = kSortBin0; b < kRunBin0 && result == SPG_OK; ++b) {
       if (p->num_count[b] == 0) continue;
       RowArgs r = ra;
       r.rows = p->rows_num + p->num_start[b];

@@ -41,7 +41,11 @@ constexpr int kDenseBin0 = kHeavyBin + 1;     // 13
 // products.
 constexpr int kSortBins = 8;
 constexpr int kSortBin0 = kDenseBin0 + kDenseMaxLog2W - kDenseMinLog2W + 1;  // 17
-constexpr int kNumBins = kSortBin0 + kSortBins;                              // 25
+// kRunBin0 + t = first row of a run of shifted rows (numeric phase only), teams
+// of 2^t warps.
+constexpr int kRunBins = 4;
+constexpr int kRunBin0 = kSortBin0 + kSortBins;  // 25
+constexpr int kNumBins = kRunBin0 + kRunBins;    // 29
 constexpr int kDenseVals = 256;  // entries of a bitmap-path row (numeric)
 
 }  // namespace spg

@@ -42,6 +42,7 @@ constexpr int64_t kSortMaxMerge2 = 3;
 // 8.62 / 5.97 / 0.88; tables and sorted rows up to 5,400 entries as before the
 // panels 8.58 / 6.51 / 1.62.
 constexpr int64_t kPanelMinRow = 256;
+constexpr int64_t kPanelMinWideRow = 800;  // over three panels or more: a 27-point row stays hashed
 constexpr int32_t kPanelMinSpan = 600;
 constexpr int64_t kPanelMinProducts = 64;
 constexpr int64_t kPanelMinSliceSmall = 5;
@@ -84,7 +85,27 @@ struct BinSource {
   int sort_rows;
   // rows for the panel kernel go heavy whatever their table (0: no such rule)
   int panels;
+  // runs of shifted rows (nullptr: none): rows back to the run's first row, and
+  // at that row the run's length and the doubles 32 of its rows need
+  const uint8_t* lead;
+  const uint16_t* runlen;
+  const uint16_t* need;
 };
+
+// Runs: the fewest rows, and the limits of a row (products, columns spanned) and
+// of its operands for 32 rows (doubles), split over the teams of a CTA.
+constexpr int kRunMinRows = 8;
+constexpr int kRunMaxProducts = 768;
+constexpr int kRunMaxSpan = 1 << 18;
+constexpr int kRunBuffer = 9216;
+
+// Team size (log2 warps) of a run whose rows have m entries: a warp per 16
+// entries, and a share of the buffer that holds the operands.
+__host__ __device__ __forceinline__ int run_team(int64_t m, int need) {
+  int t = m <= 16 ? 0 : m <= 32 ? 1 : m <= 64 ? 2 : 3;
+  while (t < 3 && need > (kRunBuffer >> (3 - t))) ++t;
+  return t;
+}
 
 __host__ __device__ __forceinline__ int ceil_log2_64(int64_t x) {
   int l = 0;
@@ -113,6 +134,7 @@ __host__ __device__ __forceinline__ bool paneled_row(int64_t f, int32_t len, int
                                                      int32_t hi) {
   if (f < kPanelMinRow || hi - lo < kPanelMinSpan) return false;
   const int64_t panels = (hi >> 10) - (lo >> 10) + 1;
+  if (panels > 2 && f < kPanelMinWideRow) return false;
   return f >= kPanelMinProducts * panels &&
          (f > kWarpRowMaxProducts ||
           f >= (f > kSortMaxProducts ? kPanelMinSlice : kPanelMinSliceSmall) * panels * len);
@@ -124,6 +146,7 @@ __host__ __device__ __forceinline__ bool paneled_row(int64_t f, int32_t len, int
 // Bin b in 1..kNumTableBins means 2^(b+kMinTableLog2−1) slots.
 __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
   int64_t size;
+  if (s.lead && s.lead[i]) return kEmptyBin;  // its run's first row stands for it
   if (s.mode == 0) {
     int64_t f = s.f[i];
     if (f <= 0) return kEmptyBin;
@@ -134,6 +157,7 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
     if (m <= 0) return kEmptyBin;
     size = m;
   }
+  if (s.mode == 1 && s.lead && s.runlen[i]) return kRunBin0 + run_team(size, s.need[i]);
   const int64_t want = size * 100 / s.load_pct + 1;
   if (s.force_heavy || (s.panels && paneled_row(s.f[i], s.arowptr[i + 1] - s.arowptr[i], s.lo[i], s.hi[i]))) return kHeavyBin;
   if (s.mode == 1 && s.sort_rows && want <= ((int64_t)1 << s.max_log2) &&
@@ -221,6 +245,7 @@ struct RowArgs {
   // DEV_ERR_SMALL_CAP; nullptr: every row is processed
   const int64_t* fsmall;
   int64_t fcap;
+  const uint16_t* runlen;   // runs of shifted rows: rows of the run that starts here
 };
 
 // Writes m sorted packed words ((col − lo) << LOG2T | slot) as a row's columns
@@ -280,6 +305,26 @@ cudaError_t launch_hash_bin(int bin, bool numeric, bool gram, const RowArgs& a, 
 cudaError_t launch_dense_bin(int bin, bool numeric, const RowArgs& a, int num_sms,
                              cudaStream_t s);
 int hash_bin_lanes(int bin, int lanes_cfg);
+// The pre-pass of the regular plans (k_runs.cu): products and column span per
+// row, the validation of A and, with `lead`, the runs of shifted rows.  Per row
+// of B: info; per row of A: the others; marks: two ints; pieces:
+// prepass_pieces(nnz).
+// (rows of more than 256 entries, in pieces of 1024: at most 1.25 nnz / 256)
+constexpr int64_t prepass_pieces(int64_t nnz) { return nnz / 200 + 1; }
+struct PrepassArrays {
+  int4* info;
+  int64_t* f;
+  int32_t *lo, *hi, *marks;
+  int2* pieces;
+  uint8_t *flag_a, *flag_b, *lead;
+  uint16_t *need, *runlen;
+};
+cudaError_t launch_prepass_rows(const MatView& A, const MatView& B, const PrepassArrays& w,
+                                int num_sms, uint32_t* status, cudaStream_t s);
+// Runs of shifted rows: their counts after the symbolic phase, and the numeric
+// phase of the runs whose first rows are listed (teams of 2^team warps).
+cudaError_t launch_run_counts(const uint8_t* lead, int32_t n, int32_t* rownnz, cudaStream_t s);
+cudaError_t launch_runs(int team, const RowArgs& a, int num_sms, cudaStream_t s);
 // Sorted rows of up to max_products <= kSortMaxProducts products each, numeric
 // phase (k_sort_rows.cu; not Gram).
 cudaError_t launch_sort_rows(int max_products, const RowArgs& a, int num_sms, cudaStream_t s);

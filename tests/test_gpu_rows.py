@@ -134,3 +134,49 @@ def test_paneled_rows_without_table():
     with Engine("cuda:0", small_max_nnz=-1) as e:
         e.binned = True
         assert "num/panels" in product(e, from_rows(n, rows, 12), "AA")
+
+
+def by_offsets(n, offsets, seed):
+    """Row i holds the columns i + o that lie in the matrix: runs of shifted rows."""
+    return from_rows(n, [[i + o for o in offsets if 0 <= i + o < n] for i in range(n)], seed)
+
+
+# whether runs are taken: enough rows (8), products (768) and room for the rows of
+# B, which lie side by side or not; runs are cut at 256 rows
+@pytest.mark.parametrize("n,offsets,taken", [
+    (7, [0], False), (9, [0], True), (300, [0], True), (261, [-1, 0, 1], True),
+    (1000, [-30, -1, 0, 1, 30], True), (1500, list(range(-13, 14)), True),
+    (1501, list(range(-13, 15)), False), (700, list(range(-60, 60, 5)), False),
+    (2600, [-700, -3, 0, 1, 2, 50, 51, 900], True), (70001, [-30000, -1, 0, 1, 33000], True)])
+@pytest.mark.parametrize("task", ["AA", "AAt"])
+def test_shifted_rows(n, offsets, taken, task):
+    from appt_spgemm_b200.engine import Engine
+    with Engine("cuda:0", small_max_nnz=-1) as e:
+        e.binned = True
+        labels = product(e, by_offsets(n, offsets, seed=n), task)
+        assert any(x.startswith("num/runs") for x in labels) == taken
+
+
+@pytest.mark.parametrize("side", [8, 9, 21, 34, 45])
+def test_shifted_rows_stencil(eng, side):
+    product(eng, csr.stencil27(side, seed=side), "AAt")
+    product(eng, csr.laplace2d(side * side // 3), "AA")
+
+
+def test_shifted_rows_interrupted(eng):
+    # single entries dropped, added and moved break the runs; consecutive instances
+    # of a batch must not be taken for one run's columns
+    rng = np.random.default_rng(13)
+    rows = [[i + o for o in (-90, -1, 0, 1, 2, 90) if 0 <= i + o < 3000] for i in range(3000)]
+    for i in rng.integers(0, 3000, 40):
+        rows[i] = rows[i][1:] if i % 2 else rows[i] + [int(rng.integers(0, 3000))]
+    A = from_rows(3000, rows, 14)
+    product(eng, A, "AA")
+    product(eng, A, "AAt")
+    from appt_spgemm_b200.engine import CsrDevice
+    As = [by_offsets(n, [-1, 0, 1], n) for n in (40, 41, 300, 7)] + [csr.stencil27(9, seed=2)]
+    R = eng.multiply_batched([CsrDevice.from_host(M, "cuda:0") for M in As], "AA")
+    for b, M in enumerate(As):
+        rp, col, val = R.instance(b)
+        assert_same_csr((rp.cpu().numpy(), col.cpu().numpy(), val.cpu().numpy()),
+                        oracle.multiply(M, "AA"), f"instance {b}")

@@ -195,6 +195,7 @@ struct spg_plan {
   bool small = false;
   uint16_t* runlen = nullptr;  // runs of shifted rows (nullptr: none looked for)
   int small_log2 = 6;
+  int small_narrow = 0, small_lanes = 32;  // > 0: narrow rows of up to this many columns
   int small_sort = 0;  // > 0: sorted rows of up to this many products instead
   int32_t* hqueue = nullptr;  // next row of the CTA-per-row kernels, one counter per bin
                               // (zeroed before each launch; bins may run at once)
@@ -416,7 +417,6 @@ int64_t exec_workspace(int64_t n, bool gram, int64_t nnz_low) {
 int64_t plan_workspace_bound(const spg_config& cfg, spg_task task, int64_t n, int64_t nnz) {
   const int64_t nn = n > 0 ? n : 1, nz = nnz > 0 ? nnz : 1;
   const int64_t scan = (int64_t)scan_tmp_bytes(n);
-  const int64_t nblocks = (n + kBinRowsPerBlock - 1) / kBinRowsPerBlock;
   int64_t b = 0;
   if (task != SPG_TASK_AA) {
     b += 8 * nz;                                  // values of Aᵀ
@@ -425,7 +425,7 @@ int64_t plan_workspace_bound(const spg_config& cfg, spg_task task, int64_t n, in
   }
   b += 8 * nn + 4 * nn + 4 * nn + 4;                              // f, lo, hi, queue
   b += 16 * nn + 8 * prepass_pieces(nz) + 8 + 7 * nn;                             // pre-pass, runs
-  b += 4 * kNumBins * (nblocks > 0 ? nblocks : 1) + 8 * 4 * kNumBins + 4 * nn;  // binning
+  b += nn + 8 * (2 * kBinWork + kRowStats) + 4 * nn;              // binning, statistics
   b += 4 * nn + 8 * (nn + 1) + scan;                              // heavy block offsets
   const int64_t per_row_blocks = (nn + 1023) / 1024 + 1;
   const int64_t blocks = nn > cfg.heavy_block_budget / per_row_blocks ? cfg.heavy_block_budget
@@ -483,7 +483,7 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   const size_t nn = (size_t)(n > 0 ? n : 1), nz = (size_t)(nnz > 0 ? nnz : 1);
   const size_t o_f = take(8 * nn), o_lo = take(4 * nn), o_hi = take(4 * nn),
                o_cnt = take(4 * nn), o_rp = take(8 * (nn + 1)), o_scan = take(scan_tmp_bytes(n)),
-               o_stats = take(32), o_q = take(4 * kNumBins);
+               o_stats = take(8 * kRowStats), o_q = take(4 * kNumBins);
   size_t o_bp = 0, o_bi = 0, o_bx = 0, o_tc = 0, o_tu = 0, o_ts = 0, o_tk = 0, o_tv = 0,
          o_ll = 0, o_lc = 0;
   if (aat) {
@@ -554,16 +554,14 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   }
   {
     ProfScope ps(ctx, "plan/scan", st);
-    TRY_CUDA(launch_scan_stats_small(p->rownnz, p->f, n, p->rowptr, stats, w + o_scan, st),
-             "row pointer scan");
+    TRY_CUDA(launch_row_pointers(p->rownnz, nullptr, p->f, p->lo, p->hi, n, p->rowptr, stats,
+                                 w + o_scan, st), "row pointer scan");
   }
   int64_t* hp = ctx->h_pin;
   TRY_CUDA(cudaMemcpyAsync(hp, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st),
            "readback");
-  TRY_CUDA(cudaMemcpyAsync(hp + 1, p->rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st),
+  TRY_CUDA(cudaMemcpyAsync(hp + 1, stats, sizeof(int64_t) * kRowStats, cudaMemcpyDeviceToHost, st),
            "readback");
-  TRY_CUDA(cudaMemcpyAsync(hp + 2, stats, sizeof(unsigned long long) * 3, cudaMemcpyDeviceToHost,
-                           st), "readback");
   TRY_CUDA(cudaStreamSynchronize(st), "plan sync");
   const uint32_t bits = *(const uint32_t*)hp;
   if (bits & DEV_ERR_INVALID_CSR) return status_from_bits(DEV_ERR_INVALID_CSR);
@@ -572,8 +570,8 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
     return SPG_OK;
   }
   TRY(status_from_bits(bits));
-  const unsigned long long* sv = (const unsigned long long*)(hp + 2);
-  p->nnz_c = n > 0 ? hp[1] : 0;
+  const unsigned long long* sv = (const unsigned long long*)(hp + 1);
+  p->nnz_c = (int64_t)sv[4];
   p->info.nnz_c = p->nnz_c;
   p->info.products = (int64_t)sv[0];
   p->info.products_computed = (int64_t)sv[0];
@@ -588,6 +586,14 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   int lg = ceil_log2_64((int64_t)sv[2] * 100 / ctx->cfg.num_load_pct + 1);
   p->small_log2 = lg < kMinTableLog2 ? kMinTableLog2 : (lg > 11 ? 11 : lg);
   // products that hardly merge: sorted rows, sized from the largest row
+  // narrow rows: by the widest row and the means over all rows
+  if (n > 0 && sv[0] > 0 && sv[1] <= (unsigned long long)kNarrowMaxProducts &&
+      (int64_t)sv[0] >= kNarrowMinProducts * n &&
+      narrow_row_rule((int64_t)sv[0] / n, (int32_t)((nnz + n - 1) / n), (int64_t)sv[3])) {
+    p->small_narrow = kNarrowMin;
+    while (p->small_narrow < (int64_t)sv[3]) p->small_narrow <<= 1;
+    p->small_lanes = (int64_t)sv[0] > kNarrowHalfMean * nnz ? 32 : 16;
+  }
   if ((int64_t)sv[0] >= kSortMinProducts * n && sorted_row((int64_t)sv[1], kSortMaxProducts, n) &&
       2 * (int64_t)sv[0] <= kSortMaxMerge2 * p->nnz_c)
     p->small_sort = (int)sv[1];
@@ -678,12 +684,13 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   TRY(palloc(p, &p->lo, n));
   TRY(palloc(p, &p->hi, n));
   TRY(palloc(p, &p->hqueue, kNumBins));
-  const int nblocks = (n + kBinRowsPerBlock - 1) / kBinRowsPerBlock;
-  int32_t* hist;
-  int64_t* counts;
+  uint8_t* bin;
+  int64_t *work, *work_num;  // binning; the numeric one and the row statistics side by side
   int32_t* rows_sym;
-  TRY(palloc(p, &hist, (int64_t)kNumBins * (nblocks > 0 ? nblocks : 1)));
-  TRY(palloc(p, &counts, 4 * kNumBins));
+  TRY(palloc(p, &bin, n));
+  TRY(palloc(p, &work, 2 * kBinWork + kRowStats));
+  work_num = work + kBinWork;
+  unsigned long long* stats = (unsigned long long*)(work_num + kBinWork);
   TRY(palloc(p, &rows_sym, n));
   const int force = ctx->cfg.force_heavy ? 1 : 0;
   const int num_lg = table_log2_cap(ctx->cfg.max_smem_slots);
@@ -724,21 +731,16 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
                  numeric_heavy_min(num_lg, ctx->cfg.num_load_pct),
                  p->A.rowptr, split, short_lg,
                  numeric_heavy_min(short_lg, ctx->cfg.num_load_pct), dense_lw, 0, panels,
-                 pre.lead, pre.runlen, pre.need};
+                 pre.lead, pre.runlen, pre.need, gram ? 0 : 1};
   // column blocks of the heavy rows: 1024 columns (windows are packed from
   // the counts; a block above the window cap, 675 columns at the default
   // load, is cut into fixed 512-column windows); wider when that many counts
   // would exceed heavy_block_budget (chosen after the readback below)
   p->blk_log2 = 10;
   heavy_shape(ctx->cfg, n, &p->window_bits, &p->heavy_threads);
-  int32_t* nblk;
-  void* btmp;
-  TRY(palloc(p, &nblk, n));
-  TRY(palloc(p, &p->blk_off, (int64_t)n + 1));
-  TRY(palloc(p, (char**)&btmp, (int64_t)scan_tmp_bytes(n)));
   int64_t* hp = p->ctx->h_pin;
-  // pre-pass, binning and block offsets over the current B, then one readback
-  // of the bin sizes, the heavy blocks' total and the two status words
+  // pre-pass and binning over the current B, then one readback of the bin sizes
+  // with the heavy blocks' total, and the two status words
   auto bin_pass = [&]() -> spg_status {
     {  // A is validated in the same reads (the verdict comes back below)
       ProfScope ps(ctx, "plan/prepass", st);
@@ -746,26 +748,19 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     }
     {
       ProfScope ps(ctx, "plan/bin_sym", st);
-      TRY_CUDA(launch_bin_rows(bsym, hist, counts, rows_sym, st), "symbolic binning");
+      TRY_CUDA(launch_bin_rows(bsym, bin, work, rows_sym, st), "symbolic binning");
     }
-    {
-      ProfScope ps(ctx, "plan/heavy_blocks", st);
-      TRY_CUDA(launch_heavy_blocks(bsym, p->blk_log2, nblk, p->blk_off, btmp, st),
-               "heavy blocks");
-    }
-    TRY_CUDA(cudaMemcpyAsync(hp, counts, sizeof(int64_t) * 2 * kNumBins, cudaMemcpyDeviceToHost,
+    TRY_CUDA(cudaMemcpyAsync(hp, work, sizeof(int64_t) * (kNumBins + 1), cudaMemcpyDeviceToHost,
                              st), "bin readback");
-    TRY_CUDA(cudaMemcpyAsync(hp + 2 * kNumBins, p->blk_off + n, sizeof(int64_t),
-                             cudaMemcpyDeviceToHost, st), "bin readback");
-    TRY_CUDA(cudaMemcpyAsync(hp + 2 * kNumBins + 1, ctx->d_status, 2 * sizeof(uint32_t),
+    TRY_CUDA(cudaMemcpyAsync(hp + kNumBins + 1, ctx->d_status, 2 * sizeof(uint32_t),
                              cudaMemcpyDeviceToHost, st), "status readback");
     TRY_CUDA(cudaStreamSynchronize(st), "bin sync");
-    const uint32_t* words = (const uint32_t*)(hp + 2 * kNumBins + 1);
+    const uint32_t* words = (const uint32_t*)(hp + kNumBins + 1);
     if (words[0] & DEV_ERR_INVALID_CSR) return status_from_bits(DEV_ERR_INVALID_CSR);
     return SPG_OK;
   };
   TRY(bin_pass());
-  if (p->symmetric && ((const uint32_t*)(hp + 2 * kNumBins + 1))[1] != 0) {
+  if (p->symmetric && ((const uint32_t*)(hp + kNumBins + 1))[1] != 0) {
     // A·Aᵀ of a pattern that is not symmetric: transpose and bin again
     TRY(build_transpose());
     TRY(bin_pass());
@@ -774,12 +769,13 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   int64_t sym_count[kNumBins], sym_start[kNumBins];
   for (int b = 0; b < kNumBins; ++b) {
     sym_count[b] = hp[b];
-    sym_start[b] = hp[kNumBins + b];
+    sym_start[b] = b ? sym_start[b - 1] + sym_count[b - 1] : 0;
   }
   // A row's blocks of 2^b columns are at most its blocks of 1024 columns times
   // 2^(10−b), or for b > 10 divided by 2^(b−10) plus two, so other widths need
   // no second readback
-  int64_t total_blocks = hp[2 * kNumBins];
+  const int64_t blocks_1024 = hp[kNumBins];
+  int64_t total_blocks = blocks_1024;
   const int64_t heavy_sym = sym_count[kHeavyBin];
   const int64_t budget = ctx->cfg.heavy_block_budget;
   // panels of 1024 columns, narrower while they are too few to fill the GPU's
@@ -795,12 +791,17 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   while (total_blocks > budget && p->blk_log2 < 20 &&
          p->window_bits % (2 << p->blk_log2) == 0) {
     ++p->blk_log2;
-    total_blocks = p->blk_log2 <= 10 ? hp[2 * kNumBins] << (10 - p->blk_log2)
-                                     : (hp[2 * kNumBins] >> (p->blk_log2 - 10)) + 2 * heavy_sym;
+    total_blocks = p->blk_log2 <= 10 ? blocks_1024 << (10 - p->blk_log2)
+                                     : (blocks_1024 >> (p->blk_log2 - 10)) + 2 * heavy_sym;
   }
   if (p->pan_log2 > 0 && p->blk_log2 > p->pan_log2)
     p->pan_log2 = p->blk_log2 <= 12 ? p->blk_log2 : 0;
-  if (p->blk_log2 != 10) {
+  if (heavy_sym > 0) {
+    int32_t* nblk;
+    void* btmp;
+    TRY(palloc(p, &nblk, n));
+    TRY(palloc(p, &p->blk_off, (int64_t)n + 1));
+    TRY(palloc(p, (char**)&btmp, (int64_t)scan_tmp_bytes(n)));
     ProfScope ps(ctx, "plan/heavy_blocks", st);
     TRY_CUDA(launch_heavy_blocks(bsym, p->blk_log2, nblk, p->blk_off, btmp, st), "heavy blocks");
   }
@@ -838,6 +839,16 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     ProfScope ps(ctx, "sym/bin", bs, b);
     TRY_CUDA(launch_hash_bin(b, false, gram, r, ctx->num_sms, bs), "symbolic");
   }
+  for (int b = kNarrowBin0; b < kNumBins; ++b) {
+    if (sym_count[b] == 0) continue;
+    RowArgs r = ra;
+    r.rows = rows_sym + sym_start[b];
+    r.nrows = (int32_t)sym_count[b];
+    const int w = kNarrowMin << ((b - kNarrowBin0) >> 1), lanes = (b - kNarrowBin0) & 1 ? 32 : 16;
+    const cudaStream_t bs = fork.next();
+    ProfScope ps(ctx, "sym/narrow", bs, w);
+    TRY_CUDA(launch_narrow(false, w, lanes, r, ctx->num_sms, bs), "symbolic");
+  }
   for (int b = kDenseBin0; b < kSortBin0; ++b) {
     if (sym_count[b] == 0) continue;
     RowArgs r = ra;
@@ -866,18 +877,14 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   }
   TRY_CUDA(fork.join(), "join");
 
-  if (runs) {
-    ProfScope ps(ctx, "plan/run_counts", st);
-    TRY_CUDA(launch_run_counts(pre.lead, n, p->rownnz, st), "run counts");
-  }
-
   // C row pointers (and lower-part offsets of the Gram mirror)
   void* scan_tmp;
   TRY(palloc(p, (char**)&scan_tmp, (int64_t)scan_tmp_bytes(n)));
   TRY(palloc(p, &p->rowptr, (int64_t)n + 1));
   {
     ProfScope ps(ctx, "plan/scan", st);
-    TRY_CUDA(launch_scan_i32_i64(p->rownnz, p->rowptr, n, scan_tmp, st), "row pointer scan");
+    TRY_CUDA(launch_row_pointers(p->rownnz, pre.lead, p->f, p->lo, p->hi, n, p->rowptr, stats,
+                                 scan_tmp, st), "row pointer scan");
   }
   if (gram) {
     void* scan_tmp2;
@@ -890,35 +897,29 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   TRY(palloc(p, &p->rows_num, n));
   BinSource bnum{1, n, p->f, p->lo, p->hi, p->rownnz, gram ? p->rowlow : nullptr, num_lg, force,
                  ctx->cfg.num_load_pct, 0, p->A.rowptr, split, short_lg, 0, dense_lw,
-                 gram ? 0 : 1, panels, pre.lead, pre.runlen, pre.need};
+                 gram ? 0 : 1, panels, pre.lead, pre.runlen, pre.need, gram ? 0 : 1};
   {
     ProfScope ps(ctx, "plan/bin_num", st);
-    TRY_CUDA(launch_bin_rows(bnum, hist, counts + 2 * kNumBins, p->rows_num, st),
+    TRY_CUDA(launch_bin_rows(bnum, bin, work_num, p->rows_num, st),
              "numeric binning");
   }
-  unsigned long long* stats = nullptr;
-  TRY(palloc(p, &stats, 4));
-  TRY_CUDA(launch_row_stats(p->f, p->rownnz, n, stats, st), "row stats");
-  TRY_CUDA(cudaMemcpyAsync(hp, counts + 2 * kNumBins, sizeof(int64_t) * 2 * kNumBins,
-                           cudaMemcpyDeviceToHost, st), "readback");
-  TRY_CUDA(cudaMemcpyAsync(hp + 2 * kNumBins, p->rowptr + n, sizeof(int64_t),
-                           cudaMemcpyDeviceToHost, st), "readback");
+  constexpr int kBack = kBinWork + kRowStats;
+  TRY_CUDA(cudaMemcpyAsync(hp, work_num, sizeof(int64_t) * kBack, cudaMemcpyDeviceToHost, st),
+           "readback");
   if (gram)
-    TRY_CUDA(cudaMemcpyAsync(hp + 2 * kNumBins + 1, p->lowptr + n, sizeof(int64_t),
-                             cudaMemcpyDeviceToHost, st), "readback");
-  TRY_CUDA(cudaMemcpyAsync(hp + 2 * kNumBins + 2, stats, sizeof(unsigned long long) * 3,
-                           cudaMemcpyDeviceToHost, st), "readback");
-  TRY_CUDA(cudaMemcpyAsync(hp + 2 * kNumBins + 5, ctx->d_status, sizeof(uint32_t),
+    TRY_CUDA(cudaMemcpyAsync(hp + kBack, p->lowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost,
+                             st), "readback");
+  TRY_CUDA(cudaMemcpyAsync(hp + kBack + 1, ctx->d_status, sizeof(uint32_t),
                            cudaMemcpyDeviceToHost, st), "readback");
   TRY_CUDA(cudaStreamSynchronize(st), "plan sync");
-  TRY(status_from_bits(*(uint32_t*)(hp + 2 * kNumBins + 5)));
+  TRY(status_from_bits(*(uint32_t*)(hp + kBack + 1)));
   for (int b = 0; b < kNumBins; ++b) {
     p->num_count[b] = hp[b];
-    p->num_start[b] = hp[kNumBins + b];
+    p->num_start[b] = b ? p->num_start[b - 1] + p->num_count[b - 1] : 0;
   }
-  p->nnz_c = n > 0 ? hp[2 * kNumBins] : 0;
-  p->nnz_low = (gram && n > 0) ? hp[2 * kNumBins + 1] : 0;
-  const unsigned long long* sv = (const unsigned long long*)(hp + 2 * kNumBins + 2);
+  const unsigned long long* sv = (const unsigned long long*)(hp + kBinWork);
+  p->nnz_c = (int64_t)sv[4];
+  p->nnz_low = (gram && n > 0) ? hp[kBack] : 0;
   p->info.nnz_c = p->nnz_c;
   p->info.products = (int64_t)sv[0];
   p->info.products_computed = (int64_t)sv[0];
@@ -1037,7 +1038,9 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       const int bin = p->small_log2 - kMinTableLog2 + 1;
       r.G = hash_bin_lanes(bin, p->G);
       ProfScope ps(ctx, "num/small", st);
-      cudaError_t e = p->small_sort ? launch_sort_rows(p->small_sort, r, ctx->num_sms, st)
+      cudaError_t e = p->small_narrow
+                          ? launch_narrow(true, p->small_narrow, p->small_lanes, r, ctx->num_sms, st)
+                      : p->small_sort ? launch_sort_rows(p->small_sort, r, ctx->num_sms, st)
                                     : launch_hash_bin(bin, true, false, r, ctx->num_sms, st);
       if (e != cudaSuccess) result = cuda_status(e, "numeric");
     }
@@ -1053,8 +1056,19 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       cudaError_t e = launch_hash_bin(b, true, gram, r, ctx->num_sms, bs);
       if (e != cudaSuccess) result = cuda_status(e, "numeric");
     }
+    for (int b = kNarrowBin0; b < kNumBins && result == SPG_OK; ++b) {
+      if (p->num_count[b] == 0) continue;
+      RowArgs r = ra;
+      r.rows = p->rows_num + p->num_start[b];
+      r.nrows = (int32_t)p->num_count[b];
+      const int w = kNarrowMin << ((b - kNarrowBin0) >> 1), lanes = (b - kNarrowBin0) & 1 ? 32 : 16;
+      const cudaStream_t bs = fork.next();
+      ProfScope ps(ctx, "num/narrow", bs, w);
+      cudaError_t e = launch_narrow(true, w, lanes, r, ctx->num_sms, bs);
+      if (e != cudaSuccess) result = cuda_status(e, "numeric");
+    }
     ra.runlen = p->runlen;
-    for (int b = kRunBin0; b < kNumBins && result == SPG_OK; ++b) {
+    for (int b = kRunBin0; b < kNarrowBin0 && result == SPG_OK; ++b) {
       if (p->num_count[b] == 0) continue;
       RowArgs r = ra;
       r.rows = p->rows_num + p->num_start[b];

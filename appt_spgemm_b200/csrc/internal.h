@@ -45,7 +45,12 @@ constexpr int kSortBin0 = kDenseBin0 + kDenseMaxLog2W - kDenseMinLog2W + 1;  // 
 // of 2^t warps.
 constexpr int kRunBins = 4;
 constexpr int kRunBin0 = kSortBin0 + kSortBins;  // 25
-constexpr int kNumBins = kRunBin0 + kRunBins;    // 29
+// kNarrowBin0 + 2 · w + h = narrow row of up to kNarrowMin << w columns, a warp
+// (h = 1) or half of one per row.
+constexpr int kNarrowBins = 8;
+constexpr int kNarrowMin = 128;
+constexpr int kNarrowBin0 = kRunBin0 + kRunBins;  // 29
+constexpr int kNumBins = kNarrowBin0 + kNarrowBins;  // 37
 constexpr int kDenseVals = 256;  // entries of a bitmap-path row (numeric)
 
 }  // namespace spg

@@ -752,12 +752,6 @@ __global__ void __launch_bounds__(256) k_find_runs(
   need[i] = sneed[first];
 }
 
-// The rows of a run take its first row's count.
-__global__ void k_run_counts(const uint8_t* __restrict__ lead, int32_t n, int32_t* rownnz) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && lead[i]) rownnz[i] = rownnz[i - lead[i]];
-}
-
 int lanes_for(const MatView& A) {
   const double mean = A.n > 0 ? (double)A.nnz / A.n : 1.0;
   return mean <= 8 ? 8 : mean <= 16 ? 16 : 32;
@@ -806,13 +800,6 @@ cudaError_t launch_prepass_rows(const MatView& A, const MatView& B, const Prepas
   }
   k_find_runs<<<blocks, 256, 0, s>>>(A, w.info, G, w.flag_a, flag_b, w.f, w.lo, w.hi, w.lead,
                                      w.runlen, w.need, w.marks);
-  SPG_COUNT_LAUNCH();
-  return cudaGetLastError();
-}
-
-cudaError_t launch_run_counts(const uint8_t* lead, int32_t n, int32_t* rownnz, cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  k_run_counts<<<(unsigned)(((int64_t)n + 255) / 256), 256, 0, s>>>(lead, n, rownnz);
   SPG_COUNT_LAUNCH();
   return cudaGetLastError();
 }

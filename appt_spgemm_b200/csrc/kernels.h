@@ -50,6 +50,15 @@ constexpr int64_t kPanelMinSlice = 2;
 // one warp walks a windowed heavy row alone: a larger row would set its tail
 constexpr int64_t kWarpRowMaxProducts = (int64_t)1 << 17;
 
+// Narrow rows: the fewest products per entry of A's row (mean B-row length; up
+// to kNarrowHalfMean half a warp takes the row), the fewest products per column
+// spanned (1 / kNarrowFill), and the fewest and the most products.
+constexpr int64_t kNarrowMinMean = 6;
+constexpr int64_t kNarrowHalfMean = 20;
+constexpr int64_t kNarrowFill = 4;
+constexpr int64_t kNarrowMinProducts = 48;
+constexpr int64_t kNarrowMaxProducts = 1 << 16;
+
 // What a row's bin is computed from.
 struct BinSource {
   int mode;                 // 0: symbolic (from products and span), 1: numeric (from counts)
@@ -90,7 +99,21 @@ struct BinSource {
   const uint8_t* lead;
   const uint16_t* runlen;
   const uint16_t* need;
+  int narrow;               // narrow rows (0: no such rule)
 };
+
+// A row of f products from `len` entries of A over `span` columns: summed densely?
+// (The same answer for the symbolic and the numeric binning.)
+__host__ __device__ __forceinline__ bool narrow_row_rule(int64_t f, int32_t len, int64_t span) {
+  return span <= kNarrowMin << (kNarrowBins / 2 - 1) && f >= kNarrowMinMean * len &&
+         f * kNarrowFill >= span && f >= kNarrowMinProducts &&
+         f <= (span > kPanelMinSpan ? kSortMaxProducts : kNarrowMaxProducts);  // (else panels)
+}
+__host__ __device__ __forceinline__ int narrow_bin(int64_t f, int32_t len, int64_t span) {
+  int w = 0;
+  while (span > (kNarrowMin << w)) ++w;
+  return kNarrowBin0 + 2 * w + (f > kNarrowHalfMean * len ? 1 : 0);
+}
 
 // Runs: the fewest rows, and the limits of a row (products, columns spanned) and
 // of its operands for 32 rows (doubles), split over the teams of a CTA.
@@ -108,9 +131,21 @@ __host__ __device__ __forceinline__ int run_team(int64_t m, int need) {
 }
 
 __host__ __device__ __forceinline__ int ceil_log2_64(int64_t x) {
-  int l = 0;
-  while (((int64_t)1 << l) < x) ++l;
-  return l;
+  if (x <= 1) return 0;
+#ifdef __CUDA_ARCH__
+  return 64 - __clzll(x - 1);
+#else
+  return 64 - __builtin_clzll((unsigned long long)(x - 1));
+#endif
+}
+
+// log2 slots of the table that holds `size` entries at `load` percent: the
+// smallest L with 2^L >= size · 100 / load + 1 (integer division), that is with
+// size · 100 < load · 2^L.
+__host__ __device__ __forceinline__ int table_log2(int64_t size, int load) {
+  int l = ceil_log2_64(size);
+  while (size * 100 >= ((int64_t)load << l)) ++l;
+  return l < kMinTableLog2 ? kMinTableLog2 : l;
 }
 
 // Products of a row in sorted-row bin b: 128, 256, 512 (a warp), then 768, 1024,
@@ -157,10 +192,16 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
     if (m <= 0) return kEmptyBin;
     size = m;
   }
+  if (s.narrow && !s.force_heavy) {
+    const int32_t len = s.arowptr[i + 1] - s.arowptr[i];
+    const int64_t span = (int64_t)s.hi[i] - s.lo[i] + 1;
+    if (!(s.mode == 1 && s.lead && s.runlen[i]) && narrow_row_rule(s.f[i], len, span))
+      return narrow_bin(s.f[i], len, span);
+  }
   if (s.mode == 1 && s.lead && s.runlen[i]) return kRunBin0 + run_team(size, s.need[i]);
-  const int64_t want = size * 100 / s.load_pct + 1;
   if (s.force_heavy || (s.panels && paneled_row(s.f[i], s.arowptr[i + 1] - s.arowptr[i], s.lo[i], s.hi[i]))) return kHeavyBin;
-  if (s.mode == 1 && s.sort_rows && want <= ((int64_t)1 << s.max_log2) &&
+  int lg = table_log2(size, s.load_pct);
+  if (s.mode == 1 && s.sort_rows && lg <= s.max_log2 &&
       sorted_row(s.f[i], size, (int64_t)s.hi[i] - s.lo[i] + 1)) {
     int b = 0;
     while (sort_bin_products(b) < s.f[i]) ++b;
@@ -181,8 +222,6 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
       return kDenseBin0 + lw - kDenseMinLog2W;
     }
   }
-  int lg = ceil_log2_64(want);
-  if (lg < kMinTableLog2) lg = kMinTableLog2;
   if (lg > s.max_log2) return kHeavyBin;
   if (s.short_split > 0 &&
       s.f[i] < s.short_split * ((int64_t)s.arowptr[i + 1] - s.arowptr[i]) &&
@@ -193,11 +232,14 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
 
 constexpr int kBinRowsPerBlock = 1024;  // rows per block of the binning kernels
 
-// Stable binning: rows of each bin listed in increasing row order.
-//   hist:  int32[kNumBins * nblocks] (bin-major), nblocks = ceil(n / 1024)
-//   counts_out: int64[2*kNumBins] on the device → {count[b]} then {start[b]}
-cudaError_t launch_bin_rows(const BinSource& src, int32_t* hist, int64_t* counts_out,
-                            int32_t* rows_out, cudaStream_t s);
+// Binning: the rows of each bin listed one bin after another (in row order within
+// blocks of kBinRowsPerBlock rows).
+//   bin: a byte per row; work: kBinWork int64 on the device, of which the first
+//   kNumBins + 1 come back: the rows of each bin, and (symbolic) the blocks of
+//   1024 columns that the heavy rows span
+constexpr int kBinWork = 2 * kNumBins + 1;
+cudaError_t launch_bin_rows(const BinSource& src, uint8_t* bin, int64_t* work, int32_t* rows_out,
+                            cudaStream_t s);
 
 // Exclusive scan of int32 counts into int64 offsets out[0..n], out[n] = total.
 // `tmp` needs scan_tmp_bytes(n) bytes.
@@ -276,6 +318,49 @@ __device__ __forceinline__ void emit_packed(const RowArgs& a, int row, int lo, i
   }
 }
 
+// Marks the columns of a row's products, column − lo < span, with a byte each
+// (symbolic phase): plain stores of 1, in no order.  G lanes per row; the B rows
+// are walked in pieces of G entries, eight pieces' loads in flight.
+template <int G>
+__device__ __forceinline__ void narrow_mark(const RowArgs& a, const WarpGroup& g, int row, int lo,
+                                            int span, unsigned char* seen) {
+  constexpr int kAhead = 8;
+  const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+  for (int32_t pb = ps; pb < pe; pb += G) {
+    const int cnt = min(G, pe - pb);
+    int bs = 0, len = 0;
+    if (g.lane < cnt) {
+      const int32_t k = a.A.col[pb + g.lane];
+      bs = a.B.rowptr[k];
+      len = a.B.rowptr[k + 1] - bs;
+    }
+    for (int t0 = 0; t0 < cnt; t0 += kAhead) {
+      int b[kAhead], l[kAhead], x[kAhead];
+      int longest = 0;
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int t = min(t0 + u, G - 1);
+        b[u] = __shfl_sync(g.mask, bs, t, G);
+        l[u] = __shfl_sync(g.mask, len, t, G);
+        if (t0 + u >= cnt) l[u] = 0;
+        longest = max(longest, l[u]);
+        x[u] = g.lane < l[u] ? a.B.col[b[u] + g.lane] - lo : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if ((unsigned)x[u] < (unsigned)span) seen[x[u]] = 1;
+      for (int q = G; q < longest; q += G) {  // what is left of the longer ones
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+          x[u] = q + g.lane < l[u] ? a.B.col[b[u] + q + g.lane] - lo : -1;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+          if ((unsigned)x[u] < (unsigned)span) seen[x[u]] = 1;
+      }
+    }
+  }
+}
+
 // Number of bits needed for the column field of a row spanning [lo, hi].
 __device__ __forceinline__ int span_bits(int lo, int hi) {
   const uint32_t span = (uint32_t)(hi - lo);
@@ -305,6 +390,9 @@ cudaError_t launch_hash_bin(int bin, bool numeric, bool gram, const RowArgs& a, 
 cudaError_t launch_dense_bin(int bin, bool numeric, const RowArgs& a, int num_sms,
                              cudaStream_t s);
 int hash_bin_lanes(int bin, int lanes_cfg);
+// Narrow rows of up to W columns, `lanes` (16 or 32) per row (k_narrow.cu; not Gram).
+cudaError_t launch_narrow(bool numeric, int W, int lanes, const RowArgs& a, int num_sms,
+                          cudaStream_t s);
 // The pre-pass of the regular plans (k_runs.cu): products and column span per
 // row, the validation of A and, with `lead`, the runs of shifted rows.  Per row
 // of B: info; per row of A: the others; marks: two ints; pieces:
@@ -321,9 +409,8 @@ struct PrepassArrays {
 };
 cudaError_t launch_prepass_rows(const MatView& A, const MatView& B, const PrepassArrays& w,
                                 int num_sms, uint32_t* status, cudaStream_t s);
-// Runs of shifted rows: their counts after the symbolic phase, and the numeric
-// phase of the runs whose first rows are listed (teams of 2^team warps).
-cudaError_t launch_run_counts(const uint8_t* lead, int32_t n, int32_t* rownnz, cudaStream_t s);
+// Runs of shifted rows: the numeric phase of the runs whose first rows are listed
+// (teams of 2^team warps).
 cudaError_t launch_runs(int team, const RowArgs& a, int num_sms, cudaStream_t s);
 // Sorted rows of up to max_products <= kSortMaxProducts products each, numeric
 // phase (k_sort_rows.cu; not Gram).
@@ -486,14 +573,13 @@ struct DescAccum {        // device accumulators of spg_describe
 };
 cudaError_t launch_describe(const MatView& A, const int32_t* colcount, DescAccum* acc,
                             cudaStream_t s);
-// out[0] = Σ f, out[1] = max f, out[2] = max rownnz (out zeroed by the launcher).
-cudaError_t launch_row_stats(const int64_t* f, const int32_t* rownnz, int32_t n,
-                             unsigned long long* out, cudaStream_t s);
-// Row pointers of a small plan and its row statistics: one launch when n fits
-// one scan tile, else the scan and launch_row_stats.
-cudaError_t launch_scan_stats_small(const int32_t* cnt, const int64_t* f, int64_t n,
-                                    int64_t* rowptr, unsigned long long* stats, void* tmp,
-                                    cudaStream_t s);
+// Row pointers of C from the row counts (with `lead`, a run's rows take its
+// first row's count first), and kRowStats statistics: Σ products, max products,
+// max row count, max column span, nnz(C).  tmp: scan_tmp_bytes(n).
+constexpr int kRowStats = 5;
+cudaError_t launch_row_pointers(int32_t* cnt, const uint8_t* lead, const int64_t* f,
+                                const int32_t* lo, const int32_t* hi, int64_t n, int64_t* rowptr,
+                                unsigned long long* stats, void* tmp, cudaStream_t s);
 cudaError_t launch_col_count(const MatView& A, int32_t* cnt, cudaStream_t s);
 
 }  // namespace spg

@@ -104,7 +104,7 @@ def hub_rows(n, hubs, width, seed):
 @pytest.mark.parametrize("task", ["AA", "AAt", "AAtS"])
 def test_paneled_rows(eng, n, hubs, width, task):
     labels = product(eng, hub_rows(n, hubs, width, seed=n), task)
-    assert "num/panels" in labels
+    assert "num/panels" in labels or n < 1024  # (up to 1024 columns: narrow rows)
 
 
 def test_paneled_rows_signed_zeros():
@@ -180,3 +180,48 @@ def test_shifted_rows_interrupted(eng):
         rp, col, val = R.instance(b)
         assert_same_csr((rp.cpu().numpy(), col.cpu().numpy(), val.cpu().numpy()),
                         oracle.multiply(M, "AA"), f"instance {b}")
+
+
+# spans either side of each width (128 … 1024 columns) and beyond the last, B rows
+# of less than half a warp, of a warp and of several segments
+@pytest.mark.parametrize("bw,fill", [(8, 0.9), (16, 0.5), (31, 0.4), (32, 0.4), (33, 0.9),
+                                     (63, 0.2), (64, 0.3), (65, 0.8), (127, 0.1), (128, 0.5),
+                                     (129, 0.3), (255, 0.2), (256, 0.3), (257, 0.3), (300, 0.1)])
+def test_narrow_rows(eng, bw, fill):
+    A = csr.banded(3001, bw, fill, bw)
+    labels = product(eng, A, "AA")
+    if eng.binned:  # (at the edges of the matrix the widest bands have narrow rows too)
+        assert any(x.startswith("num/narrow") for x in labels)
+    product(eng, A, "AAt")
+
+
+def test_narrow_rows_signed_zeros(eng):
+    # every product a zero of either sign, or an underflow: all stay entries
+    A = csr.banded(2000, 40, 0.4, 3)
+    A.val = np.random.default_rng(4).choice([0.0, -0.0, 1e-200, -1e-200, 1.0], A.nnz)
+    product(eng, A, "AA")
+    product(eng, from_rows(3006, [[(i // 9) * 9 + 8 - i % 3] if i % 5 else [] for i in range(3000)],
+                           5), "AAt")
+
+
+def test_row_pointers_and_bins_of_many_tiles(eng):
+    # rows of every kind next to one another, n over several scan tiles and binning
+    # blocks and not a multiple of either
+    rng = np.random.default_rng(15)
+    n = 9001
+    rows = []
+    for i in range(n):
+        kind = (i // 37) % 5
+        if kind == 0:
+            rows.append([j for j in (i - 70, i - 1, i, i + 1, i + 70) if 0 <= j < n])
+        elif kind == 1:
+            rows.append(i // 2 + rng.integers(0, 200, 30))
+        elif kind == 2:
+            rows.append(rng.integers(0, n, 25))
+        elif kind == 3:
+            rows.append([])
+        else:
+            rows.append(rng.integers(0, n, 300 if i % 50 == 0 else 3))
+    A = from_rows(n, rows, 16)
+    for task in ("AA", "AAt", "AAtS"):
+        product(eng, A, task)

@@ -156,14 +156,11 @@ struct spg_plan {
   int32_t* lo = nullptr;
   int32_t* hi = nullptr;
   int32_t* rownnz = nullptr;
-  int32_t* rowlow = nullptr;
   int64_t* rowptr = nullptr;
-  int64_t* lowptr = nullptr;
   int32_t* rows_num = nullptr;
   int64_t num_count[kNumBins] = {};
   int64_t num_start[kNumBins] = {};
   int64_t nnz_c = 0;
-  int64_t nnz_low = 0;
   spg_plan_info info{};
   std::vector<void*> ptrs;
   int64_t ws_bytes = 0;
@@ -400,15 +397,6 @@ spg_status validate_device(spg_ctx* ctx, const MatView& A, cudaStream_t st,
   return status_from_bits(h[0]);
 }
 
-// Bytes execute_impl takes from the pool for the duration of an execute for
-// the Gram mirror: its cursors, lower parts and segment-sort list (0 for the
-// other tasks; the heavy rows' cursors are added by the caller).
-int64_t exec_workspace(int64_t n, bool gram, int64_t nnz_low) {
-  if (!gram) return 0;
-  const int64_t nn = n > 0 ? n : 1;
-  return 4 * nn + 12 * (nnz_low > 0 ? nnz_low : 1) + 4 * nn + 4;
-}
-
 // Upper bound of the workspace plan_build allocates (a plan's workspace_bytes)
 // for a matrix of n rows and nnz entries, from the sizes alone: every palloc of
 // plan_build at its largest (the transpose counted whenever the task needs
@@ -432,7 +420,6 @@ int64_t plan_workspace_bound(const spg_config& cfg, spg_task task, int64_t n, in
                                                                       : nn * per_row_blocks;
   b += 2 * blocks;                                                // heavy block counts
   b += 4 * nn;                                                    // row counts
-  if (task == SPG_TASK_AATS) b += 4 * nn + scan + 8 * (nn + 1);   // lower counts, offsets
   b += scan + 8 * (nn + 1);                                       // C row pointers
   b += 4 * nn + 32;                                               // numeric rows, stats
   return b + 64 * 1024;  // pool rounding of the ~40 allocations
@@ -466,7 +453,7 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   cudaStream_t st = p->stream;
   const int32_t n = Ad->n;
   const int64_t nnz = Ad->nnz;
-  const bool aat = p->task == SPG_TASK_AAT;
+  const bool aat = p->task != SPG_TASK_AA;
   p->small = true;
   p->n = n;
   p->A = MatView{n, nnz, Ad->rowptr, Ad->col, Ad->val};
@@ -524,6 +511,13 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
     // slots an invalid input leaves unwritten hold column 0, so the row sort
     // stays in range; the plan then fails on the verdict
     TRY_CUDA(cudaMemsetAsync(tw.tmp_col, 0, 4 * nz, st), "memset");
+    if (p->task == SPG_TASK_AATS) {
+      // the symmetric variant's plans say whether the pattern is symmetric (the
+      // values gathered on the way are not used)
+      ProfScope ps(ctx, "plan/transpose_sym", st);
+      TRY_CUDA(launch_sym_transpose_vals(p->A, tw.tmp_val, (int*)(ctx->d_status + 1), st),
+               "symmetry check");
+    }
     ProfScope ps(ctx, "plan/transpose", st);
     TRY_CUDA(launch_transpose(p->A, p->bt_rowptr, p->bt_col, p->bt_val, tw, ctx->num_sms, st),
              "transpose");
@@ -550,7 +544,7 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   ra.fcap = kSmallCap;
   if (n > 0) {
     ProfScope ps(ctx, "sym/small", st);
-    TRY_CUDA(launch_hash_w32(kSmallSymLog2, false, false, ra, ctx->num_sms, st), "symbolic");
+    TRY_CUDA(launch_hash_w32(kSmallSymLog2, false, ra, ctx->num_sms, st), "symbolic");
   }
   {
     ProfScope ps(ctx, "plan/scan", st);
@@ -558,7 +552,7 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
                                  w + o_scan, st), "row pointer scan");
   }
   int64_t* hp = ctx->h_pin;
-  TRY_CUDA(cudaMemcpyAsync(hp, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st),
+  TRY_CUDA(cudaMemcpyAsync(hp, ctx->d_status, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st),
            "readback");
   TRY_CUDA(cudaMemcpyAsync(hp + 1, stats, sizeof(int64_t) * kRowStats, cudaMemcpyDeviceToHost, st),
            "readback");
@@ -579,7 +573,7 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   p->info.max_row_nnz = (int64_t)sv[2];
   p->info.heavy_rows = 0;
   p->info.bins_used = 1;
-  p->info.symmetric_pattern = 0;
+  p->info.symmetric_pattern = p->task == SPG_TASK_AATS && ((const uint32_t*)hp)[1] == 0;
   // numeric table: the exact largest row at the numeric load, 16 to 2048
   // slots; tables below 2048 slots run rows on lane groups sized to B's mean
   // row length (several rows per warp), 2048 a warp per row
@@ -613,7 +607,7 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
 
 bool small_plan_eligible(const spg_ctx* ctx, spg_task task, const spg_csr_dev* A) {
   const spg_config& c = ctx->cfg;
-  return (task == SPG_TASK_AA || task == SPG_TASK_AAT) && c.small_max_nnz > 0 &&
+  return c.small_max_nnz > 0 &&
          A->nnz <= c.small_max_nnz && A->n <= kSmallMaxN && !c.force_heavy;
 }
 
@@ -621,7 +615,6 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   spg_ctx* ctx = p->ctx;
   cudaStream_t st = p->stream;
   const int32_t n = Ad->n;
-  const bool gram = p->task == SPG_TASK_AATS;
   p->n = n;
   p->A = MatView{n, Ad->nnz, Ad->rowptr, Ad->col, Ad->val};
   p->info.n = n;
@@ -659,6 +652,9 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     TRY(palloc(p, &w.long_list, n));
     TRY(palloc(p, &w.long_count, 1));
     w.status = ctx->d_status;
+    // (A is not validated yet: slots that an invalid one leaves unwritten hold
+    // column 0, so the row sort stays in range)
+    TRY_CUDA(cudaMemsetAsync(w.tmp_col, 0, 4 * (size_t)(Ad->nnz > 0 ? Ad->nnz : 1), st), "memset");
     ProfScope ps(ctx, "plan/transpose", st);
     TRY_CUDA(launch_transpose(p->A, bp, bi, bx, w, ctx->num_sms, st), "transpose");
     p->B = MatView{n, Ad->nnz, bp, bi, bx};
@@ -701,16 +697,15 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   const int short_lg = std::min(num_lg, 11);
   // panels, unless the configuration shapes the heavy path itself
   const int panels = ctx->cfg.heavy_split == 0 && ctx->cfg.heavy_vcap < 0;
-  // bitmap bins (not for the Gram path): the largest bitmap the config allows
+  // bitmap bins: the largest bitmap the config allows
   int dense_lw = -1;
-  if (!gram && ctx->cfg.dense_max_words >= (1 << kDenseMinLog2W)) {
+  if (ctx->cfg.dense_max_words >= (1 << kDenseMinLog2W)) {
     dense_lw = kDenseMinLog2W;
     while (dense_lw < kDenseMaxLog2W && ((int64_t)2 << dense_lw) <= ctx->cfg.dense_max_words)
       ++dense_lw;
   }
-  // runs of shifted rows (not for the Gram path, nor where every row is forced
-  // onto the heavy path)
-  const bool runs = !gram && !force && n > 0;
+  // runs of shifted rows, unless every row is forced onto the heavy path
+  const bool runs = !force && n > 0;
   PrepassArrays pre{};
   pre.f = p->f;
   pre.lo = p->lo;
@@ -726,12 +721,12 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     TRY(palloc(p, &pre.runlen, n));
     p->runlen = pre.runlen;
   }
-  BinSource bsym{0, n, p->f, p->lo, p->hi, nullptr, nullptr, kMaxTableLog2, force,
+  BinSource bsym{0, n, p->f, p->lo, p->hi, nullptr, kMaxTableLog2, force,
                  ctx->cfg.sym_load_pct,
                  numeric_heavy_min(num_lg, ctx->cfg.num_load_pct),
                  p->A.rowptr, split, short_lg,
                  numeric_heavy_min(short_lg, ctx->cfg.num_load_pct), dense_lw, 0, panels,
-                 pre.lead, pre.runlen, pre.need, gram ? 0 : 1};
+                 pre.lead, pre.runlen, pre.need};
   // column blocks of the heavy rows: 1024 columns (windows are packed from
   // the counts; a block above the window cap, 675 columns at the default
   // load, is cut into fixed 512-column windows); wider when that many counts
@@ -741,14 +736,15 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   int64_t* hp = p->ctx->h_pin;
   // pre-pass and binning over the current B, then one readback of the bin sizes
   // with the heavy blocks' total, and the two status words
-  auto bin_pass = [&]() -> spg_status {
+  auto bin_pass = [&](const int* skip) -> spg_status {
     {  // A is validated in the same reads (the verdict comes back below)
       ProfScope ps(ctx, "plan/prepass", st);
-      TRY_CUDA(launch_prepass_rows(p->A, p->B, pre, ctx->num_sms, ctx->d_status, st), "prepass");
+      TRY_CUDA(launch_prepass_rows(p->A, p->B, pre, ctx->num_sms, ctx->d_status, st, skip),
+               "prepass");
     }
     {
       ProfScope ps(ctx, "plan/bin_sym", st);
-      TRY_CUDA(launch_bin_rows(bsym, bin, work, rows_sym, st), "symbolic binning");
+      TRY_CUDA(launch_bin_rows(bsym, bin, work, rows_sym, st, skip), "symbolic binning");
     }
     TRY_CUDA(cudaMemcpyAsync(hp, work, sizeof(int64_t) * (kNumBins + 1), cudaMemcpyDeviceToHost,
                              st), "bin readback");
@@ -759,11 +755,13 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     if (words[0] & DEV_ERR_INVALID_CSR) return status_from_bits(DEV_ERR_INVALID_CSR);
     return SPG_OK;
   };
-  TRY(bin_pass());
+  // (a pattern found not to be symmetric by now is binned once, transposed; A is
+  // then validated in that pass)
+  TRY(bin_pass(p->symmetric ? (const int*)(ctx->d_status + 1) : nullptr));
   if (p->symmetric && ((const uint32_t*)(hp + kNumBins + 1))[1] != 0) {
     // A·Aᵀ of a pattern that is not symmetric: transpose and bin again
     TRY(build_transpose());
-    TRY(bin_pass());
+    TRY(bin_pass(nullptr));
   }
   p->info.symmetric_pattern = p->symmetric ? 1 : 0;
   int64_t sym_count[kNumBins], sym_start[kNumBins];
@@ -810,16 +808,10 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   // symbolic phase
   TRY(palloc(p, &p->rownnz, n));
   TRY_CUDA(cudaMemsetAsync(p->rownnz, 0, sizeof(int32_t) * (size_t)(n > 0 ? n : 1), st), "memset");
-  if (gram) {
-    TRY(palloc(p, &p->rowlow, n));
-    TRY_CUDA(cudaMemsetAsync(p->rowlow, 0, sizeof(int32_t) * (size_t)(n > 0 ? n : 1), st),
-             "memset");
-  }
   RowArgs ra{};
   ra.A = p->A;
   ra.B = p->B;
   ra.rownnz = p->rownnz;
-  ra.rowlow = p->rowlow;
   ra.status = ctx->d_status;
   ra.queue = p->hqueue;
   ra.lo = p->lo;
@@ -837,7 +829,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     r.queue = p->hqueue + b;
     const cudaStream_t bs = fork.next();
     ProfScope ps(ctx, "sym/bin", bs, b);
-    TRY_CUDA(launch_hash_bin(b, false, gram, r, ctx->num_sms, bs), "symbolic");
+    TRY_CUDA(launch_hash_bin(b, false, r, ctx->num_sms, bs), "symbolic");
   }
   for (int b = kNarrowBin0; b < kNumBins; ++b) {
     if (sym_count[b] == 0) continue;
@@ -872,12 +864,12 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     h.queue = p->hqueue + kHeavyBin;
     const cudaStream_t bs = fork.next();
     ProfScope ps(ctx, "sym/heavy", bs);
-    TRY_CUDA(launch_heavy(false, gram, h, p->heavy_threads, ctx->num_sms, bs),
+    TRY_CUDA(launch_heavy(false, h, p->heavy_threads, ctx->num_sms, bs),
              "symbolic heavy");
   }
   TRY_CUDA(fork.join(), "join");
 
-  // C row pointers (and lower-part offsets of the Gram mirror)
+  // C row pointers
   void* scan_tmp;
   TRY(palloc(p, (char**)&scan_tmp, (int64_t)scan_tmp_bytes(n)));
   TRY(palloc(p, &p->rowptr, (int64_t)n + 1));
@@ -886,18 +878,11 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     TRY_CUDA(launch_row_pointers(p->rownnz, pre.lead, p->f, p->lo, p->hi, n, p->rowptr, stats,
                                  scan_tmp, st), "row pointer scan");
   }
-  if (gram) {
-    void* scan_tmp2;
-    TRY(palloc(p, (char**)&scan_tmp2, (int64_t)scan_tmp_bytes(n)));
-    TRY(palloc(p, &p->lowptr, (int64_t)n + 1));
-    TRY_CUDA(launch_scan_i32_i64(p->rowlow, p->lowptr, n, scan_tmp2, st), "lower scan");
-  }
-
   // numeric binning by exact counts, stats; host sync #2 (nnz(C))
   TRY(palloc(p, &p->rows_num, n));
-  BinSource bnum{1, n, p->f, p->lo, p->hi, p->rownnz, gram ? p->rowlow : nullptr, num_lg, force,
+  BinSource bnum{1, n, p->f, p->lo, p->hi, p->rownnz, num_lg, force,
                  ctx->cfg.num_load_pct, 0, p->A.rowptr, split, short_lg, 0, dense_lw,
-                 gram ? 0 : 1, panels, pre.lead, pre.runlen, pre.need, gram ? 0 : 1};
+                 1, panels, pre.lead, pre.runlen, pre.need};
   {
     ProfScope ps(ctx, "plan/bin_num", st);
     TRY_CUDA(launch_bin_rows(bnum, bin, work_num, p->rows_num, st),
@@ -906,20 +891,16 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   constexpr int kBack = kBinWork + kRowStats;
   TRY_CUDA(cudaMemcpyAsync(hp, work_num, sizeof(int64_t) * kBack, cudaMemcpyDeviceToHost, st),
            "readback");
-  if (gram)
-    TRY_CUDA(cudaMemcpyAsync(hp + kBack, p->lowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                             st), "readback");
-  TRY_CUDA(cudaMemcpyAsync(hp + kBack + 1, ctx->d_status, sizeof(uint32_t),
+  TRY_CUDA(cudaMemcpyAsync(hp + kBack, ctx->d_status, sizeof(uint32_t),
                            cudaMemcpyDeviceToHost, st), "readback");
   TRY_CUDA(cudaStreamSynchronize(st), "plan sync");
-  TRY(status_from_bits(*(uint32_t*)(hp + kBack + 1)));
+  TRY(status_from_bits(*(uint32_t*)(hp + kBack)));
   for (int b = 0; b < kNumBins; ++b) {
     p->num_count[b] = hp[b];
     p->num_start[b] = b ? p->num_start[b - 1] + p->num_count[b - 1] : 0;
   }
   const unsigned long long* sv = (const unsigned long long*)(hp + kBinWork);
   p->nnz_c = (int64_t)sv[4];
-  p->nnz_low = (gram && n > 0) ? hp[kBack] : 0;
   p->info.nnz_c = p->nnz_c;
   p->info.products = (int64_t)sv[0];
   p->info.products_computed = (int64_t)sv[0];
@@ -940,7 +921,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
                    std::max<int64_t>((int64_t)64 << 20, p->info.output_bytes / 8);
   }
   p->info.exec_workspace_bytes =
-      exec_workspace(n, gram, p->nnz_low) + (p->heavy_windows ? 16 * Ad->nnz : 0) +
+      (p->heavy_windows ? 16 * Ad->nnz : 0) +
       (p->npan > 0 ? panel_workspace(n, p->npan, p->num_count[kHeavyBin], p->pan_table) : 0);
   return SPG_OK;
 }
@@ -948,7 +929,6 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
 spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
   spg_ctx* ctx = p->ctx;
   const int32_t n = p->n;
-  const bool gram = p->task == SPG_TASK_AATS;
   if (!C) return set_error(SPG_ERR_INVALID_ARG, "null output");
   if (C->n != n) return set_error(SPG_ERR_INVALID_ARG, "output n %d != %d", C->n, n);
   if (!C->rowptr || (p->nnz_c > 0 && (!C->col || !C->val)))
@@ -994,7 +974,6 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
     ra.B = p->B;
     ra.rowptr = p->rowptr;
     ra.cnt_in = p->rownnz;
-    ra.low_in = p->rowlow;
     ra.ccol = C->col;
     ra.cval = C->val;
     ra.status = ctx->d_status;
@@ -1002,18 +981,6 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
     ra.lo = p->lo;
     ra.hi = p->hi;
     ra.colbase = p->colbase;
-    if (gram) {
-      void *cur, *lc, *lv;
-      if ((result = talloc(&cur, sizeof(int32_t) * (size_t)n)) != SPG_OK) break;
-      if ((result = talloc(&lc, sizeof(int32_t) * (size_t)p->nnz_low)) != SPG_OK) break;
-      if ((result = talloc(&lv, sizeof(double) * (size_t)p->nnz_low)) != SPG_OK) break;
-      cudaError_t e = cudaMemsetAsync(cur, 0, sizeof(int32_t) * (size_t)n, st);
-      if (e != cudaSuccess) { result = cuda_status(e, "memset"); break; }
-      ra.lowptr = p->lowptr;
-      ra.cursor = (int32_t*)cur;
-      ra.lcol = (int32_t*)lc;
-      ra.lval = (double*)lv;
-    }
     // the heavy rows' cursors are taken from the pool before the bins fork, so
     // their allocation is ordered before every stream that uses them
     int4* hcur = nullptr;
@@ -1041,7 +1008,7 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       cudaError_t e = p->small_narrow
                           ? launch_narrow(true, p->small_narrow, p->small_lanes, r, ctx->num_sms, st)
                       : p->small_sort ? launch_sort_rows(p->small_sort, r, ctx->num_sms, st)
-                                    : launch_hash_bin(bin, true, false, r, ctx->num_sms, st);
+                                    : launch_hash_bin(bin, true, r, ctx->num_sms, st);
       if (e != cudaSuccess) result = cuda_status(e, "numeric");
     }
     for (int b = 1; b <= kNumTableBins && result == SPG_OK; ++b) {
@@ -1053,7 +1020,7 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       r.queue = p->hqueue + b;
       const cudaStream_t bs = fork.next();
       ProfScope ps(ctx, "num/bin", bs, b);
-      cudaError_t e = launch_hash_bin(b, true, gram, r, ctx->num_sms, bs);
+      cudaError_t e = launch_hash_bin(b, true, r, ctx->num_sms, bs);
       if (e != cudaSuccess) result = cuda_status(e, "numeric");
     }
     for (int b = kNarrowBin0; b < kNumBins && result == SPG_OK; ++b) {
@@ -1136,45 +1103,24 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       if (p->npan > 0) {
         const cudaStream_t bs = fork.next();
         ProfScope ps(ctx, "num/panels", bs);
-        e = launch_panels(gram, h, panel_ws, p->pan_table, ctx->num_sms, bs);
+        e = launch_panels(h, panel_ws, p->pan_table, ctx->num_sms, bs);
       }
       if (e == cudaSuccess && windows) {
         const cudaStream_t bs = fork.next();
         ProfScope ps(ctx, "num/heavy_w32", bs);
-        e = launch_heavy_w32(gram, h, ctx->num_sms, bs);
+        e = launch_heavy_w32(h, ctx->num_sms, bs);
       }
       if (e == cudaSuccess) {
         const cudaStream_t bs = fork.next();
         ProfScope ps(ctx, "num/heavy", bs);
-        e = shared_values ? launch_heavy_win(gram, h, win_threads, ctx->num_sms, bs)
-                          : launch_heavy(true, gram, h, p->heavy_threads, ctx->num_sms, bs);
+        e = shared_values ? launch_heavy_win(h, win_threads, ctx->num_sms, bs)
+                          : launch_heavy(true, h, p->heavy_threads, ctx->num_sms, bs);
       }
       if (e != cudaSuccess) { result = cuda_status(e, "numeric heavy"); break; }
     }
     {
       const cudaError_t e = fork.join();
       if (e != cudaSuccess) { result = cuda_status(e, "join"); break; }
-    }
-    if (gram && p->nnz_low > 0) {
-      void *ll, *lcnt;
-      if ((result = talloc(&ll, sizeof(int32_t) * (size_t)n)) != SPG_OK) break;
-      if ((result = talloc(&lcnt, sizeof(int32_t))) != SPG_OK) break;
-      SegSortArgs sa{};
-      sa.nseg = n;
-      sa.src_off64 = p->lowptr;
-      sa.dst_off64 = p->rowptr;
-      sa.lens = p->rowlow;
-      sa.src_key = ra.lcol;
-      sa.src_val = ra.lval;
-      sa.dst_key = C->col;
-      sa.dst_val = C->val;
-      sa.key_bound = n;
-      sa.long_list = (int32_t*)ll;
-      sa.long_count = (int32_t*)lcnt;
-      sa.status = ctx->d_status;
-      ProfScope ps(ctx, "num/mirror_sort", st);
-      cudaError_t e = launch_segsort(sa, ctx->num_sms, st);
-      if (e != cudaSuccess) { result = cuda_status(e, "mirror sort"); break; }
     }
   } while (0);
   for (void* ptr : tmp) cudaFreeAsync(ptr, st);

@@ -40,8 +40,8 @@ size_t heavy_smem_bytes(bool numeric, int threads, int window_bits) {
 // warp each.
 constexpr int kLongBRow = 256;
 
-// Mark the columns of row `row` that fall in [w0, w0 + 32·nwords) (and, for
-// the Gram upper part, are >= row) in the shared bitmap.  Marking is an OR, so
+// Mark the columns of row `row` that fall in [w0, w0 + 32·nwords) in the shared
+// bitmap.  Marking is an OR, so
 // the B rows need no order: per chunk of blockDim entries of A's row, the
 // long B rows (listed in st_long) are swept by the whole CTA one after another
 // and the short ones are dealt out to the warps, a B row per warp — no search
@@ -91,7 +91,6 @@ __device__ __forceinline__ void mark_window(const RowArgs& a, int row, long long
 // At most 32 registers (no spills): 512-thread CTAs over windows of up to 2^18
 // columns then run four per SM instead of two (R-MAT 2^18: 9.59 -> 7.90 ms;
 // 2^19, three per SM: 24.2 -> 20.0 ms).
-template <bool GRAM>
 __global__ void __launch_bounds__(1024, 2) k_heavy_sym(HeavyArgs h) {
   extern __shared__ __align__(16) unsigned char smem[];
   const RowArgs& a = h.r;
@@ -107,7 +106,7 @@ __global__ void __launch_bounds__(1024, 2) k_heavy_sym(HeavyArgs h) {
     if (r >= a.nrows) break;
     const int row = a.rows[r];
     const int lo = h.lo[row], hi = h.hi[row];
-    long long c = 0, cl = 0;
+    long long c = 0;
     // windows start on a column block's first column
     const int lo_blk = lo >> h.blk_log2 << h.blk_log2;
     for (long long w0 = lo_blk; w0 <= hi; w0 += h.window_bits) {
@@ -117,7 +116,7 @@ __global__ void __launch_bounds__(1024, 2) k_heavy_sym(HeavyArgs h) {
       mark_window(a, row, w0, nwords, bm, st_bs, st_ex, st_long, scratch);
       // a warp per column block of the window (32 or more words): the bit
       // counts are the row totals and, when asked for, the block counts
-      int lc = 0, lcl = 0;
+      int lc = 0;
       const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
       const int wpb = 1 << (h.blk_log2 - 5);
       const long long blk0 = (w0 - lo_blk) >> h.blk_log2;
@@ -126,11 +125,6 @@ __global__ void __launch_bounds__(1024, 2) k_heavy_sym(HeavyArgs h) {
         for (int i = blk * wpb + lane; i < min((blk + 1) * wpb, nwords); i += 32) {
           const uint32_t wd = bm[i];
           bc += __popc(wd);
-          if (GRAM) {
-            const long long c0 = w0 + 32LL * i;
-            if (c0 + 32 <= row) lcl += __popc(wd);
-            else if (c0 < row) lcl += __popc(wd & ((1u << (unsigned)(row - c0)) - 1u));
-          }
         }
         lc += bc;
         if (h.blk_cnt) {
@@ -139,11 +133,9 @@ __global__ void __launch_bounds__(1024, 2) k_heavy_sym(HeavyArgs h) {
         }
       }
       c += block_sum64(lc, (long long*)scratch);
-      if (GRAM) cl += block_sum64(lcl, (long long*)scratch);
     }
     if (threadIdx.x == 0) {
       a.rownnz[row] = (int)c;
-      if (GRAM) a.rowlow[row] = (int)cl;
     }
     __syncthreads();
   }
@@ -166,7 +158,7 @@ __device__ __forceinline__ int window_rank(const uint32_t* bm, const int* pre4, 
 // 90.4 ms for A·A.
 constexpr int kNumMinBlocks512 = 3;
 
-template <bool GRAM, int MAXT, int MINB>
+template <int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num(HeavyArgs h) {
   extern __shared__ __align__(16) unsigned char smem[];
   const RowArgs& a = h.r;
@@ -186,11 +178,10 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num(HeavyArgs h) {
     if (r >= a.nrows) break;
     const int row = a.rows[r];
     const int hi = h.hi[row];
-    const int lo = GRAM ? max(h.lo[row], row) : h.lo[row];
-    const int32_t low = GRAM ? a.low_in[row] : 0;
-    const long long expect = (long long)a.cnt_in[row] - low;
+    const int lo = h.lo[row];
+    const long long expect = (long long)a.cnt_in[row];
     if (heavy_row_paneled(h, row) || heavy_row_windowed(h, row)) continue;  // another kernel's row
-    const int64_t base = a.rowptr[row] + low;
+    const int64_t base = a.rowptr[row];
     const int cb = a.colbase ? a.colbase[row] : 0;
     long long written = 0;
     for (long long w0 = lo; w0 <= hi; w0 += h.window_bits) {
@@ -303,22 +294,6 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num(HeavyArgs h) {
       written += tot;
     }
     if (written != expect && tid == 0) report(a.status, DEV_ERR_OVERFLOW);
-    if (GRAM) {
-      const long long m = written < expect ? written : expect;
-      for (long long t = tid; t < m; t += HT) {
-        const int j = a.ccol[base + t] + cb;
-        if (j > row) {
-          const int pos = atomicAdd(&a.cursor[j], 1);
-          if (pos < a.low_in[j]) {
-            const int64_t d = a.lowptr[j] + pos;
-            a.lcol[d] = row - cb;
-            a.lval[d] = a.cval[base + t];
-          } else {
-            report(a.status, DEV_ERR_OVERFLOW);
-          }
-        }
-      }
-    }
     __syncthreads();
   }
 }
@@ -362,7 +337,7 @@ cudaError_t launch_heavy_blocks(const BinSource& bsym, int blk_log2, int32_t* nb
   return launch_scan_i32_i64(nblk, blk_off, bsym.n, scan_tmp, s);
 }
 
-cudaError_t launch_heavy(bool numeric, bool gram, const HeavyArgs& h, int threads, int num_sms,
+cudaError_t launch_heavy(bool numeric, const HeavyArgs& h, int threads, int num_sms,
                          cudaStream_t s) {
   if (h.r.nrows <= 0) return cudaSuccess;
   const size_t smem = heavy_smem_bytes(numeric, threads, h.window_bits);
@@ -370,13 +345,9 @@ cudaError_t launch_heavy(bool numeric, bool gram, const HeavyArgs& h, int thread
   cudaError_t e = cudaMemsetAsync(h.queue, 0, sizeof(int32_t), s);
   if (e != cudaSuccess) return e;
   if (numeric && threads <= 512)
-    return gram ? launch_h(k_heavy_num<true, 512, kNumMinBlocks512>, threads, smem, h, num_sms, s)
-                : launch_h(k_heavy_num<false, 512, kNumMinBlocks512>, threads, smem, h, num_sms, s);
-  if (numeric)
-    return gram ? launch_h(k_heavy_num<true, 1024, 1>, threads, smem, h, num_sms, s)
-                : launch_h(k_heavy_num<false, 1024, 1>, threads, smem, h, num_sms, s);
-  return gram ? launch_h(k_heavy_sym<true>, threads, smem, h, num_sms, s)
-              : launch_h(k_heavy_sym<false>, threads, smem, h, num_sms, s);
+    return launch_h(k_heavy_num<512, kNumMinBlocks512>, threads, smem, h, num_sms, s);
+  if (numeric) return launch_h(k_heavy_num<1024, 1>, threads, smem, h, num_sms, s);
+  return launch_h(k_heavy_sym, threads, smem, h, num_sms, s);
 }
 
 }  // namespace spg

@@ -62,7 +62,7 @@ __device__ __forceinline__ int window_end(const uint16_t* cnt, int b, int nb, in
 
 // One window [c0, c1) of row `row`: accumulate, sort and write its entries at
 // base + written; returns the number of entries written.
-template <int LOG2T, bool GRAM>
+template <int LOG2T>
 __device__ __forceinline__ int heavy_window(const HeavyArgs& h, int row, int ps, int pe, int c0, int c1,
                            int* keys, double* vals, int64_t base, int64_t room) {
   constexpr int T = 1 << LOG2T;
@@ -161,12 +161,12 @@ __device__ __forceinline__ int heavy_window(const HeavyArgs& h, int row, int ps,
   }
   const uint32_t* sorted = radix_sort_words<1, 8>((uint32_t*)keys, (uint32_t*)(vals + m), m,
                                                   LOG2T, span_bits(c0, c1 - 1), keys + m, nullptr);
-  emit_packed<LOG2T, GRAM>(a, row, c0, m, sorted, vals, base, lane, 32);
+  emit_packed<LOG2T>(a, row, c0, m, sorted, vals, base, lane, 32);
   __syncwarp();
   return m;
 }
 
-template <int LOG2T, bool GRAM>
+template <int LOG2T>
 __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int T = 1 << LOG2T;
@@ -181,11 +181,10 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
     const int row = a.rows[r];
     const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
     const int lo = h.lo[row], hi = h.hi[row];
-    const int lo_r = GRAM ? max(lo, row) : lo;
-    const int32_t low = GRAM ? a.low_in[row] : 0;
-    const int64_t expect = (int64_t)a.cnt_in[row] - low;
+    const int lo_r = lo;
+    const int64_t expect = (int64_t)a.cnt_in[row];
     if (!heavy_row_windowed(h, row)) continue;  // the CTA kernel's row
-    const int64_t base = a.rowptr[row] + low;
+    const int64_t base = a.rowptr[row];
     int64_t written = 0;
     if (lo_r <= hi) {
       // cursors at the first B entry >= lo_r of every B row of the row
@@ -193,14 +192,6 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
         const int32_t k = a.A.col[p];
         int s = a.B.rowptr[k];
         const int e = a.B.rowptr[k + 1];
-        if (GRAM) {
-          int l = s, u = e;  // lower bound of lo_r in the sorted B row
-          while (l < u) {
-            const int mid = (l + u) >> 1;
-            if (a.B.col[mid] < lo_r) l = mid + 1; else u = mid;
-          }
-          s = l;
-        }
         h.hcur[p] = make_int4(s, e, s < e ? a.B.col[s] : INT_MAX, 0);
       }
       __syncwarp();
@@ -216,7 +207,7 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
           const int bend = (int)min((int64_t)bstart + bw, (int64_t)hi + 1);
           for (int c0 = max(bstart, lo_r); c0 < bend;) {
             const int c1 = min(bend, bstart + ((c0 - bstart) / sw + 1) * sw);
-            written += heavy_window<LOG2T, GRAM>(h, row, ps, pe, c0, c1, keys, vals,
+            written += heavy_window<LOG2T>(h, row, ps, pe, c0, c1, keys, vals,
                                                  base + written, expect - written);
             c0 = c1;
           }
@@ -225,7 +216,7 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
           const int e = window_end(cnt, b, nb, h.cap, max_blocks);
           const int c0 = max(bstart, lo_r);
           const int c1 = (int)min((int64_t)lo_blk + ((int64_t)e << h.blk_log2), (int64_t)hi + 1);
-          written += heavy_window<LOG2T, GRAM>(h, row, ps, pe, c0, c1, keys, vals, base + written,
+          written += heavy_window<LOG2T>(h, row, ps, pe, c0, c1, keys, vals, base + written,
                                                expect - written);
           b = e;
         }
@@ -237,10 +228,10 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
 
 }  // namespace
 
-cudaError_t launch_heavy_w32(bool gram, const HeavyArgs& h, int num_sms, cudaStream_t s) {
+cudaError_t launch_heavy_w32(const HeavyArgs& h, int num_sms, cudaStream_t s) {
   if (h.r.nrows <= 0) return cudaSuccess;
   constexpr int LOG2T = kHeavyTableLog2;
-  auto kernel = gram ? k_heavy_w32<LOG2T, true> : k_heavy_w32<LOG2T, false>;
+  auto kernel = k_heavy_w32<LOG2T>;
   const int warps = 2;
   const size_t smem = (size_t)warps * ((size_t)12 << LOG2T);
   cudaError_t e;

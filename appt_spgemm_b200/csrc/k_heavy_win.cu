@@ -55,7 +55,7 @@ size_t heavy_win_smem_bytes(int threads, int vcap, int wcap_bits) {
          (size_t)threads * 4 * sizeof(int) + 64 * sizeof(int);
 }
 
-template <bool GRAM, int MAXT, int MINB>
+template <int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
   extern __shared__ __align__(16) unsigned char smem[];
   const RowArgs& a = h.r;
@@ -84,10 +84,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
     const int row = a.rows[r];
     if (heavy_row_paneled(h, row) || heavy_row_windowed(h, row)) continue;  // the windowed warp kernel's row
     const int lo = h.lo[row], hi = h.hi[row];
-    const int lo_r = GRAM ? max(lo, row) : lo;
-    const int32_t low = GRAM ? a.low_in[row] : 0;
-    const long long expect = (long long)a.cnt_in[row] - low;
-    const int64_t base = a.rowptr[row] + low;
+    const int lo_r = lo;
+    const long long expect = (long long)a.cnt_in[row];
+    const int64_t base = a.rowptr[row];
     const int cb = a.colbase ? a.colbase[row] : 0;
     const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
     long long written = 0;
@@ -97,14 +96,6 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
         const int32_t k = a.A.col[p];
         int s = a.B.rowptr[k];
         const int e = a.B.rowptr[k + 1];
-        if (GRAM) {
-          int l = s, u = e;
-          while (l < u) {
-            const int mid = (l + u) >> 1;
-            if (a.B.col[mid] < lo_r) l = mid + 1; else u = mid;
-          }
-          s = l;
-        }
         h.hcur[p] = make_int4(s, e, s < e ? a.B.col[s] : INT_MAX, 0);
       }
       const int64_t b0 = h.blk_off[row];
@@ -289,23 +280,6 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
       }
     }
     if (written != expect && tid == 0) report(a.status, DEV_ERR_OVERFLOW);
-    if (GRAM) {
-      __syncthreads();  // the row's C entries are written
-      const long long m = written < expect ? written : expect;
-      for (long long t = tid; t < m; t += HT) {
-        const int j = a.ccol[base + t] + cb;
-        if (j > row) {
-          const int pos = atomicAdd(&a.cursor[j], 1);
-          if (pos < a.low_in[j]) {
-            const int64_t d = a.lowptr[j] + pos;
-            a.lcol[d] = row - cb;
-            a.lval[d] = a.cval[base + t];
-          } else {
-            report(a.status, DEV_ERR_OVERFLOW);
-          }
-        }
-      }
-    }
     __syncthreads();
   }
 }
@@ -327,7 +301,7 @@ static cudaError_t launch_win(K kernel, int threads, size_t smem, const HeavyArg
   return cudaGetLastError();
 }
 
-cudaError_t launch_heavy_win(bool gram, const HeavyArgs& h, int threads, int num_sms,
+cudaError_t launch_heavy_win(const HeavyArgs& h, int threads, int num_sms,
                              cudaStream_t s) {
   if (h.r.nrows <= 0) return cudaSuccess;
   if (!h.queue || !h.hcur || !h.blk_cnt || h.vcap < 1024 || h.wcap_bits < 1024 ||
@@ -337,10 +311,8 @@ cudaError_t launch_heavy_win(bool gram, const HeavyArgs& h, int threads, int num
   cudaError_t e = cudaMemsetAsync(h.queue, 0, sizeof(int32_t), s);
   if (e != cudaSuccess) return e;
   if (threads <= 512)
-    return gram ? launch_win(k_heavy_num_win<true, 512, 2>, threads, smem, h, num_sms, s)
-                : launch_win(k_heavy_num_win<false, 512, 2>, threads, smem, h, num_sms, s);
-  return gram ? launch_win(k_heavy_num_win<true, 1024, 1>, threads, smem, h, num_sms, s)
-              : launch_win(k_heavy_num_win<false, 1024, 1>, threads, smem, h, num_sms, s);
+    return launch_win(k_heavy_num_win<512, 2>, threads, smem, h, num_sms, s);
+  return launch_win(k_heavy_num_win<1024, 1>, threads, smem, h, num_sms, s);
 }
 
 }  // namespace spg

@@ -36,9 +36,8 @@ constexpr int kPanelUnroll = 4;     // groups of 32 products loaded ahead
 constexpr long long kAbsent = (long long)0x8000000000000000ull;  // −0.0
 
 // First and one-past-last panel of the row's output columns.
-template <bool GRAM>
 __device__ __forceinline__ int2 row_panels(const HeavyArgs& h, int row) {
-  const int lo = GRAM ? max(h.lo[row], row) : h.lo[row];
+  const int lo = h.lo[row];
   const int hi = h.hi[row];
   if (lo > hi) return make_int2(0, 0);
   return make_int2(lo >> h.pan_log2, (hi >> h.pan_log2) + 1);
@@ -80,7 +79,6 @@ __global__ void k_panel_bounds(MatView B, int pan_log2, int npan, int32_t* __res
 // of two, so that a hub row's tasks start early and none of them is left to
 // the end), and their task offsets; off[nrows] is the number of tasks.
 constexpr int kOrderThreads = 1024;
-template <bool GRAM>
 __global__ void __launch_bounds__(kOrderThreads) k_panel_order(HeavyArgs h,
                                                                int32_t* __restrict__ order,
                                                                int64_t* __restrict__ off) {
@@ -113,7 +111,7 @@ __global__ void __launch_bounds__(kOrderThreads) k_panel_order(HeavyArgs h,
     int n = 0;
     if (r < nrows) {
       const int row = order[r];
-      const int2 p = row_panels<GRAM>(h, row);
+      const int2 p = row_panels(h, row);
       if (heavy_row_paneled(h, row)) n = p.y - p.x;
     }
     int tot;
@@ -140,7 +138,6 @@ __device__ __forceinline__ int task_row(const int64_t* off, int nrows, int64_t t
   return lo;
 }
 
-template <bool GRAM>
 __global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h,
                                                    const int32_t* __restrict__ order,
                                                    const int64_t* __restrict__ off) {
@@ -161,12 +158,11 @@ __global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h,
     if (t >= total) break;
     const int r = task_row(off, a.nrows, t);
     const int row = order[r];
-    const int2 pr = row_panels<GRAM>(h, row);
+    const int2 pr = row_panels(h, row);
     const int p = pr.x + (int)(t - off[r]);
     const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
     const int cb = a.colbase ? a.colbase[row] : 0;
     const int w0 = p << h.pan_log2;
-    const int first_col = GRAM ? max(row, w0) - w0 : 0;
 
     // 32 entries of A's row at a time: the next 32's slice bounds and the columns
     // of the 32 after them are on their way meanwhile
@@ -248,7 +244,7 @@ __global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h,
 #pragma unroll
       for (int u = 0; u < kPanelUnroll; ++u) {
         const unsigned j = (unsigned)(col[u] - w0);
-        x[u] = col[u] >= 0 && j < (unsigned)W && (!GRAM || (int)j >= first_col) ? (int)j : -1;
+        x[u] = col[u] >= 0 && j < (unsigned)W ? (int)j : -1;
         v[u] = __dadd_rn(__dmul_rn(lv[u], rv[u]), 0.0);
         st[u] = starts[u];
       }
@@ -278,19 +274,17 @@ __global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h,
       }
     }
 
-    // the panel's first slot: the distinct columns of the blocks before it (the
-    // Gram upper part starts inside its first panel)
-    const int32_t low = GRAM ? a.low_in[row] : 0;
+    // the panel's first slot: the distinct columns of the blocks before it
     int64_t before = 0;
     if (p > pr.x) {
       const int nb = (p << (h.pan_log2 - h.blk_log2)) - (h.lo[row] >> h.blk_log2);
       const uint16_t* cnt = h.blk_cnt + h.blk_off[row];
       int s = 0;
       for (int i = lane; i < nb; i += 32) s += cnt[i];
-      before = __reduce_add_sync(kFull, s) - low;
+      before = __reduce_add_sync(kFull, s);
     }
-    const int64_t base = a.rowptr[row] + low + before;
-    const int64_t room = (int64_t)a.cnt_in[row] - low - before;
+    const int64_t base = a.rowptr[row] + before;
+    const int64_t room = (int64_t)a.cnt_in[row] - before;
 
     // write the panel in column order and leave its places absent
     int64_t written = 0;
@@ -311,16 +305,6 @@ __global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h,
         if (pos < room) {
           a.ccol[base + pos] = j + e - cb;
           a.cval[base + pos] = e ? v.y : v.x;
-          if (GRAM && j + e > row) {
-            const int slot = atomicAdd(&a.cursor[j + e], 1);
-            if (slot < a.low_in[j + e]) {
-              const int64_t d = a.lowptr[j + e] + slot;
-              a.lcol[d] = row - cb;
-              a.lval[d] = e ? v.y : v.x;
-            } else {
-              report(a.status, DEV_ERR_OVERFLOW);
-            }
-          }
         }
         ++pos;
       }
@@ -340,7 +324,7 @@ int64_t panel_workspace(int64_t n, int npan, int64_t nrows, bool table) {
          align256(8 * (nrows + 1)) + 256;
 }
 
-cudaError_t launch_panels(bool gram, HeavyArgs& h, void* workspace, bool table, int num_sms,
+cudaError_t launch_panels(HeavyArgs& h, void* workspace, bool table, int num_sms,
                           cudaStream_t s) {
   if (h.r.nrows <= 0) return cudaSuccess;
   char* w = (char*)workspace;
@@ -360,12 +344,11 @@ cudaError_t launch_panels(bool gram, HeavyArgs& h, void* workspace, bool table, 
     k_panel_bounds<<<(unsigned)blocks, 256, 0, s>>>(h.r.B, h.pan_log2, h.npan, ptr);
     SPG_COUNT_LAUNCH();
   }
-  if (gram) k_panel_order<true><<<1, kOrderThreads, 0, s>>>(h, order, off);
-  else k_panel_order<false><<<1, kOrderThreads, 0, s>>>(h, order, off);
+  k_panel_order<<<1, kOrderThreads, 0, s>>>(h, order, off);
   SPG_COUNT_LAUNCH();
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
 
-  auto kernel = gram ? k_panel_num<true> : k_panel_num<false>;
+  auto kernel = k_panel_num;
   const size_t per = panel_warp_bytes(h.pan_log2);
   // two CTAs per SM, each of as many warps as half of its shared memory holds
   const int warps = (int)std::max<size_t>(1, std::min<size_t>(16, (size_t)112 * 1024 / per));

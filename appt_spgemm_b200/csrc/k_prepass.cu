@@ -131,7 +131,9 @@ cudaError_t launch_prepass(const MatView& A, const MatView& B, int64_t* f, int32
 // two, which kept the lists sorted, took 78 against 29 µs on a million rows: the
 // scan ran in one CTA.
 __global__ void __launch_bounds__(256) k_bin_count(BinSource src, uint8_t* __restrict__ bin,
-                                                   unsigned long long* __restrict__ work) {
+                                                   unsigned long long* __restrict__ work,
+                                                   const int* skip) {
+  if (skip && *skip) return;
   __shared__ int cnt[kNumBins];
   __shared__ unsigned long long blocks;
   if (threadIdx.x < kNumBins) cnt[threadIdx.x] = 0;
@@ -156,7 +158,9 @@ __global__ void __launch_bounds__(256) k_bin_count(BinSource src, uint8_t* __res
 
 __global__ void __launch_bounds__(256) k_bin_scatter(int64_t n, const uint8_t* __restrict__ bin,
                                                      unsigned long long* __restrict__ work,
-                                                     int32_t* __restrict__ rows_out) {
+                                                     int32_t* __restrict__ rows_out,
+                                                     const int* skip) {
+  if (skip && *skip) return;
   __shared__ int place[kNumBins];        // next place of each bin's rows of this block
   __shared__ int warp_cnt[8][kNumBins];
   __shared__ int cnt[kNumBins];
@@ -205,13 +209,13 @@ __global__ void __launch_bounds__(256) k_bin_scatter(int64_t n, const uint8_t* _
 }
 
 cudaError_t launch_bin_rows(const BinSource& src, uint8_t* bin, int64_t* work, int32_t* rows_out,
-                            cudaStream_t s) {
+                            cudaStream_t s, const int* skip) {
   cudaError_t e = cudaMemsetAsync(work, 0, sizeof(int64_t) * kBinWork, s);
   const int nblocks = (int)((src.n + kBinRowsPerBlock - 1) / kBinRowsPerBlock);
   if (e != cudaSuccess || nblocks == 0) return e;
-  k_bin_count<<<nblocks, 256, 0, s>>>(src, bin, (unsigned long long*)work);
+  k_bin_count<<<nblocks, 256, 0, s>>>(src, bin, (unsigned long long*)work, skip);
   SPG_COUNT_LAUNCH();
-  k_bin_scatter<<<nblocks, 256, 0, s>>>(src.n, bin, (unsigned long long*)work, rows_out);
+  k_bin_scatter<<<nblocks, 256, 0, s>>>(src.n, bin, (unsigned long long*)work, rows_out, skip);
   SPG_COUNT_LAUNCH();
   return cudaGetLastError();
 }

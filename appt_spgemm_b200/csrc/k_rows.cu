@@ -114,7 +114,7 @@ __device__ __forceinline__ int grp_compact(const CtaGroup& g, int* keys, double*
   return m;
 }
 
-template <int LOG2T, bool NUMERIC, bool GRAM, class Grp>
+template <int LOG2T, bool NUMERIC, class Grp>
 __device__ __forceinline__ void hash_row(const Grp& g, const RowArgs& a, const int row,
                                          int* __restrict__ keys, double* __restrict__ vals,
                                          int* st_bs, int* st_len, double* st_a, void* scratch,
@@ -138,7 +138,6 @@ __device__ __forceinline__ void hash_row(const Grp& g, const RowArgs& a, const i
       const double av = NUMERIC ? st_a[t] : 0.0;
       for (int q = g.lane; q < len; q += g.G) {
         const int32_t j = a.B.col[bs + q];
-        if (NUMERIC && GRAM && j < row) continue;
         // claim-first probe, as in the warp kernels (reading the slot before
         // claiming measured slower: R-MAT 2^18 A·A 62.3 against 60.2 ms)
         insert_acc<LOG2T, NUMERIC>(keys, vals, j,
@@ -150,19 +149,16 @@ __device__ __forceinline__ void hash_row(const Grp& g, const RowArgs& a, const i
   g.sync();
 
   if (!NUMERIC) {
-    int c = 0, cl = 0;
+    int c = 0;
     for (int s = g.lane; s < T; s += g.G) {
       const int k = keys[s];
       if (k != kEmptyKey) {
         ++c;
-        if (GRAM && k < row) ++cl;
       }
     }
     c = grp_sum(g, c, scratch);
-    if (GRAM) cl = grp_sum(g, cl, scratch);
     if (g.lane == 0) {
       a.rownnz[row] = c;
-      if (GRAM) a.rowlow[row] = cl;
     }
     g.sync();
     return;
@@ -172,15 +168,14 @@ __device__ __forceinline__ void hash_row(const Grp& g, const RowArgs& a, const i
     const int lo = a.lo[row];
     if ((int64_t)a.hi[row] - lo < ((int64_t)1 << (32 - LOG2T))) {
       int m = cta_compact_packed<LOG2T>(keys, lo, scratch);
-      const int32_t low = GRAM ? a.low_in[row] : 0;
-      const int expect = a.cnt_in[row] - low;
+      const int expect = a.cnt_in[row];
       if (m != expect) {
         if (g.lane == 0) report(a.status, DEV_ERR_OVERFLOW);
         if (m > expect) m = expect;
       }
       const uint32_t* sorted = radix_sort_words<(T >> 9), 8>(
           (uint32_t*)keys, rtmp, m, LOG2T, span_bits(lo, a.hi[row]), rcnt, (int*)scratch);
-      emit_packed<LOG2T, GRAM>(a, row, lo, m, sorted, vals, a.rowptr[row] + low, g.lane, g.G);
+      emit_packed<LOG2T>(a, row, lo, m, sorted, vals, a.rowptr[row], g.lane, g.G);
       g.sync();  // the table is reused by the next row
       return;
     }
@@ -192,34 +187,23 @@ __device__ __forceinline__ void hash_row(const Grp& g, const RowArgs& a, const i
   g.sync();
   bitonic_sort_pairs(g, keys, vals, P);
 
-  const int32_t low = GRAM ? a.low_in[row] : 0;
-  const int expect = a.cnt_in[row] - low;
+  const int expect = a.cnt_in[row];
   if (m != expect) {
     if (g.lane == 0) report(a.status, DEV_ERR_OVERFLOW);
     if (m > expect) m = expect;
   }
-  const int64_t base = a.rowptr[row] + low;
+  const int64_t base = a.rowptr[row];
   const int cb = a.colbase ? a.colbase[row] : 0;
   for (int t = g.lane; t < m; t += g.G) {
     const int j = keys[t];
     const double v = vals[t];
     a.ccol[base + t] = j - cb;
     a.cval[base + t] = v;
-    if (GRAM && j > row) {
-      const int pos = atomicAdd(&a.cursor[j], 1);
-      if (pos < a.low_in[j]) {
-        const int64_t d = a.lowptr[j] + pos;
-        a.lcol[d] = row - cb;
-        a.lval[d] = v;
-      } else {
-        report(a.status, DEV_ERR_OVERFLOW);
-      }
-    }
   }
   g.sync();  // the table is reused by the group's next row
 }
 
-template <int LOG2T, bool NUMERIC, bool GRAM>
+template <int LOG2T, bool NUMERIC>
 __global__ void __launch_bounds__(256) k_hash_warp(RowArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int T = 1 << LOG2T;
@@ -240,11 +224,11 @@ __global__ void __launch_bounds__(256) k_hash_warp(RowArgs a) {
   }
   st_len = st_bs + a.G;
   for (int r = blockIdx.x * rows_per_cta + gi; r < a.nrows; r += gridDim.x * rows_per_cta)
-    hash_row<LOG2T, NUMERIC, GRAM>(g, a, a.rows ? a.rows[r] : r, keys, vals, st_bs, st_len,
+    hash_row<LOG2T, NUMERIC>(g, a, a.rows ? a.rows[r] : r, keys, vals, st_bs, st_len,
                                    st_a, nullptr, nullptr, nullptr);
 }
 
-template <int LOG2T, bool NUMERIC, bool GRAM>
+template <int LOG2T, bool NUMERIC>
 __global__ void __launch_bounds__(1024) k_hash_cta(RowArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int T = 1 << LOG2T;
@@ -269,7 +253,7 @@ __global__ void __launch_bounds__(1024) k_hash_cta(RowArgs a) {
   for (int it = 0;; ++it) {
     const int r = cta_item(a.queue, a.nrows, it, &s_next);
     if (r >= a.nrows) break;
-    hash_row<LOG2T, NUMERIC, GRAM>(g, a, a.rows[r], keys, vals, st_bs, st_len, st_a, scratch,
+    hash_row<LOG2T, NUMERIC>(g, a, a.rows[r], keys, vals, st_bs, st_len, st_a, scratch,
                                    rtmp, rcnt);
   }
 }
@@ -306,7 +290,7 @@ static cudaError_t launch_kernel(K kernel, int threads, size_t smem, int nwork_c
   return cudaGetLastError();
 }
 
-template <int LOG2T, bool NUMERIC, bool GRAM>
+template <int LOG2T, bool NUMERIC>
 static cudaError_t launch_lg(const RowArgs& a, int num_sms, cudaStream_t s) {
   constexpr int T = 1 << LOG2T;
   if (LOG2T >= 11) {
@@ -317,7 +301,7 @@ static cudaError_t launch_lg(const RowArgs& a, int num_sms, cudaStream_t s) {
       const cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(int32_t), s);
       if (e != cudaSuccess) return e;
     }
-    return launch_kernel(k_hash_cta<LOG2T, NUMERIC, GRAM>, threads, smem, a.nrows, num_sms, a, s);
+    return launch_kernel(k_hash_cta<LOG2T, NUMERIC>, threads, smem, a.nrows, num_sms, a, s);
   }
   const int G = a.G;
   const size_t per = row_group_bytes(T, G, NUMERIC);
@@ -331,36 +315,33 @@ static cudaError_t launch_lg(const RowArgs& a, int num_sms, cudaStream_t s) {
   const int threads = rows * G;
   const size_t smem = per * rows;
   const int nwork = (a.nrows + rows - 1) / rows;
-  return launch_kernel(k_hash_warp<LOG2T, NUMERIC, GRAM>, threads, smem, nwork, num_sms, a, s);
+  return launch_kernel(k_hash_warp<LOG2T, NUMERIC>, threads, smem, nwork, num_sms, a, s);
 }
 
-template <bool NUMERIC, bool GRAM>
+template <bool NUMERIC>
 static cudaError_t launch_mode(int bin, const RowArgs& a, int num_sms, cudaStream_t s) {
   switch (bin + kMinTableLog2 - 1) {
-    case 4: return launch_lg<4, NUMERIC, GRAM>(a, num_sms, s);
-    case 5: return launch_lg<5, NUMERIC, GRAM>(a, num_sms, s);
-    case 6: return launch_lg<6, NUMERIC, GRAM>(a, num_sms, s);
-    case 7: return launch_lg<7, NUMERIC, GRAM>(a, num_sms, s);
-    case 8: return launch_lg<8, NUMERIC, GRAM>(a, num_sms, s);
-    case 9: return launch_lg<9, NUMERIC, GRAM>(a, num_sms, s);
-    case 10: return launch_lg<10, NUMERIC, GRAM>(a, num_sms, s);
-    case 11: return launch_lg<11, NUMERIC, GRAM>(a, num_sms, s);
-    case 12: return launch_lg<12, NUMERIC, GRAM>(a, num_sms, s);
-    case 13: return launch_lg<13, NUMERIC, GRAM>(a, num_sms, s);
-    case 14: return launch_lg<14, NUMERIC, GRAM>(a, num_sms, s);
+    case 4: return launch_lg<4, NUMERIC>(a, num_sms, s);
+    case 5: return launch_lg<5, NUMERIC>(a, num_sms, s);
+    case 6: return launch_lg<6, NUMERIC>(a, num_sms, s);
+    case 7: return launch_lg<7, NUMERIC>(a, num_sms, s);
+    case 8: return launch_lg<8, NUMERIC>(a, num_sms, s);
+    case 9: return launch_lg<9, NUMERIC>(a, num_sms, s);
+    case 10: return launch_lg<10, NUMERIC>(a, num_sms, s);
+    case 11: return launch_lg<11, NUMERIC>(a, num_sms, s);
+    case 12: return launch_lg<12, NUMERIC>(a, num_sms, s);
+    case 13: return launch_lg<13, NUMERIC>(a, num_sms, s);
+    case 14: return launch_lg<14, NUMERIC>(a, num_sms, s);
   }
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_hash_bin(int bin, bool numeric, bool gram, const RowArgs& a, int num_sms,
+cudaError_t launch_hash_bin(int bin, bool numeric, const RowArgs& a, int num_sms,
                             cudaStream_t s) {
   if (a.nrows <= 0) return cudaSuccess;
   const int lg = bin + kMinTableLog2 - 1;
-  if (a.G == 32 && lg >= 6 && lg <= 11) return launch_hash_w32(lg, numeric, gram, a, num_sms, s);
-  if (numeric) return gram ? launch_mode<true, true>(bin, a, num_sms, s)
-                           : launch_mode<true, false>(bin, a, num_sms, s);
-  return gram ? launch_mode<false, true>(bin, a, num_sms, s)
-              : launch_mode<false, false>(bin, a, num_sms, s);
+  if (a.G == 32 && lg >= 6 && lg <= 11) return launch_hash_w32(lg, numeric, a, num_sms, s);
+  return numeric ? launch_mode<true>(bin, a, num_sms, s) : launch_mode<false>(bin, a, num_sms, s);
 }
 
 }  // namespace spg

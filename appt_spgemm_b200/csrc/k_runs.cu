@@ -402,7 +402,8 @@ cudaError_t launch_runs_t(const RowArgs& a, int num_sms, cudaStream_t s) {
 // What the pre-pass reads of a row of B: {first entry, end, first column, last
 // column}, one 16-byte gather per entry of A instead of four loads (end < first:
 // a row pointer out of range).
-__global__ void k_row_info(MatView B, int4* __restrict__ info) {
+__global__ void k_row_info(MatView B, int4* __restrict__ info, const int* skip) {
+  if (skip && *skip) return;
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= B.n) return;
   const int32_t s = B.rowptr[k], e = B.rowptr[k + 1];
@@ -480,7 +481,8 @@ __global__ void __launch_bounds__(256) k_prepass_rows(
     MatView A, int32_t n_b, const int4* __restrict__ info, int G, int rows,
     int64_t* __restrict__ f, int32_t* __restrict__ lo, int32_t* __restrict__ hi,
     uint8_t* __restrict__ flag, int2* __restrict__ pieces, int64_t max_pieces,
-    int32_t* __restrict__ marks, uint32_t* status) {
+    int32_t* __restrict__ marks, uint32_t* status, const int* skip) {
+  if (skip && *skip) return;
   __shared__ int s_flagged;
   __shared__ int32_t ptr[kRunBlock + 2];  // row pointers of rows row0 − 1 … row0 + rows
   const WarpGroup g(G);
@@ -649,7 +651,8 @@ __global__ void __launch_bounds__(256) k_find_runs(
     const uint8_t* __restrict__ flag_b, const int64_t* __restrict__ f,
     const int32_t* __restrict__ lo, const int32_t* __restrict__ hi, uint8_t* __restrict__ lead,
     uint16_t* __restrict__ runlen, uint16_t* __restrict__ need,
-    const int32_t* __restrict__ marks) {
+    const int32_t* __restrict__ marks, const int* skip) {
+  if (skip && *skip) return;
   __shared__ uint32_t firsts[kRunBlock / 32];  // rows that start a run, one bit each
   __shared__ uint16_t sneed[kRunBlock];
   __shared__ uint8_t list[kRunBlock / kRunMinRows], sflag[kRunBlock];
@@ -771,20 +774,20 @@ cudaError_t launch_runs(int team, const RowArgs& a, int num_sms, cudaStream_t s)
 }
 
 cudaError_t launch_prepass_rows(const MatView& A, const MatView& B, const PrepassArrays& w,
-                                int num_sms, uint32_t* status, cudaStream_t s) {
+                                int num_sms, uint32_t* status, cudaStream_t s, const int* skip) {
   if (A.n == 0) return launch_validate(A, status, s);
   cudaError_t e = cudaMemsetAsync(w.marks, 0, 2 * sizeof(int32_t), s);
   if (e != cudaSuccess) return e;
   const int G = lanes_for(A);
   const unsigned blocks = (unsigned)(((int64_t)A.n + kRunBlock - 1) / kRunBlock);
-  k_row_info<<<blocks, 256, 0, s>>>(B, w.info);
+  k_row_info<<<blocks, 256, 0, s>>>(B, w.info, skip);
   SPG_COUNT_LAUNCH();
   // fewer rows per CTA where 256 would leave SMs without one
   int rows = kRunBlock;
   while (rows > kRowsAhead * (256 / G) && rows > 32 && A.n / rows < num_sms * 8) rows >>= 1;
   k_prepass_rows<<<(unsigned)((A.n + rows - 1) / rows), 256, 0, s>>>(
       A, B.n, w.info, G, rows, w.f, w.lo, w.hi, w.flag_a, w.pieces, prepass_pieces(A.nnz),
-      w.marks, status);
+      w.marks, status, skip);
   SPG_COUNT_LAUNCH();
   if (A.nnz > kLongRow) {
     k_prepass_long<<<num_sms * 4, 256, 0, s>>>(A, B.n, w.info, w.f, w.lo, w.hi, w.pieces,
@@ -799,7 +802,7 @@ cudaError_t launch_prepass_rows(const MatView& A, const MatView& B, const Prepas
     flag_b = w.flag_b;
   }
   k_find_runs<<<blocks, 256, 0, s>>>(A, w.info, G, w.flag_a, flag_b, w.f, w.lo, w.hi, w.lead,
-                                     w.runlen, w.need, w.marks);
+                                     w.runlen, w.need, w.marks, skip);
   SPG_COUNT_LAUNCH();
   return cudaGetLastError();
 }

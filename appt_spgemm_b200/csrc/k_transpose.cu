@@ -1,5 +1,5 @@
-// CSR → CSR-of-Aᵀ by counting sort, and the segment sort it (and the Gram
-// mirror) finishes with.
+// CSR → CSR-of-Aᵀ by counting sort, and the segment sort it
+// finishes with.
 //
 // The reference builds Aᵀ with a global atomicAdd histogram, a Thrust scan and
 // a one-thread-per-row atomic-cursor scatter (k_colcount / k_scatter /
@@ -100,16 +100,6 @@ constexpr int kMidSeg = 8192;       // CTA + shared bitonic
 constexpr int kLongThreads = 512;
 constexpr int kLongWindow = 1 << 18;  // bitmap bits of the long-segment counting sort
 
-__device__ __forceinline__ int64_t seg_src(const SegSortArgs& a, int64_t s) {
-  return a.src_off64 ? a.src_off64[s] : (int64_t)a.src_off32[s];
-}
-__device__ __forceinline__ int64_t seg_dst(const SegSortArgs& a, int64_t s) {
-  return a.dst_off64 ? a.dst_off64[s] : (int64_t)a.dst_off32[s];
-}
-__device__ __forceinline__ int64_t seg_len(const SegSortArgs& a, int64_t s) {
-  return a.lens ? (int64_t)a.lens[s] : seg_src(a, s + 1) - seg_src(a, s);
-}
-
 // One segment of at most 32·E entries by one warp: (key << 8 | index) words
 // sorted in registers, then keys written and payloads gathered by index.
 template <int E>
@@ -143,9 +133,9 @@ __global__ void __launch_bounds__(256, 4) k_segsort_short(SegSortArgs a) {
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t s = warp; s < a.nseg; s += nwarps) {
-    const int64_t len = seg_len(a, s);
+    const int64_t len = (int64_t)a.off[s + 1] - a.off[s];
     if (len <= 0) continue;
-    const int64_t so = seg_src(a, s), dof = seg_dst(a, s);
+    const int64_t so = a.off[s], dof = so;
     if (len > kShortSeg) {
       if (lane == 0) a.long_list[atomicAdd(a.long_count, 1)] = (int32_t)s;
       continue;
@@ -187,8 +177,8 @@ __global__ void __launch_bounds__(kLongThreads) k_segsort_long(SegSortArgs a) {
   const int nlong = *a.long_count;
   for (int li = blockIdx.x; li < nlong; li += gridDim.x) {
     const int64_t s = a.long_list[li];
-    const int64_t len = seg_len(a, s);
-    const int64_t so = seg_src(a, s), dof = seg_dst(a, s);
+    const int64_t len = (int64_t)a.off[s + 1] - a.off[s];
+    const int64_t so = a.off[s], dof = so;
     if (len <= kMidSeg) {
       double* vals = (double*)smem;
       int* keys = (int*)(vals + kMidSeg);
@@ -311,8 +301,7 @@ cudaError_t launch_transpose(const MatView& A, int32_t* t_rowptr, int32_t* t_col
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   SegSortArgs sa{};
   sa.nseg = n;
-  sa.src_off32 = t_rowptr;
-  sa.dst_off32 = t_rowptr;
+  sa.off = t_rowptr;
   sa.src_key = w.tmp_col;
   sa.src_val = w.tmp_val;
   sa.dst_key = t_col;

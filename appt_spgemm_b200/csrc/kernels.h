@@ -66,8 +66,7 @@ struct BinSource {
   const int64_t* f;
   const int32_t* lo;
   const int32_t* hi;
-  const int32_t* rownnz;    // numeric: entries of the row (plain) or the row total (gram)
-  const int32_t* rowlow;    // numeric gram: lower-part count (bin uses rownnz − rowlow)
+  const int32_t* rownnz;    // numeric: entries of the row
   int max_log2;             // largest shared table (log2 slots) before the heavy path
   int force_heavy;
   int load_pct;             // table sized for at most this load (percent)
@@ -87,9 +86,9 @@ struct BinSource {
   // rows whose output span fits 2^dense_max_log2w bitmap words and is at most
   // 8 columns per product, with at least 64 products (and, numeric, at most
   // kDenseVals entries) take the bitmap bins; dense_max_log2w < kDenseMinLog2W:
-  // never (the Gram path, or switched off)
+  // never
   int dense_max_log2w;
-  // numeric, not Gram: rows of up to kSortMaxProducts products of which few
+  // numeric: rows of up to kSortMaxProducts products of which few
   // merge take the sorted-row kernels
   int sort_rows;
   // rows for the panel kernel go heavy whatever their table (0: no such rule)
@@ -99,7 +98,6 @@ struct BinSource {
   const uint8_t* lead;
   const uint16_t* runlen;
   const uint16_t* need;
-  int narrow;               // narrow rows (0: no such rule)
 };
 
 // A row of f products from `len` entries of A over `span` columns: summed densely?
@@ -188,11 +186,11 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
     int64_t span = (int64_t)s.hi[i] - (int64_t)s.lo[i] + 1;
     size = f < span ? f : span;
   } else {
-    int64_t m = s.rownnz[i] - (s.rowlow ? s.rowlow[i] : 0);
+    int64_t m = s.rownnz[i];
     if (m <= 0) return kEmptyBin;
     size = m;
   }
-  if (s.narrow && !s.force_heavy) {
+  if (!s.force_heavy) {
     const int32_t len = s.arowptr[i + 1] - s.arowptr[i];
     const int64_t span = (int64_t)s.hi[i] - s.lo[i] + 1;
     if (!(s.mode == 1 && s.lead && s.runlen[i]) && narrow_row_rule(s.f[i], len, span))
@@ -238,8 +236,9 @@ constexpr int kBinRowsPerBlock = 1024;  // rows per block of the binning kernels
 //   kNumBins + 1 come back: the rows of each bin, and (symbolic) the blocks of
 //   1024 columns that the heavy rows span
 constexpr int kBinWork = 2 * kNumBins + 1;
+// `skip` (device, may be null): where it is not 0 nothing is done (work stays 0).
 cudaError_t launch_bin_rows(const BinSource& src, uint8_t* bin, int64_t* work, int32_t* rows_out,
-                            cudaStream_t s);
+                            cudaStream_t s, const int* skip = nullptr);
 
 // Exclusive scan of int32 counts into int64 offsets out[0..n], out[n] = total.
 // `tmp` needs scan_tmp_bytes(n) bytes.
@@ -259,18 +258,11 @@ struct RowArgs {
   int32_t G;                // lanes per row (warp bins); CTA bins use blockDim
   // symbolic outputs
   int32_t* rownnz;
-  int32_t* rowlow;          // gram: columns < row
   // numeric inputs / outputs
   const int64_t* rowptr;    // C row pointers
   const int32_t* cnt_in;    // symbolic counts (expected entries)
-  const int32_t* low_in;    // gram: lower counts
   int32_t* ccol;
   double* cval;
-  // gram mirror: strict-upper entries appended to a temporary lower store
-  const int64_t* lowptr;
-  int32_t* cursor;
-  int32_t* lcol;
-  double* lval;
   uint32_t* status;
   // output column span per row (pre-pass): keys of row i lie in [lo[i], hi[i]]
   const int32_t* lo;
@@ -292,9 +284,8 @@ struct RowArgs {
 
 // Writes m sorted packed words ((col − lo) << LOG2T | slot) as a row's columns
 // and the values of their table slots, lanes first, first + stride, … (so the
-// stores are coalesced); the Gram path also mirrors each entry above the
-// diagonal into the lower store through the column's atomic cursor.
-template <int LOG2T, bool GRAM>
+// stores are coalesced).
+template <int LOG2T>
 __device__ __forceinline__ void emit_packed(const RowArgs& a, int row, int lo, int m,
                                             const uint32_t* sorted, const double* vals,
                                             int64_t base, int first, int stride) {
@@ -305,16 +296,6 @@ __device__ __forceinline__ void emit_packed(const RowArgs& a, int row, int lo, i
     const double v = vals[pk & ((1u << LOG2T) - 1u)];
     a.ccol[base + e] = j - cb;
     a.cval[base + e] = v;
-    if (GRAM && j > row) {
-      const int pos = atomicAdd(&a.cursor[j], 1);
-      if (pos < a.low_in[j]) {
-        const int64_t d = a.lowptr[j] + pos;
-        a.lcol[d] = row - cb;
-        a.lval[d] = v;
-      } else {
-        report(a.status, DEV_ERR_OVERFLOW);
-      }
-    }
   }
 }
 
@@ -378,19 +359,17 @@ cudaError_t launch_gather_kept(const int64_t* rowptr, const int32_t* col, const 
 
 // Warp-per-row kernels (k_rows_w32.cu) for table bins of up to 2048 slots
 // with 32 lanes per row; returns cudaErrorNotSupported for other bins.
-cudaError_t launch_hash_w32(int log2t, bool numeric, bool gram, const RowArgs& a, int num_sms,
+cudaError_t launch_hash_w32(int log2t, bool numeric, const RowArgs& a, int num_sms,
                             cudaStream_t s);
 
-// Launch the kernel of one table bin (1..kNumTableBins).  `gram` selects the
-// A·Aᵀ upper-triangle variant (symbolic: split lower/upper counts; numeric:
-// upper part only plus the mirror append).
-cudaError_t launch_hash_bin(int bin, bool numeric, bool gram, const RowArgs& a, int num_sms,
+// Launch the kernel of one table bin (1..kNumTableBins).
+cudaError_t launch_hash_bin(int bin, bool numeric, const RowArgs& a, int num_sms,
                             cudaStream_t s);
-// Warp-per-row bitmap kernels of the dense bins (k_dense_w32.cu; not Gram).
+// Warp-per-row bitmap kernels of the dense bins (k_dense_w32.cu).
 cudaError_t launch_dense_bin(int bin, bool numeric, const RowArgs& a, int num_sms,
                              cudaStream_t s);
 int hash_bin_lanes(int bin, int lanes_cfg);
-// Narrow rows of up to W columns, `lanes` (16 or 32) per row (k_narrow.cu; not Gram).
+// Narrow rows of up to W columns, `lanes` (16 or 32) per row (k_narrow.cu).
 cudaError_t launch_narrow(bool numeric, int W, int lanes, const RowArgs& a, int num_sms,
                           cudaStream_t s);
 // The pre-pass of the regular plans (k_runs.cu): products and column span per
@@ -408,12 +387,13 @@ struct PrepassArrays {
   uint16_t *need, *runlen;
 };
 cudaError_t launch_prepass_rows(const MatView& A, const MatView& B, const PrepassArrays& w,
-                                int num_sms, uint32_t* status, cudaStream_t s);
+                                int num_sms, uint32_t* status, cudaStream_t s,
+                                const int* skip = nullptr);
 // Runs of shifted rows: the numeric phase of the runs whose first rows are listed
 // (teams of 2^team warps).
 cudaError_t launch_runs(int team, const RowArgs& a, int num_sms, cudaStream_t s);
 // Sorted rows of up to max_products <= kSortMaxProducts products each, numeric
-// phase (k_sort_rows.cu; not Gram).
+// phase (k_sort_rows.cu).
 cudaError_t launch_sort_rows(int max_products, const RowArgs& a, int num_sms, cudaStream_t s);
 
 // ---- heavy rows: dense column windows (k_heavy.cu) --------------------------
@@ -465,7 +445,7 @@ __device__ __forceinline__ bool heavy_row_windowed(const HeavyArgs& h, int row) 
   const int64_t len = (int64_t)h.r.A.rowptr[row + 1] - h.r.A.rowptr[row];
   return h.f[row] < h.split * len;
 }
-cudaError_t launch_heavy(bool numeric, bool gram, const HeavyArgs& a, int threads, int num_sms,
+cudaError_t launch_heavy(bool numeric, const HeavyArgs& a, int threads, int num_sms,
                          cudaStream_t s);
 size_t heavy_smem_bytes(bool numeric, int threads, int window_bits);
 
@@ -476,19 +456,19 @@ cudaError_t launch_heavy_blocks(const BinSource& bsym, int blk_log2, int32_t* nb
 
 // Numeric phase of the CTA rows with their values in shared memory, window by
 // window (k_heavy_win.cu); needs blk_cnt, hcur and queue.
-cudaError_t launch_heavy_win(bool gram, const HeavyArgs& a, int threads, int num_sms,
+cudaError_t launch_heavy_win(const HeavyArgs& a, int threads, int num_sms,
                              cudaStream_t s);
 size_t heavy_win_smem_bytes(int threads, int vcap, int wcap_bits);
 
 // Windowed numeric phase of heavy rows (k_heavy_w32.cu): a warp per row walks
 // the row's column blocks in windows of at most `cap` distinct columns.
-cudaError_t launch_heavy_w32(bool gram, const HeavyArgs& a, int num_sms, cudaStream_t s);
+cudaError_t launch_heavy_w32(const HeavyArgs& a, int num_sms, cudaStream_t s);
 // Numeric phase of the rows cut into panels (k_panel.cu), in `workspace` of
 // panel_workspace bytes (with or without the table of slice bounds); sets h.ptr
 // and h.task_queue.
 __host__ __device__ constexpr size_t panel_warp_bytes(int pan_log2) { return ((size_t)8 << pan_log2) + 512; }
 int64_t panel_workspace(int64_t n, int npan, int64_t nrows, bool table);
-cudaError_t launch_panels(bool gram, HeavyArgs& h, void* workspace, bool table, int num_sms,
+cudaError_t launch_panels(HeavyArgs& h, void* workspace, bool table, int num_sms,
                           cudaStream_t s);
 constexpr int kHeavyTableLog2 = 10;  // its shared table: 1024 slots per warp
 
@@ -519,11 +499,7 @@ cudaError_t launch_sym_transpose_vals(const MatView& A, double* t_val, int* asym
 // [dst_off[s], +len), len = lens ? lens[s] : src_off[s+1] − src_off[s].
 struct SegSortArgs {
   int32_t nseg;
-  const int64_t* src_off64;
-  const int32_t* src_off32;
-  const int64_t* dst_off64;
-  const int32_t* dst_off32;
-  const int32_t* lens;
+  const int32_t* off;    // segment s: entries off[s] … off[s + 1] of both sides
   const int32_t* src_key;
   const double* src_val;
   int32_t* dst_key;

@@ -254,7 +254,7 @@ class Engine:
         return Plan(self, p, A, task)
 
     def multiply(self, A: CsrDevice, task: str = "AA", stream=None) -> CsrResult:
-        """C = A·A, A·Aᵀ ("AAt") or A·Aᵀ via the Gram path ("AAtS").
+        """C = A·A or A·Aᵀ ("AAt"; "AAtS", the symmetric variant's name, is the same).
 
         The plan/execute pair of plan().execute() without the Plan object: one
         stream lookup, only n and nnz(C) read from the plan's info, so that a

@@ -6,7 +6,7 @@ through the public API with host buffers.
 
 Workload: the 3-D 27-point stencil on a 96³ grid (n = 884,736, nnz = 23.4M,
 values uniform(−1,1) from a seed), structurally symmetric, numerically
-unsymmetric; one step = one A·A plus one A·Aᵀ (through Aᵀ; the Gram path,
+unsymmetric; one step = one A·A plus one A·Aᵀ (through Aᵀ; the task AAtS,
 which gives the same C, is timed per call beside the line).
 Inputs (284 MB) and outputs (2 × 1.3 GB) exceed the 126 MB L2, so no flush
 is needed between steps.
@@ -53,9 +53,8 @@ def parse_args():
     ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
     ap.add_argument("--side", type=int, default=SIDE, help="stencil grid side (96 = the benchmark)")
     ap.add_argument("--aat-task", default="AAt", choices=["AAt", "AAtS"],
-                    help="engine task used for A·Aᵀ (AAt: the product through Aᵀ, the faster "
-                         "path on this matrix; AAtS: the Gram path, upper triangle + mirror, "
-                         "also timed beside the line)")
+                    help="engine task used for A·Aᵀ (AAtS, the symmetric variant's name, is the "
+                         "same product; also timed beside the line)")
     ap.add_argument("--no-baselines", action="store_true",
                     help="skip the CPU oracle, cuSPARSE and reference-GPU baselines")
     ap.add_argument("--no-sub", action="store_true",
@@ -1001,8 +1000,8 @@ def main():
                     "share_of_step": round(rec["ms"] / (ms * args.steps), 4)}
     call_alg = sum(4 * (n + 1) + 12 * nnz + 8 * (n + 1) + 12 * i["nnz_c"] for i in infos.values())
 
-    # per-call times of the three tasks (the Gram path gives the same C as
-    # A·Aᵀ; it is timed here beside the line, not inside the step)
+    # per-call times of the three tasks (AAtS gives the same C as A·Aᵀ; it is
+    # timed here beside the line, not inside the step)
     per_task_ms = {}
     for task in ("AA", "AAt", "AAtS"):
         ts = []

@@ -1,8 +1,8 @@
 /*
  * spgemm_b200.h — C ABI of the B200 (sm_100a) FP64 SpGEMM engine.
  *
- * Computes C = A·A, C = A·Aᵀ (plain) and C = A·Aᵀ through the symmetric Gram
- * path (upper triangle computed, lower triangle mirrored) for a square n×n CSR
+ * Computes C = A·A and C = A·Aᵀ (as "AAt" and, for callers of the reference's
+ * symmetric variant, as "AAtS": the same C, bit for bit) for a square n×n CSR
  * matrix A with int32 row pointers / column indices and FP64 values, on one GPU.
  *
  * The reference surface this replaces is the header-only engine
@@ -56,7 +56,7 @@ typedef enum spg_status {
 typedef enum spg_task {
   SPG_TASK_AA = 0,    /* C = A·A                                        ("AA")   */
   SPG_TASK_AAT = 1,   /* C = A·Aᵀ, Aᵀ built by the engine's transpose   ("AAt")  */
-  SPG_TASK_AATS = 2   /* C = A·Aᵀ via upper triangle + mirror           ("AAtS") */
+  SPG_TASK_AATS = 2   /* C = A·Aᵀ, the symmetric variant's name         ("AAtS") */
 } spg_task;
 
 /* Square CSR matrix on the device, borrowed (int32 row pointers: nnz < 2^31). */
@@ -164,7 +164,7 @@ typedef struct spg_plan_info {
   int64_t nnz_a;
   int64_t nnz_c;              /* exact, structural                              */
   int64_t products;           /* Σ_{(i,k)} nnz(B_k): A·A  Σ_k nnz(A_k)… (metric) */
-  int64_t products_computed;  /* products actually multiplied (AAtS: ~half)     */
+  int64_t products_computed;  /* products actually multiplied                   */
   int64_t max_row_products;
   int64_t max_row_nnz;
   int64_t heavy_rows;         /* rows on the heavy (CTA-per-row) path           */
@@ -228,7 +228,7 @@ spg_status spg_plan_get_info(const spg_plan* plan, spg_plan_info* info);
  * allocates per call, src/spgemm_engine.cuh:137-181). */
 spg_status spg_plan_workspace_bound(const spg_ctx* ctx, spg_task task, int32_t count,
                                     const spg_csr_dev* As, int32_t batched, int64_t* bytes);
-/* Numeric phase + in-row sort (+ mirror for AAtS) into caller-owned buffers:
+/* Numeric phase into caller-owned buffers:
  * C->rowptr (n+1), C->col / C->val (info.nnz_c).  Asynchronous on `stream`.
  * A plan fixes the structure only: a plan may be executed again after A's
  * values (not its pattern) changed, and uses the current values.  Executes of

@@ -528,7 +528,8 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   }
   {  // the pre-pass also validates A
     ProfScope ps(ctx, "plan/prepass", st);
-    TRY_CUDA(launch_prepass(p->A, p->B, p->f, p->lo, p->hi, st, ctx->d_status), "prepass");
+    TRY_CUDA(launch_prepass(p->A, p->B, p->f, p->lo, p->hi, st, ctx->d_status, kSmallCap),
+             "prepass");
   }
   RowArgs ra{};
   ra.A = p->A;
@@ -609,6 +610,14 @@ bool small_plan_eligible(const spg_ctx* ctx, spg_task task, const spg_csr_dev* A
   const spg_config& c = ctx->cfg;
   return c.small_max_nnz > 0 &&
          A->nnz <= c.small_max_nnz && A->n <= kSmallMaxN && !c.force_heavy;
+}
+
+// The heavy rows' classes as the one list that they are.
+void merge_heavy(int64_t* count) {
+  for (int c = 1; c < kHeavyClasses; ++c) {
+    count[kHeavyBin] += count[kHeavyBin + c];
+    count[kHeavyBin + c] = 0;
+  }
 }
 
 spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
@@ -769,6 +778,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     sym_count[b] = hp[b];
     sym_start[b] = b ? sym_start[b - 1] + sym_count[b - 1] : 0;
   }
+  merge_heavy(sym_count);
   // A row's blocks of 2^b columns are at most its blocks of 1024 columns times
   // 2^(10−b), or for b > 10 divided by 2^(b−10) plus two, so other widths need
   // no second readback
@@ -899,6 +909,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     p->num_count[b] = hp[b];
     p->num_start[b] = b ? p->num_start[b - 1] + p->num_count[b - 1] : 0;
   }
+  merge_heavy(p->num_count);
   const unsigned long long* sv = (const unsigned long long*)(hp + kBinWork);
   p->nnz_c = (int64_t)sv[4];
   p->info.nnz_c = p->nnz_c;

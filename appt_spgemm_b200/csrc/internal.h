@@ -34,23 +34,26 @@ constexpr int kNumTableBins = kMaxTableLog2 - kMinTableLog2 + 1;  // 11
 // warp row over a bitmap of 2^(kDenseMinLog2W + b) words of its column span.
 constexpr int kEmptyBin = 0;
 constexpr int kHeavyBin = kNumTableBins + 1;  // 12
+// Heavy rows are listed in kHeavyClasses bins from kHeavyBin on, by products (2^20
+// and more, 2^18, … 2^12, the rest): one list, the longest rows first.
+constexpr int kHeavyClasses = 6;
 constexpr int kDenseMinLog2W = 8;
 constexpr int kDenseMaxLog2W = 11;
-constexpr int kDenseBin0 = kHeavyBin + 1;     // 13
+constexpr int kDenseBin0 = kHeavyBin + kHeavyClasses;  // 18
 // kSortBin0 + b = sorted row (numeric phase only) of up to sort_bin_products(b)
 // products.
 constexpr int kSortBins = 8;
-constexpr int kSortBin0 = kDenseBin0 + kDenseMaxLog2W - kDenseMinLog2W + 1;  // 17
+constexpr int kSortBin0 = kDenseBin0 + kDenseMaxLog2W - kDenseMinLog2W + 1;  // 22
 // kRunBin0 + t = first row of a run of shifted rows (numeric phase only), teams
 // of 2^t warps.
 constexpr int kRunBins = 4;
-constexpr int kRunBin0 = kSortBin0 + kSortBins;  // 25
+constexpr int kRunBin0 = kSortBin0 + kSortBins;  // 30
 // kNarrowBin0 + 2 · w + h = narrow row of up to kNarrowMin << w columns, a warp
 // (h = 1) or half of one per row.
 constexpr int kNarrowBins = 8;
 constexpr int kNarrowMin = 128;
-constexpr int kNarrowBin0 = kRunBin0 + kRunBins;  // 29
-constexpr int kNumBins = kNarrowBin0 + kNarrowBins;  // 37
+constexpr int kNarrowBin0 = kRunBin0 + kRunBins;  // 34
+constexpr int kNumBins = kNarrowBin0 + kNarrowBins;  // 42
 constexpr int kDenseVals = 256;  // entries of a bitmap-path row (numeric)
 
 }  // namespace spg

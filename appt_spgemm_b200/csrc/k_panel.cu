@@ -75,48 +75,46 @@ __global__ void k_panel_bounds(MatView B, int pan_log2, int npan, int32_t* __res
   }
 }
 
-// One CTA: the rows that take panels, largest product counts first (by powers
-// of two, so that a hub row's tasks start early and none of them is left to
-// the end), and their task offsets; off[nrows] is the number of tasks.
-constexpr int kOrderThreads = 1024;
-__global__ void __launch_bounds__(kOrderThreads) k_panel_order(HeavyArgs h,
-                                                               int32_t* __restrict__ order,
-                                                               int64_t* __restrict__ off) {
-  __shared__ int start[64];
+// One CTA: the task offsets of the rows, a task per panel of those that take
+// panels; off[nrows] is the number of tasks.  The rows are listed by product
+// count, largest first, so a hub row's tasks start early and none of them is
+// left to the end.
+constexpr int kOffsetThreads = 1024, kOffsetRows = 8;
+__global__ void __launch_bounds__(kOffsetThreads) k_panel_offsets(HeavyArgs h,
+                                                                  int64_t* __restrict__ off) {
   __shared__ int scratch[33];
   __shared__ long long carry;
   const int tid = threadIdx.x, nrows = h.r.nrows;
-  if (tid < 64) start[tid] = 0;
+  if (tid == 0) carry = 0;
   __syncthreads();
-  for (int r = tid; r < nrows; r += kOrderThreads)
-    atomicAdd(&start[min(63, __clzll(h.f[h.r.rows[r]]))], 1);
-  __syncthreads();
-  if (tid == 0) {
-    int run = 0;
-    for (int c = 0; c < 64; ++c) {
-      const int n = start[c];
-      start[c] = run;
-      run += n;
+  for (int r0 = 0; r0 < nrows; r0 += kOffsetThreads * kOffsetRows) {
+    // each step's loads issued together (rows past the end count the last one)
+    int n[kOffsetRows], lo[kOffsetRows], hi[kOffsetRows], len[kOffsetRows], sum = 0;
+    int64_t f[kOffsetRows];
+#pragma unroll
+    for (int u = 0; u < kOffsetRows; ++u)
+      n[u] = h.r.rows[min(r0 + tid * kOffsetRows + u, nrows - 1)];
+#pragma unroll
+    for (int u = 0; u < kOffsetRows; ++u) {
+      lo[u] = h.lo[n[u]];
+      hi[u] = h.hi[n[u]];
+      f[u] = h.f[n[u]];
+      len[u] = h.r.A.rowptr[n[u] + 1] - h.r.A.rowptr[n[u]];
     }
-    carry = 0;
-  }
-  __syncthreads();
-  for (int r = tid; r < nrows; r += kOrderThreads) {
-    const int row = h.r.rows[r];
-    order[atomicAdd(&start[min(63, __clzll(h.f[row]))], 1)] = row;
-  }
-  __syncthreads();
-  for (int r0 = 0; r0 < nrows; r0 += kOrderThreads) {
-    const int r = r0 + tid;
-    int n = 0;
-    if (r < nrows) {
-      const int row = order[r];
-      const int2 p = row_panels(h, row);
-      if (heavy_row_paneled(h, row)) n = p.y - p.x;
+#pragma unroll
+    for (int u = 0; u < kOffsetRows; ++u) {
+      const bool takes = r0 + tid * kOffsetRows + u < nrows && paneled_row(f[u], len[u], lo[u], hi[u]);
+      n[u] = takes ? (hi[u] >> h.pan_log2) - (lo[u] >> h.pan_log2) + 1 : 0;
+      sum += n[u];
     }
     int tot;
-    const int ex = block_exclusive_scan(n, scratch, &tot);
-    if (r < nrows) off[r] = carry + ex;
+    long long at = carry + block_exclusive_scan(sum, scratch, &tot);
+#pragma unroll
+    for (int u = 0; u < kOffsetRows; ++u) {
+      const int r = r0 + tid * kOffsetRows + u;
+      if (r < nrows) off[r] = at;
+      at += n[u];
+    }
     __syncthreads();
     if (tid == 0) carry += tot;
     __syncthreads();
@@ -138,9 +136,7 @@ __device__ __forceinline__ int task_row(const int64_t* off, int nrows, int64_t t
   return lo;
 }
 
-__global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h,
-                                                   const int32_t* __restrict__ order,
-                                                   const int64_t* __restrict__ off) {
+__global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h, const int64_t* __restrict__ off) {
   extern __shared__ __align__(16) unsigned char smem[];
   const RowArgs& a = h.r;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -157,7 +153,7 @@ __global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h,
     t = __shfl_sync(kFull, t, 0);
     if (t >= total) break;
     const int r = task_row(off, a.nrows, t);
-    const int row = order[r];
+    const int row = a.rows[r];
     const int2 pr = row_panels(h, row);
     const int p = pr.x + (int)(t - off[r]);
     const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
@@ -320,8 +316,7 @@ __global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h,
 static int64_t align256(int64_t b) { return (b + 255) & ~(int64_t)255; }
 
 int64_t panel_workspace(int64_t n, int npan, int64_t nrows, bool table) {
-  return (table ? align256(4 * n * (npan + 1)) : 0) + align256(4 * nrows) +
-         align256(8 * (nrows + 1)) + 256;
+  return (table ? align256(4 * n * (npan + 1)) : 0) + align256(8 * (nrows + 1)) + 256;
 }
 
 cudaError_t launch_panels(HeavyArgs& h, void* workspace, bool table, int num_sms,
@@ -331,8 +326,6 @@ cudaError_t launch_panels(HeavyArgs& h, void* workspace, bool table, int num_sms
   const int64_t nptr = (int64_t)h.r.B.n * (h.npan + 1);
   int32_t* ptr = table ? (int32_t*)w : nullptr;
   if (table) w += align256(4 * nptr);
-  int32_t* order = (int32_t*)w;
-  w += align256(4 * (int64_t)h.r.nrows);
   int64_t* off = (int64_t*)w;
   w += align256(8 * ((int64_t)h.r.nrows + 1));
   h.ptr = ptr;
@@ -344,7 +337,7 @@ cudaError_t launch_panels(HeavyArgs& h, void* workspace, bool table, int num_sms
     k_panel_bounds<<<(unsigned)blocks, 256, 0, s>>>(h.r.B, h.pan_log2, h.npan, ptr);
     SPG_COUNT_LAUNCH();
   }
-  k_panel_order<<<1, kOrderThreads, 0, s>>>(h, order, off);
+  k_panel_offsets<<<1, kOffsetThreads, 0, s>>>(h, off);
   SPG_COUNT_LAUNCH();
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
 
@@ -361,7 +354,7 @@ cudaError_t launch_panels(HeavyArgs& h, void* workspace, bool table, int num_sms
   if (per_sm < 1) per_sm = 1;
   const int64_t most = (int64_t)h.r.nrows * h.npan;  // tasks
   const int64_t grid = std::min<int64_t>((int64_t)per_sm * num_sms, (most + warps - 1) / warps);
-  kernel<<<(unsigned)grid, warps * 32, bytes, s>>>(h, order, off);
+  kernel<<<(unsigned)grid, warps * 32, bytes, s>>>(h, off);
   SPG_COUNT_LAUNCH();
   return cudaGetLastError();
 }

@@ -206,13 +206,15 @@ __global__ void __launch_bounds__(256, 5) k_hash_w32(RowArgs a) {
   double* vals = (double*)base_p;
   int* keys = (int*)(base_p + (NUMERIC ? (size_t)T * 8 : 0));
 
+  // (a matrix with a row beyond the one-readback plan's table, as the pre-pass
+  // found, is planned again: nothing to count)
+  if (!NUMERIC && a.fsmall && (*a.status & DEV_ERR_SMALL_CAP)) return;
   for (int r = blockIdx.x * nw + w; r < a.nrows; r += gridDim.x * nw) {
     const int row = a.rows ? a.rows[r] : r;
     if (!NUMERIC && a.fsmall) {
       const int64_t fr = a.fsmall[row];
       if (fr < 0 || fr > a.fcap) {
         if (lane == 0) {
-          if (fr > a.fcap) report(a.status, DEV_ERR_SMALL_CAP);
           a.rownnz[row] = 0;
         }
         continue;

@@ -24,14 +24,17 @@ cudaError_t launch_validate(const MatView& A, uint32_t* status, cudaStream_t s);
 // Per row i of C = A·B: products f_i = Σ_{k∈A_i} nnz(B_k) and the column span
 // [lo_i, hi_i] of the output row (B rows sorted).  Rows with f_i = 0 get
 // lo = INT_MAX, hi = -1; rows that meet an index out of range f_i = −1.  With
-// `status`, A is validated in the same pass (launch_validate's checks).
+// `status`, A is validated in the same pass (launch_validate's checks), and a row
+// of more than fcap products reports DEV_ERR_SMALL_CAP.
 cudaError_t launch_prepass(const MatView& A, const MatView& B, int64_t* f, int32_t* lo,
-                           int32_t* hi, cudaStream_t s, uint32_t* status = nullptr);
+                           int32_t* hi, cudaStream_t s, uint32_t* status = nullptr,
+                           int64_t fcap = INT64_MAX);
 
 // Sorted rows: the fewest and the most products, the most products per two entries.
 constexpr int64_t kSortMinProducts = 48;
 constexpr int64_t kSortMaxProducts = 4096;
 constexpr int64_t kSortMaxMerge2 = 3;
+constexpr int64_t kSortMaxMerge2Large = 6;  // beyond the warp kernels' largest table
 
 // Paneled rows: the fewest products, the narrowest span, the fewest products per
 // 1024 columns of it and, up to kWarpRowMaxProducts products, the fewest per
@@ -155,9 +158,17 @@ __host__ __device__ __forceinline__ int sort_bin_products(int b) {
 
 // A row of f products and m entries whose columns span `span`: sorted rather
 // than hashed?  The words (column − lo) << log2 F | place must fit 32 bits.
-__host__ __device__ __forceinline__ bool sorted_row(int64_t f, int64_t m, int64_t span) {
-  return f >= kSortMinProducts && f <= kSortMaxProducts && 2 * f <= kSortMaxMerge2 * m &&
+__host__ __device__ __forceinline__ bool sorted_row(int64_t f, int64_t m, int64_t span,
+                                                    int64_t merge2 = kSortMaxMerge2) {
+  return f >= kSortMinProducts && f <= kSortMaxProducts && 2 * f <= merge2 * m &&
          span <= ((int64_t)1 << (32 - ceil_log2_64(f < 128 ? 128 : f)));
+}
+
+// Class of a heavy row's products: 0 (2^20 and more) … kHeavyClasses − 1.
+__host__ __device__ __forceinline__ int heavy_class(int64_t f) {
+  int c = 0;
+  while (c < kHeavyClasses - 1 && f < (int64_t)1 << (20 - 2 * c)) ++c;
+  return c;
 }
 
 // A row of f products from `len` entries of A over columns [lo, hi]: cut into
@@ -200,7 +211,8 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
   if (s.force_heavy || (s.panels && paneled_row(s.f[i], s.arowptr[i + 1] - s.arowptr[i], s.lo[i], s.hi[i]))) return kHeavyBin;
   int lg = table_log2(size, s.load_pct);
   if (s.mode == 1 && s.sort_rows && lg <= s.max_log2 &&
-      sorted_row(s.f[i], size, (int64_t)s.hi[i] - s.lo[i] + 1)) {
+      sorted_row(s.f[i], size, (int64_t)s.hi[i] - s.lo[i] + 1,
+                 lg > s.short_max_log2 ? kSortMaxMerge2Large : kSortMaxMerge2)) {
     int b = 0;
     while (sort_bin_products(b) < s.f[i]) ++b;
     return kSortBin0 + b;
@@ -228,7 +240,7 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
   return lg - kMinTableLog2 + 1;
 }
 
-constexpr int kBinRowsPerBlock = 1024;  // rows per block of the binning kernels
+constexpr int kBinRowsPerBlock = 256;  // rows per block of the binning kernels
 
 // Binning: the rows of each bin listed one bin after another (in row order within
 // blocks of kBinRowsPerBlock rows).

@@ -545,27 +545,30 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   ra.fcap = kSmallCap;
   if (n > 0) {
     ProfScope ps(ctx, "sym/small", st);
-    TRY_CUDA(launch_hash_w32(kSmallSymLog2, false, ra, ctx->num_sms, st), "symbolic");
+    // a byte per column from 1024 columns on, then (beyond 8192) a bit: the table
+    // is as large as n needs, so that small matrices run in one wave
+    int lg = kSmallSymLog2;
+    while (lg > 8 && n <= 2 << lg) --lg;
+    TRY_CUDA(launch_hash_w32(lg, false, ra, ctx->num_sms, st), "symbolic");
   }
   {
     ProfScope ps(ctx, "plan/scan", st);
     TRY_CUDA(launch_row_pointers(p->rownnz, nullptr, p->f, p->lo, p->hi, n, p->rowptr, stats,
-                                 w + o_scan, st), "row pointer scan");
+                                 ctx->d_status, w + o_scan, st), "row pointer scan");
   }
   int64_t* hp = ctx->h_pin;
-  TRY_CUDA(cudaMemcpyAsync(hp, ctx->d_status, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st),
-           "readback");
-  TRY_CUDA(cudaMemcpyAsync(hp + 1, stats, sizeof(int64_t) * kRowStats, cudaMemcpyDeviceToHost, st),
+  TRY_CUDA(cudaMemcpyAsync(hp, stats, sizeof(int64_t) * kRowStats, cudaMemcpyDeviceToHost, st),
            "readback");
   TRY_CUDA(cudaStreamSynchronize(st), "plan sync");
-  const uint32_t bits = *(const uint32_t*)hp;
+  const uint32_t* words = (const uint32_t*)(hp + 5);  // verdict, asymmetry
+  const uint32_t bits = words[0];
   if (bits & DEV_ERR_INVALID_CSR) return status_from_bits(DEV_ERR_INVALID_CSR);
   if (bits & DEV_ERR_SMALL_CAP) {
     *fallback = true;
     return SPG_OK;
   }
   TRY(status_from_bits(bits));
-  const unsigned long long* sv = (const unsigned long long*)(hp + 1);
+  const unsigned long long* sv = (const unsigned long long*)hp;
   p->nnz_c = (int64_t)sv[4];
   p->info.nnz_c = p->nnz_c;
   p->info.products = (int64_t)sv[0];
@@ -574,7 +577,7 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   p->info.max_row_nnz = (int64_t)sv[2];
   p->info.heavy_rows = 0;
   p->info.bins_used = 1;
-  p->info.symmetric_pattern = p->task == SPG_TASK_AATS && ((const uint32_t*)hp)[1] == 0;
+  p->info.symmetric_pattern = p->task == SPG_TASK_AATS && words[1] == 0;
   // numeric table: the exact largest row at the numeric load, 16 to 2048
   // slots; tables below 2048 slots run rows on lane groups sized to B's mean
   // row length (several rows per warp), 2048 a warp per row
@@ -886,7 +889,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   {
     ProfScope ps(ctx, "plan/scan", st);
     TRY_CUDA(launch_row_pointers(p->rownnz, pre.lead, p->f, p->lo, p->hi, n, p->rowptr, stats,
-                                 scan_tmp, st), "row pointer scan");
+                                 ctx->d_status, scan_tmp, st), "row pointer scan");
   }
   // numeric binning by exact counts, stats; host sync #2 (nnz(C))
   TRY(palloc(p, &p->rows_num, n));
@@ -901,10 +904,8 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   constexpr int kBack = kBinWork + kRowStats;
   TRY_CUDA(cudaMemcpyAsync(hp, work_num, sizeof(int64_t) * kBack, cudaMemcpyDeviceToHost, st),
            "readback");
-  TRY_CUDA(cudaMemcpyAsync(hp + kBack, ctx->d_status, sizeof(uint32_t),
-                           cudaMemcpyDeviceToHost, st), "readback");
   TRY_CUDA(cudaStreamSynchronize(st), "plan sync");
-  TRY(status_from_bits(*(uint32_t*)(hp + kBack)));
+  TRY(status_from_bits(*(uint32_t*)(hp + kBinWork + 5)));
   for (int b = 0; b < kNumBins; ++b) {
     p->num_count[b] = hp[b];
     p->num_start[b] = b ? p->num_start[b - 1] + p->num_count[b - 1] : 0;

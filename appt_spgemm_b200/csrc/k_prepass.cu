@@ -349,7 +349,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_single(const int32_t* __r
 // gathers the statistics; in the second each tile sums the tiles before it.
 // (A scan of three launches, the run counts and the statistics as launches of
 // their own took 58 against 19 µs on a million rows.)
-//   stats: Σ products, max products, max row count, max span, Σ row counts
+//   stats: Σ products, max products, max row count, max span, Σ row counts, and
+//     the two device status words, so that one copy brings a plan's verdict
 struct RowStats {
   unsigned long long sf = 0, mf = 0, mc = 0, ms = 0;
   __device__ __forceinline__ void add(unsigned long long f, int c, int lo, int hi) {
@@ -359,8 +360,8 @@ struct RowStats {
     const unsigned long long span = hi >= lo ? (unsigned long long)((long long)hi - lo + 1) : 0;
     ms = span > ms ? span : ms;
   }
-  // per warp, then one atomic each per CTA
-  __device__ __forceinline__ void store(unsigned long long* stats) {
+  // per warp, then one atomic each per CTA (of one CTA: plain stores)
+  __device__ __forceinline__ void store(unsigned long long* stats, bool single) {
     __shared__ unsigned long long acc[4];
     if (threadIdx.x < 4) acc[threadIdx.x] = 0;
     __syncthreads();
@@ -380,7 +381,9 @@ struct RowStats {
       atomicMax(&acc[3], ms);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (single) {
+      if (threadIdx.x < 4) stats[threadIdx.x] = acc[threadIdx.x];
+    } else if (threadIdx.x == 0) {
       atomicAdd(&stats[0], acc[0]);
       atomicMax(&stats[1], acc[1]);
       atomicMax(&stats[2], acc[2]);
@@ -394,7 +397,7 @@ __global__ void __launch_bounds__(kScanThreads) k_count_tiles(
     int32_t* cnt, const uint8_t* __restrict__ lead, const int64_t* __restrict__ f,
     const int32_t* __restrict__ lo, const int32_t* __restrict__ hi, int64_t n,
     int64_t* __restrict__ rowptr, long long* __restrict__ tile_sums,
-    unsigned long long* __restrict__ stats) {
+    unsigned long long* __restrict__ stats, const uint32_t* __restrict__ status) {
   __shared__ long long scratch[32];
   const int64_t tile = (int64_t)blockIdx.x * kScanTile;
   RowStats st;
@@ -402,15 +405,33 @@ __global__ void __launch_bounds__(kScanThreads) k_count_tiles(
     const int64_t base = tile + (int64_t)threadIdx.x * kScanItems;
     int32_t v[kScanItems];
     long long s = 0;
+    if (!lead && base + kScanItems <= n) {  // (the arrays are 16-byte aligned)
+      int32_t l[kScanItems], h[kScanItems];
+      int64_t p[kScanItems];
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      const int64_t i = base + k;
-      v[k] = 0;
-      if (i >= n) continue;
-      v[k] = cnt[lead && lead[i] ? i - lead[i] : i];
-      if (lead && lead[i]) cnt[i] = v[k];
-      s += v[k];
-      st.add((unsigned long long)f[i], v[k], lo[i], hi[i]);
+      for (int k = 0; k < kScanItems; k += 4) {
+        *(int4*)(v + k) = *(const int4*)(cnt + base + k);
+        *(int4*)(l + k) = *(const int4*)(lo + base + k);
+        *(int4*)(h + k) = *(const int4*)(hi + base + k);
+        *(longlong2*)(p + k) = *(const longlong2*)(f + base + k);
+        *(longlong2*)(p + k + 2) = *(const longlong2*)(f + base + k + 2);
+      }
+#pragma unroll
+      for (int k = 0; k < kScanItems; ++k) {
+        s += v[k];
+        st.add((unsigned long long)p[k], v[k], l[k], h[k]);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kScanItems; ++k) {
+        const int64_t i = base + k;
+        v[k] = 0;
+        if (i >= n) continue;
+        v[k] = cnt[lead && lead[i] ? i - lead[i] : i];
+        if (lead && lead[i]) cnt[i] = v[k];
+        s += v[k];
+        st.add((unsigned long long)f[i], v[k], lo[i], hi[i]);
+      }
     }
     long long tot;
     long long run = block_exclusive_scan64(s, scratch, &tot);
@@ -422,6 +443,7 @@ __global__ void __launch_bounds__(kScanThreads) k_count_tiles(
     if (threadIdx.x == 0) {
       rowptr[n] = tot;
       stats[4] = (unsigned long long)tot;
+      stats[5] = status[0] | (unsigned long long)status[1] << 32;
     }
   } else {
     long long s = 0;
@@ -438,14 +460,15 @@ __global__ void __launch_bounds__(kScanThreads) k_count_tiles(
     s = block_sum64(s, scratch);
     if (threadIdx.x == 0) tile_sums[blockIdx.x] = s;
   }
-  st.store(stats);
+  st.store(stats, SINGLE);
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_count_apply(const int32_t* __restrict__ cnt,
                                                               int64_t n, int64_t ntiles,
                                                               const long long* __restrict__ tiles,
                                                               int64_t* __restrict__ rowptr,
-                                                              unsigned long long* stats) {
+                                                              unsigned long long* stats,
+                                                              const uint32_t* __restrict__ status) {
   __shared__ long long scratch[32];
   long long before = 0;
   for (int64_t t = threadIdx.x; t < blockIdx.x; t += kScanThreads) before += tiles[t];
@@ -468,6 +491,7 @@ __global__ void __launch_bounds__(kScanThreads) k_count_apply(const int32_t* __r
   if (blockIdx.x == ntiles - 1 && threadIdx.x == 0) {
     rowptr[n] = before + tot;
     stats[4] = (unsigned long long)(before + tot);
+    stats[5] = status[0] | (unsigned long long)status[1] << 32;
   }
 }
 
@@ -477,26 +501,35 @@ constexpr int64_t kMaxCountTiles = 4096;
 
 cudaError_t launch_row_pointers(int32_t* cnt, const uint8_t* lead, const int64_t* f,
                                 const int32_t* lo, const int32_t* hi, int64_t n, int64_t* rowptr,
-                                unsigned long long* stats, void* tmp, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(stats, 0, sizeof(unsigned long long) * kRowStats, s);
-  if (e != cudaSuccess) return e;
-  if (n <= 0) return cudaMemsetAsync(rowptr, 0, sizeof(int64_t), s);
+                                unsigned long long* stats, const uint32_t* status, void* tmp,
+                                cudaStream_t s) {
   long long* tiles = (long long*)tmp;
   const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
   if (ntiles == 1) {
-    k_count_tiles<true><<<1, kScanThreads, 0, s>>>(cnt, lead, f, lo, hi, n, rowptr, tiles, stats);
+    k_count_tiles<true><<<1, kScanThreads, 0, s>>>(cnt, lead, f, lo, hi, n, rowptr, tiles, stats,
+                                                   status);
     SPG_COUNT_LAUNCH();
     return cudaGetLastError();
   }
+  cudaError_t e = cudaMemsetAsync(stats, 0, sizeof(unsigned long long) * kRowStats, s);
+  if (e != cudaSuccess) return e;
+  if (n <= 0) {
+    e = cudaMemcpyAsync(stats + 5, status, 2 * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
+    return e != cudaSuccess ? e : cudaMemsetAsync(rowptr, 0, sizeof(int64_t), s);
+  }
   k_count_tiles<false><<<(unsigned)ntiles, kScanThreads, 0, s>>>(cnt, lead, f, lo, hi, n, rowptr,
-                                                                 tiles, stats);
+                                                                 tiles, stats, status);
   SPG_COUNT_LAUNCH();
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (ntiles > kMaxCountTiles) {
     if ((e = launch_scan_i32_i64(cnt, rowptr, n, tmp, s)) != cudaSuccess) return e;
-    return cudaMemcpyAsync(stats + 4, rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToDevice, s);
+    e = cudaMemcpyAsync(stats + 4, rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToDevice, s);
+    return e != cudaSuccess ? e
+                            : cudaMemcpyAsync(stats + 5, status, 2 * sizeof(uint32_t),
+                                              cudaMemcpyDeviceToDevice, s);
   }
-  k_count_apply<<<(unsigned)ntiles, kScanThreads, 0, s>>>(cnt, n, ntiles, tiles, rowptr, stats);
+  k_count_apply<<<(unsigned)ntiles, kScanThreads, 0, s>>>(cnt, n, ntiles, tiles, rowptr, stats,
+                                                          status);
   SPG_COUNT_LAUNCH();
   return cudaGetLastError();
 }

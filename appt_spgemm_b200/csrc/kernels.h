@@ -563,11 +563,13 @@ cudaError_t launch_describe(const MatView& A, const int32_t* colcount, DescAccum
                             cudaStream_t s);
 // Row pointers of C from the row counts (with `lead`, a run's rows take its
 // first row's count first), and kRowStats statistics: Σ products, max products,
-// max row count, max column span, nnz(C).  tmp: scan_tmp_bytes(n).
-constexpr int kRowStats = 5;
+// max row count, max column span, nnz(C), and the device status words as they are
+// then.  cnt, f, lo, hi: 16-byte aligned.  tmp: scan_tmp_bytes(n).
+constexpr int kRowStats = 6;
 cudaError_t launch_row_pointers(int32_t* cnt, const uint8_t* lead, const int64_t* f,
                                 const int32_t* lo, const int32_t* hi, int64_t n, int64_t* rowptr,
-                                unsigned long long* stats, void* tmp, cudaStream_t s);
+                                unsigned long long* stats, const uint32_t* status, void* tmp,
+                                cudaStream_t s);
 cudaError_t launch_col_count(const MatView& A, int32_t* cnt, cudaStream_t s);
 
 }  // namespace spg

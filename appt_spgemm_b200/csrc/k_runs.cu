@@ -21,11 +21,12 @@
 //    order, so the values are those of the other kernels, bit for bit.
 // 27-point stencil 96³, A·A: numeric phase 2.99 -> 1.24 ms (runs 1.11 ms, the
 // rows at the grid's faces in the hash kernels), symbolic 1.04 -> 0.07 ms, call
-// 4.51 -> 1.92 ms; 5-point grid 1009²: call 1.27 -> 0.63 ms.  The run kernel
+// 4.51 -> 1.88 ms; 5-point grid 1009²: call 1.27 -> 0.38 ms.  The run kernel
 // issues on 42% of cycles and moves shared-memory wavefronts on 50% (two 64-bit
 // loads a product), with two CTAs of 16 warps per SM in its 109 KB: latency is
 // what is left.  Measured and not kept: two entries' sums at a time 1.16 ms,
-// entries drawn by list length 1.16 ms, neighbouring runs to one CTA 1.16 ms.
+// entries drawn by list length 1.16 ms, neighbouring runs to one CTA 1.16 ms;
+// the entries shared out by list length, or 16 warps a team (32 per SM): no change.
 #include <climits>
 
 #include "kernels.h"
@@ -35,21 +36,33 @@ namespace spg {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kRunThreads = 256;
-constexpr int kRunWarps = kRunThreads / 32;
 constexpr int kRunOut = 8;                    // output entries a warp stages at a time
 constexpr int kStageRow = 33;                 // doubles between staged entries (32 rows)
-constexpr size_t kStageBytes = (size_t)kRunWarps * kRunOut * kStageRow * 8;
-constexpr int kMaxList = 2 * kRunMaxProducts;  // lists start at even places
 constexpr int kMaxLen = 126;                  // entries of A's row
 
-// Team buffers (also the bitmap while the places are found), the staging area
-// (also the products then), the lists, their starts, the output columns and
-// the products' columns: two CTAs per SM with the static arrays.
-constexpr size_t kRunSmem = (size_t)kRunBuffer * 8 + kStageBytes + (size_t)kMaxList * 4 +
-                            (size_t)kRunMaxProducts * 12;
-static_assert(kStageBytes >= (size_t)kRunMaxProducts * 10, "products fit the staging area");
-static_assert((size_t)kRunBuffer * 8 >= (size_t)kRunMaxSpan / 32 * 5 + 64, "bitmap fits");
+// A launch's CTA by team size: threads, and the limits of its runs' rows.  The
+// runs of few entries a row (teams of one warp) have small CTAs, six per SM
+// instead of two: a run's own steps (its entries, its rows of B, the check of
+// its columns) are a chain of loads that only other CTAs hide.  5-point grid
+// 1009²: 145 -> 127 µs.
+template <int T>
+struct RunShape {
+  static constexpr int kThreads = T == 1 ? 128 : 256;
+  static constexpr int kWarps = kThreads / 32, kTeams = kWarps / T;
+  static constexpr int kTeamBuffer = T == 1 ? kRunSmallBuffer : kRunBuffer * T / 8;  // doubles
+  static constexpr int kProducts = T == 1 ? kRunSmallProducts : kRunMaxProducts;
+  static constexpr int kSpan = T == 1 ? kRunSmallSpan : kRunMaxSpan;
+  static constexpr int kList = 2 * kProducts;  // lists start at even places
+  static constexpr size_t kBufferBytes = (size_t)kTeams * kTeamBuffer * 8;
+  static constexpr size_t kStageBytes = (size_t)kWarps * kRunOut * kStageRow * 8;
+  // team buffers (also the bitmap while the places are found), the staging area
+  // (also the products then), the lists, their starts, the output columns and the
+  // products' columns
+  static constexpr size_t kSmem = kBufferBytes + kStageBytes + (size_t)kList * 4 +
+                                  (size_t)kProducts * 12;
+  static_assert(kStageBytes >= (size_t)kProducts * 10, "products fit the staging area");
+  static_assert(kBufferBytes >= (size_t)kSpan / 32 * 5 + 64, "bitmap fits");
+};
 
 __device__ __forceinline__ void copy_async8(double* dst, const double* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
@@ -85,8 +98,10 @@ struct RowGroup {
 };
 
 template <int T>  // warps per team of 32 rows
-__global__ void __launch_bounds__(kRunThreads, 2) k_runs(RowArgs a) {
-  constexpr int kTeams = kRunWarps / T, kTeamThreads = T * 32;
+__global__ void __launch_bounds__(RunShape<T>::kThreads, T == 1 ? 5 : 2) k_runs(RowArgs a) {
+  using S = RunShape<T>;
+  constexpr int kRunThreads = S::kThreads, kRunWarps = S::kWarps, kTeams = S::kTeams;
+  constexpr int kTeamThreads = T * 32, kMaxProducts = S::kProducts;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ RowGroup groups[kMaxLen];
   __shared__ int t_src[kMaxLen], t_rel[kMaxLen];
@@ -94,20 +109,20 @@ __global__ void __launch_bounds__(kRunThreads, 2) k_runs(RowArgs a) {
   __shared__ int scratch[33];
   __shared__ int s_groups, s_distinct, s_stride;
   double* buffer = (double*)smem;
-  double* stage_all = buffer + kRunBuffer;
-  uint32_t* list = (uint32_t*)((unsigned char*)stage_all + kStageBytes);
-  uint32_t* start = list + kMaxList;  // an output entry's first place << 8 | products
-  int* out_col = (int*)(start + kRunMaxProducts);  // its column, from the row's index
-  int* prod_col = out_col + kRunMaxProducts;       // the products' columns, likewise
+  double* stage_all = buffer + kTeams * S::kTeamBuffer;
+  uint32_t* list = (uint32_t*)((unsigned char*)stage_all + S::kStageBytes);
+  uint32_t* start = list + S::kList;  // an output entry's first place << 8 | products
+  int* out_col = (int*)(start + kMaxProducts);  // its column, from the row's index
+  int* prod_col = out_col + kMaxProducts;       // the products' columns, likewise
   // while the places are found
   uint32_t* bitmap = (uint32_t*)buffer;
   uint32_t* desc = (uint32_t*)stage_all;  // per product: where its operands will lie
-  int* cur = (int*)(desc + kRunMaxProducts);
-  uint16_t* rank = (uint16_t*)(cur + kRunMaxProducts);
+  int* cur = (int*)(desc + kMaxProducts);
+  uint16_t* rank = (uint16_t*)(cur + kMaxProducts);
 
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int team = wid / T, tw = wid % T, team_tid = tid % kTeamThreads;
-  double* buf = buffer + (size_t)team * (kRunBuffer / kTeams);
+  double* buf = buffer + (size_t)team * S::kTeamBuffer;
   double* stage = stage_all + (size_t)wid * kRunOut * kStageRow;
   int have_len = -1, have_m = 0;  // the lists at hand are of a row of this many entries
 
@@ -122,7 +137,7 @@ __global__ void __launch_bounds__(kRunThreads, 2) k_runs(RowArgs a) {
     const int stride_a = len_a | 1;
     // (what the pre-pass has checked; a plan whose structure was changed since
     // must not write past the arrays)
-    if (len_a > kMaxLen || m > kRunMaxProducts || span > kRunMaxSpan) {
+    if (len_a > kMaxLen || m > kMaxProducts || span > S::kSpan) {
       if (tid == 0) report(a.status, DEV_ERR_OVERFLOW);
       continue;
     }
@@ -215,7 +230,7 @@ __global__ void __launch_bounds__(kRunThreads, 2) k_runs(RowArgs a) {
           ++groups[n - 1].rows;
           t_first[t] = (uint16_t)e;
           e += t_len[t];
-          if (off > kRunBuffer / kTeams || e > kRunMaxProducts) {  // as above
+          if (off > S::kTeamBuffer || e > kMaxProducts) {  // as above
             n = -1;
             break;
           }
@@ -378,19 +393,21 @@ __global__ void __launch_bounds__(kRunThreads, 2) k_runs(RowArgs a) {
 template <int T>
 cudaError_t launch_runs_t(const RowArgs& a, int num_sms, cudaStream_t s) {
   auto kernel = k_runs<T>;
+  constexpr int kThreads = RunShape<T>::kThreads;
+  constexpr size_t kSmem = RunShape<T>::kSmem;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kRunSmem);
+                                       (int)kSmem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                            cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kRunThreads, kRunSmem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, kSmem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   int64_t grid = (int64_t)per_sm * num_sms;
   if (grid > a.nrows) grid = a.nrows;
-  kernel<<<(unsigned)grid, kRunThreads, kRunSmem, s>>>(a);
+  kernel<<<(unsigned)grid, kThreads, kSmem, s>>>(a);
   SPG_COUNT_LAUNCH();
   return cudaGetLastError();
 }
@@ -477,6 +494,7 @@ constexpr int kRowsAhead = 4;      // rows whose loads a group has in flight tog
 // rows flagged}.  Bound by the latency of entry -> row of B, hence four rows of
 // a group at a time where none is longer than the group.
 constexpr int kRunBlock = 256;
+constexpr int kShortLanes = 8;  // lanes per row of the matrices that take k_prepass_short
 __global__ void __launch_bounds__(256) k_prepass_rows(
     MatView A, int32_t n_b, const int4* __restrict__ info, int G, int rows,
     int64_t* __restrict__ f, int32_t* __restrict__ lo, int32_t* __restrict__ hi,
@@ -538,8 +556,12 @@ __global__ void __launch_bounds__(256) k_prepass_rows(
         const int32_t p = s[u] + g.lane;
         const bool in = g.lane < len[u];
         k[u] = in ? A.col[p] : -1;
-        before[u] = in && g.lane > 0 ? A.col[p - 1] : -1;
         above[u] = in && candidate[u] ? A.col[p - len[u]] : -2;
+      }
+#pragma unroll
+      for (int u = 0; u < kRowsAhead; ++u) {
+        before[u] = __shfl_up_sync(kFull, k[u], 1);
+        if (g.lane == 0) before[u] = -1;
       }
 #pragma unroll
       for (int u = 0; u < kRowsAhead; ++u)
@@ -588,6 +610,92 @@ __global__ void __launch_bounds__(256) k_prepass_rows(
   if (flagged) atomicAdd(&s_flagged, flagged);
   __syncthreads();
   if (threadIdx.x == 0 && s_flagged) atomicAdd(&marks[1], s_flagged);
+}
+
+// The same with a thread per row, for matrices of few entries a row: a group of
+// eight lanes spends its instructions on the reductions (5-point grid 1009²:
+// 94 -> 20 µs with the row's entries in turn, four loads in flight).  Rows of
+// more than kThreadRow entries are taken by whole warps afterwards.
+constexpr int kThreadRow = 16;
+__global__ void __launch_bounds__(256) k_prepass_short(
+    MatView A, int32_t n_b, const int4* __restrict__ info, int64_t* __restrict__ f,
+    int32_t* __restrict__ lo, int32_t* __restrict__ hi, uint8_t* __restrict__ flag,
+    int2* __restrict__ pieces, int64_t max_pieces, int32_t* __restrict__ marks,
+    uint32_t* status, const int* skip) {
+  if (skip && *skip) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const bool on = i < A.n;
+  if (i == 0 && (A.rowptr[0] != 0 || (int64_t)A.rowptr[A.n] != A.nnz))
+    report(status, DEV_ERR_INVALID_CSR);
+  int32_t s = on ? A.rowptr[i] : 0, e = on ? A.rowptr[i + 1] : 0;
+  const int32_t s1 = on && i > 0 ? A.rowptr[i - 1] : -1;
+  const bool wrong = s < 0 || e < s || (int64_t)e > A.nnz;
+  if (wrong) s = e = 0;
+  const int len = e - s;
+  const bool candidate = len > 0 && len <= kMaxLen && s1 >= 0 && s - s1 == len;
+  bool same = candidate;
+  RowSums t;
+  if (len <= kThreadRow) {
+    int before = -1;
+    for (int q = 0; q < len; q += 4) {
+      int32_t k[4], above[4];
+      int4 b[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool in = q + u < len;
+        k[u] = in ? A.col[s + q + u] : -1;
+        above[u] = in && candidate ? A.col[s + q + u - len] : -2;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        b[u] = k[u] >= 0 && k[u] < n_b ? info[k[u]] : make_int4(0, 0, INT_MAX, -1);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (q + u >= len) break;
+        const unsigned n = (unsigned)(b[u].y - b[u].x);
+        t.bad = t.bad || k[u] < 0 || k[u] >= n_b || before >= k[u] || (int)n < 0;
+        t.lo16 += n & 0xffffu;
+        t.hi16 += n >> 16;
+        t.mn = min(t.mn, b[u].z);
+        t.mx = max(t.mx, b[u].w);
+        same = same && above[u] == k[u] - 1;
+        before = k[u];
+      }
+    }
+  }
+  for (unsigned more = __ballot_sync(kFull, len > kThreadRow && len <= kLongRow); more;
+       more &= more - 1u) {
+    const int src = __ffs((int)more) - 1;
+    const int32_t ws = __shfl_sync(kFull, s, src), we = __shfl_sync(kFull, e, src);
+    const bool wc = __shfl_sync(kFull, (int)candidate, src);
+    RowSums w;
+    const bool ws_same = w.add<true>(A, info, n_b, ws, ws + lane, we, 32, wc ? we - ws : 0);
+    const bool all = __all_sync(kFull, ws_same);
+    w.reduce(WarpGroup(32));
+    if (lane == src) {
+      t = w;
+      same = all && wc;
+    }
+  }
+  if (len > kLongRow) {
+    const int pc = (len + kLongPiece - 1) / kLongPiece;
+    const int64_t at = (unsigned)atomicAdd(&marks[0], pc);
+    // (rows of a valid A cannot list more)
+    if (at + pc > max_pieces) report(status, DEV_ERR_INVALID_CSR);
+    else
+      for (int c = 0; c < pc; ++c) pieces[at + c] = make_int2((int)i, s + c * kLongPiece);
+  }
+  const bool bad = t.bad || wrong;
+  if (on) {
+    if (bad) report(status, DEV_ERR_INVALID_CSR);
+    f[i] = bad ? -1 : t.products();
+    lo[i] = bad ? INT_MAX : t.mn;
+    hi[i] = bad ? -1 : t.mx;
+    flag[i] = same && !bad;
+  }
+  const int flagged = __syncthreads_count(on && same && !bad);
+  if (threadIdx.x == 0 && flagged) atomicAdd(&marks[1], flagged);
 }
 
 // The listed pieces.
@@ -678,7 +786,19 @@ __global__ void __launch_bounds__(256) k_find_runs(
   __syncthreads();
   // a row of C follows its predecessor when its row of A and the rows of B that
   // it reads do
-  for (int r0 = tid / G; r0 < kRunBlock; r0 += kRunBlock / G * kRowsAhead) {  // whole warps
+  if (G == kShortLanes) {  // few entries a row: a thread per row
+    bool follows = tid > 0 && tid < rows && sflag[tid];
+    if (follows)
+      for (int32_t q = ptr[tid]; q < ptr[tid + 1] && follows; q += 4) {
+        int32_t k[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) k[u] = A.col[min(q + u, ptr[tid + 1] - 1)];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) follows = flag_b[k[u]] && follows;
+      }
+    const unsigned starts = __ballot_sync(kFull, tid < rows && !follows);
+    if ((tid & 31) == 0) firsts[tid >> 5] = starts;
+  } else for (int r0 = tid / G; r0 < kRunBlock; r0 += kRunBlock / G * kRowsAhead) {  // whole warps
     int32_t p[kRowsAhead], e[kRowsAhead], k[kRowsAhead];
     bool follows[kRowsAhead];
 #pragma unroll
@@ -757,7 +877,7 @@ __global__ void __launch_bounds__(256) k_find_runs(
 
 int lanes_for(const MatView& A) {
   const double mean = A.n > 0 ? (double)A.nnz / A.n : 1.0;
-  return mean <= 8 ? 8 : mean <= 16 ? 16 : 32;
+  return mean <= 8 ? kShortLanes : mean <= 16 ? 16 : 32;
 }
 
 }  // namespace
@@ -785,9 +905,13 @@ cudaError_t launch_prepass_rows(const MatView& A, const MatView& B, const Prepas
   // fewer rows per CTA where 256 would leave SMs without one
   int rows = kRunBlock;
   while (rows > kRowsAhead * (256 / G) && rows > 32 && A.n / rows < num_sms * 8) rows >>= 1;
-  k_prepass_rows<<<(unsigned)((A.n + rows - 1) / rows), 256, 0, s>>>(
-      A, B.n, w.info, G, rows, w.f, w.lo, w.hi, w.flag_a, w.pieces, prepass_pieces(A.nnz),
-      w.marks, status, skip);
+  if (G == kShortLanes)
+    k_prepass_short<<<blocks, 256, 0, s>>>(A, B.n, w.info, w.f, w.lo, w.hi, w.flag_a, w.pieces,
+                                           prepass_pieces(A.nnz), w.marks, status, skip);
+  else
+    k_prepass_rows<<<(unsigned)((A.n + rows - 1) / rows), 256, 0, s>>>(
+        A, B.n, w.info, G, rows, w.f, w.lo, w.hi, w.flag_a, w.pieces, prepass_pieces(A.nnz),
+        w.marks, status, skip);
   SPG_COUNT_LAUNCH();
   if (A.nnz > kLongRow) {
     k_prepass_long<<<num_sms * 4, 256, 0, s>>>(A, B.n, w.info, w.f, w.lo, w.hi, w.pieces,

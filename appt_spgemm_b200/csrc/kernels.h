@@ -123,11 +123,20 @@ constexpr int kRunMaxProducts = 768;
 constexpr int kRunMaxSpan = 1 << 18;
 constexpr int kRunBuffer = 9216;
 
-// Team size (log2 warps) of a run whose rows have m entries: a warp per 16
-// entries, and a share of the buffer that holds the operands.
-__host__ __device__ __forceinline__ int run_team(int64_t m, int need) {
-  int t = m <= 16 ? 0 : m <= 32 ? 1 : m <= 64 ? 2 : 3;
-  while (t < 3 && need > (kRunBuffer >> (3 - t))) ++t;
+// … and of the runs that teams of one warp take.
+constexpr int kRunSmallProducts = 192;
+constexpr int kRunSmallSpan = 1 << 15;
+constexpr int kRunSmallBuffer = 704;
+
+// Team size (log2 warps) of a run whose rows have m entries of f products over
+// `span` columns: a warp per 16 entries, and a share of the buffer that holds
+// the operands.
+__host__ __device__ __forceinline__ int run_team(int64_t m, int need, int64_t f, int64_t span) {
+  int t = m <= 16 && f <= kRunSmallProducts && span <= kRunSmallSpan && need <= kRunSmallBuffer ? 0
+          : m <= 32                                                                              ? 1
+          : m <= 64                                                                              ? 2
+                                                                                                 : 3;
+  while (t > 0 && t < 3 && need > (kRunBuffer >> (3 - t))) ++t;
   return t;
 }
 
@@ -207,7 +216,8 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
     if (!(s.mode == 1 && s.lead && s.runlen[i]) && narrow_row_rule(s.f[i], len, span))
       return narrow_bin(s.f[i], len, span);
   }
-  if (s.mode == 1 && s.lead && s.runlen[i]) return kRunBin0 + run_team(size, s.need[i]);
+  if (s.mode == 1 && s.lead && s.runlen[i]) 
+    return kRunBin0 + run_team(size, s.need[i], s.f[i], (int64_t)s.hi[i] - s.lo[i] + 1);
   if (s.force_heavy || (s.panels && paneled_row(s.f[i], s.arowptr[i + 1] - s.arowptr[i], s.lo[i], s.hi[i]))) return kHeavyBin;
   int lg = table_log2(size, s.load_pct);
   if (s.mode == 1 && s.sort_rows && lg <= s.max_log2 &&

@@ -225,3 +225,38 @@ def test_row_pointers_and_bins_of_many_tiles(eng):
     A = from_rows(n, rows, 16)
     for task in ("AA", "AAt", "AAtS"):
         product(eng, A, task)
+
+
+# runs of few entries a row: either side of what teams of one warp take in span
+# (32,768 columns) and in room for their operands
+@pytest.mark.parametrize("n,offsets,label", [
+    (40001, [0, 16383], "num/runs1"), (40001, [0, 16384], "num/runs2"),
+    (999, [0, 50, 100], "num/runs1"), (999, [0, 50, 100, 150], "num/runs2"),
+    (999, list(range(8)), "num/runs1"), (999, list(range(9)), "num/runs2")])
+def test_shifted_rows_short(n, offsets, label):
+    from appt_spgemm_b200.engine import Engine
+    with Engine("cuda:0", small_max_nnz=-1) as e:
+        e.binned = True
+        assert label in product(e, by_offsets(n, offsets, seed=n), "AA")
+
+
+def test_prepass_of_short_rows():
+    # few entries a row on average: rows on either side of what a thread, a warp and
+    # a piece of a long row take, next to one another and to empty ones
+    from appt_spgemm_b200.engine import Engine
+    rng = np.random.default_rng(17)
+    n = 9001
+    rows = [np.arange(i, min(i + 3, n)) for i in range(n)]
+    lengths = [0, 1, 3, 4, 5, 15, 16, 17, 31, 32, 33, 125, 126, 127, 255, 256, 257, 1023, 1024, 1025]
+    for at, length in enumerate(lengths):
+        for i in (at, 300 + 32 * at, n - 1 - at):
+            rows[i] = rng.choice(n, length, replace=False)
+        start = int(rng.integers(0, n - length - 40))
+        for i in range(2000 + 40 * at, 2003 + 40 * at):  # shifted rows of this length
+            rows[i] = start + i - 2000 - 40 * at + np.arange(length)
+    A = from_rows(n, rows, 18)
+    assert A.nnz <= 8 * n
+    with Engine("cuda:0", small_max_nnz=-1) as e:
+        e.binned = True
+        product(e, A, "AA")
+        product(e, A, "AAt")

@@ -22,6 +22,13 @@
 //    columns without an entry;
 //  - the symbolic phase's distinct-column counts per block give the panel's
 //    first slot in C, and the panel is written in column order.
+// R-MAT 2^16: the launches of the rows that were in CTAs 2.7 ms against 6.8
+// there, and 3.2 ms now that rows of fewer products come here too.  Bound by the shared
+// and L1 pipe (LSU wavefronts 79%: a 64-bit read and write of a place per product,
+// the columns and values of the slices) and by issue (65%).  Panels of 2048 columns
+// 3.36 against 2.68 ms (fewer warps per SM), of 512 3.02 (more slices per entry of
+// A); eight tasks drawn at a time, before that, 6.4 against 3.5 ms (one warp was left
+// with a hub row's neighbouring panels).
 #include <algorithm>
 #include <climits>
 

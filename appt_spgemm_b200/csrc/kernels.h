@@ -31,7 +31,13 @@ cudaError_t launch_prepass(const MatView& A, const MatView& B, int64_t* f, int32
                            int64_t fcap = INT64_MAX);
 
 // Sorted rows: the fewest and the most products, the most products per two entries.
-constexpr int64_t kSortMinProducts = 48;
+// Measured per call, Erdős–Rényi 262,147 (81 products a row) A·Aᵀ / R-MAT 2^14 A·A:
+// rows from 96 products on 1.71 ms / -, from 48 1.19 / 1.17, 24 1.14 / 1.14, 8 1.12 /
+// 1.12.  Rows that merge more are hashed: sorting up to 2.5 or 4.5 products an entry
+// took banded rows 706 and 878 µs against 673 (hashed), the 48-matrix batch 9.2 and
+// 9.6 ms against 9.26.  Beyond the warp kernels' largest table the alternative is
+// slower: R-MAT 2^15's rows there 174 µs in windows, 10 µs more sorted rows.
+constexpr int64_t kSortMinProducts = 8;
 constexpr int64_t kSortMaxProducts = 4096;
 constexpr int64_t kSortMaxMerge2 = 3;
 constexpr int64_t kSortMaxMerge2Large = 6;  // beyond the warp kernels' largest table
@@ -55,9 +61,14 @@ constexpr int64_t kWarpRowMaxProducts = (int64_t)1 << 17;
 
 // Narrow rows: the fewest products per entry of A's row (mean B-row length; up
 // to kNarrowHalfMean half a warp takes the row), the fewest products per column
-// spanned (1 / kNarrowFill), and the fewest and the most products.
+// spanned (1 / kNarrowFill), and the fewest and the most products.  Measured per
+// call, band of 50,021 / 48-matrix batch / replay of 24: half warps up to a mean of 7
+// 402 µs / 7.48 / 3.79 ms, 10 400 / 7.45 / 3.77, 20 416 / 7.50 / 3.82, 40 448 / 7.70 /
+// 3.92.  The other lines matter little there (a mean of 3 or 12, one or a sixteenth
+// of a product per column, 24 products: all within 1.5%, the run-to-run spread, but
+// R-MAT 2^16 5.45 ms against 5.36 with a sixteenth).
 constexpr int64_t kNarrowMinMean = 6;
-constexpr int64_t kNarrowHalfMean = 20;
+constexpr int64_t kNarrowHalfMean = 10;
 constexpr int64_t kNarrowFill = 4;
 constexpr int64_t kNarrowMinProducts = 48;
 constexpr int64_t kNarrowMaxProducts = 1 << 16;
@@ -117,7 +128,10 @@ __host__ __device__ __forceinline__ int narrow_bin(int64_t f, int32_t len, int64
 }
 
 // Runs: the fewest rows, and the limits of a row (products, columns spanned) and
-// of its operands for 32 rows (doubles), split over the teams of a CTA.
+// of its operands for 32 rows (doubles), split over the teams of a CTA: two CTAs
+// share an SM's 227 KB.  Runs from 32 rows on only: 96³ stencil 2.04 ms against 1.88
+//, 47³ 617 against 599 µs; from 4 on: no faster (597
+// against 587 µs), so 8.
 constexpr int kRunMinRows = 8;
 constexpr int kRunMaxProducts = 768;
 constexpr int kRunMaxSpan = 1 << 18;
@@ -216,9 +230,11 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
     if (!(s.mode == 1 && s.lead && s.runlen[i]) && narrow_row_rule(s.f[i], len, span))
       return narrow_bin(s.f[i], len, span);
   }
-  if (s.mode == 1 && s.lead && s.runlen[i]) 
+  if (s.mode == 1 && s.lead && s.runlen[i])
     return kRunBin0 + run_team(size, s.need[i], s.f[i], (int64_t)s.hi[i] - s.lo[i] + 1);
-  if (s.force_heavy || (s.panels && paneled_row(s.f[i], s.arowptr[i + 1] - s.arowptr[i], s.lo[i], s.hi[i]))) return kHeavyBin;
+  if (s.force_heavy ||
+      (s.panels && paneled_row(s.f[i], s.arowptr[i + 1] - s.arowptr[i], s.lo[i], s.hi[i])))
+    return kHeavyBin;
   int lg = table_log2(size, s.load_pct);
   if (s.mode == 1 && s.sort_rows && lg <= s.max_log2 &&
       sorted_row(s.f[i], size, (int64_t)s.hi[i] - s.lo[i] + 1,

@@ -53,13 +53,13 @@ def from_rows(n, rows, seed):
 
 
 # rows of exactly d·d products over 20,011 columns: either side of the kernel's
-# smallest row (48), of each row capacity and of the largest (4096)
-@pytest.mark.parametrize("d", [6, 7, 11, 12, 16, 17, 19, 20, 22, 23, 27, 28, 32, 33, 39, 45, 46, 55,
+# smallest row (8), of each row capacity and of the largest (4096)
+@pytest.mark.parametrize("d", [2, 3, 6, 7, 11, 12, 16, 17, 19, 20, 22, 23, 27, 28, 32, 33, 39, 45, 46, 55,
                                64, 65])
 def test_sorted_rows(eng, d):
     labels = product(eng, csr.uniform(20011, d, seed=d), "AA")
     if eng.binned:
-        assert any(x.startswith("num/sort") for x in labels) == (7 <= d <= 64)
+        assert any(x.startswith("num/sort") for x in labels) == (3 <= d <= 64)
 
 
 def test_sorted_rows_uneven(eng):

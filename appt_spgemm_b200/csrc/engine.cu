@@ -1,5 +1,5 @@
 // Host orchestration of the engine: context, plan (pre-pass + binning +
-// symbolic), execute (numeric + mirror), multiply, transpose, descriptors and
+// symbolic), execute (numeric), multiply, transpose, descriptors and
 // the run_ours-compatible call.
 //
 // The reference's run_ours (src/spgemm_engine.cuh:132-210) allocates and frees

@@ -13,8 +13,8 @@
 // a byte per column with plain stores (every store writes 1, so they need no
 // order and no atomics) and counts the bytes.
 //
-// Random band of 50,021 rows and half-bandwidth 48: numeric 347 -> 173 µs, symbolic
-// 154 -> 117 µs, call 654 -> 418 µs.  Bound by issue (67% of slots) and
+// Random band of 50,021 rows and half-bandwidth 48: numeric 347 -> 157 µs, symbolic
+// 154 -> 117 µs, call 652 -> 385 µs.  Bound by issue (74% of slots) and
 // shared-memory wavefronts (73%): about 2.5 warp instructions a product.  Walking
 // the B rows without the list of segments took 207 against 145 µs (its loop
 // control was most of its 3.7 instructions a product).

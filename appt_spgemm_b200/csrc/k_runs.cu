@@ -23,7 +23,7 @@
 // rows at the grid's faces in the hash kernels), symbolic 1.04 -> 0.07 ms, call
 // 4.51 -> 1.88 ms; 5-point grid 1009²: call 1.27 -> 0.38 ms.  The run kernel
 // issues on 42% of cycles and moves shared-memory wavefronts on 50% (two 64-bit
-// loads a product), with two CTAs of 16 warps per SM in its 109 KB: latency is
+// loads a product), with two CTAs (16 warps) per SM, 109 KB each: latency is
 // what is left.  Measured and not kept: two entries' sums at a time 1.16 ms,
 // entries drawn by list length 1.16 ms, neighbouring runs to one CTA 1.16 ms;
 // the entries shared out by list length, or 16 warps a team (32 per SM): no change.
@@ -41,7 +41,7 @@ constexpr int kStageRow = 33;                 // doubles between staged entries 
 constexpr int kMaxLen = 126;                  // entries of A's row
 
 // A launch's CTA by team size: threads, and the limits of its runs' rows.  The
-// runs of few entries a row (teams of one warp) have small CTAs, six per SM
+// runs of few entries a row (teams of one warp) have small CTAs, five per SM
 // instead of two: a run's own steps (its entries, its rows of B, the check of
 // its columns) are a chain of loads that only other CTAs hide.  5-point grid
 // 1009²: 145 -> 127 µs.

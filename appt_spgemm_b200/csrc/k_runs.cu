@@ -19,13 +19,14 @@
 //    memory once, and an output entry of all 32 rows is one walk over its list,
 //    the same for every lane.  Sums start from 0.0 and take the products in k
 //    order, so the values are those of the other kernels, bit for bit.
-// 27-point stencil 96³, A·A: numeric phase 2.99 -> 1.24 ms (runs 1.11 ms, the
-// rows at the grid's faces in the hash kernels), symbolic 1.04 -> 0.07 ms, call
+// 27-point stencil 96³, A·A: numeric phase 2.99 -> 1.42 ms (runs 1.26 ms, the
+// rows at the grid's faces in the hash kernels), symbolic 1.04 -> 0.09 ms, call
 // 4.51 -> 1.88 ms; 5-point grid 1009²: call 1.27 -> 0.38 ms.  The run kernel
-// issues on 42% of cycles and moves shared-memory wavefronts on 50% (two 64-bit
+// issues on 44% of cycles and moves wavefronts on 56% (two 64-bit shared-memory
 // loads a product), with two CTAs (16 warps) per SM, 109 KB each: latency is
-// what is left.  Measured and not kept: two entries' sums at a time 1.16 ms,
-// entries drawn by list length 1.16 ms, neighbouring runs to one CTA 1.16 ms;
+// what is left.  Measured and not kept (against 1.11 ms for the largest launch in
+// those runs): two entries' sums at a time 1.16, entries drawn by list length 1.16,
+// neighbouring runs to one CTA 1.16 ms;
 // the entries shared out by list length, or 16 warps a team (32 per SM): no change.
 #include <climits>
 

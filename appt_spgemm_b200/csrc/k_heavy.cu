@@ -301,11 +301,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num(HeavyArgs h) {
 template <typename K>
 static cudaError_t launch_h(K kernel, int threads, size_t smem, const HeavyArgs& h, int num_sms,
                             cudaStream_t s) {
-  cudaError_t e;
-  if (smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  // (the widest window with the most threads: 180 KB)
+  cudaError_t e = allow_shared_memory(kernel, heavy_smem_bytes(true, 1024, 1 << 20));
+  if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
   if (e != cudaSuccess) return e;

@@ -287,8 +287,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
 template <typename K>
 static cudaError_t launch_win(K kernel, int threads, size_t smem, const HeavyArgs& h,
                               int num_sms, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+  // (the most values with the widest window and the most threads: 192 KB)
+  cudaError_t e = allow_shared_memory(kernel, heavy_win_smem_bytes(1024, 16384, 1 << 18));
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);

@@ -184,13 +184,9 @@ __global__ void __launch_bounds__(256) k_narrow_sym(RowArgs a, int W) {
 template <typename K>
 cudaError_t launch_narrow_k(K kernel, int rows, int threads, size_t smem, const RowArgs& a, int W,
                             int num_sms, cudaStream_t s) {
-  cudaError_t e;
-  if (smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           cudaSharedmemCarveoutMaxShared);
+  // (smem is at most 48 KB: two rows of 1024 columns take 18 KB)
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);

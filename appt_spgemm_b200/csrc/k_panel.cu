@@ -351,9 +351,10 @@ cudaError_t launch_panels(HeavyArgs& h, void* workspace, bool table, int num_sms
   auto kernel = k_panel_num;
   const size_t per = panel_warp_bytes(h.pan_log2);
   // two CTAs per SM, each of as many warps as half of its shared memory holds
-  const int warps = (int)std::max<size_t>(1, std::min<size_t>(16, (size_t)112 * 1024 / per));
+  constexpr size_t kMostBytes = (size_t)112 * 1024;
+  const int warps = (int)std::max<size_t>(1, std::min<size_t>(16, kMostBytes / per));
   const size_t bytes = per * warps;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  e = allow_shared_memory(kernel, kMostBytes);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, bytes);

@@ -296,8 +296,8 @@ cudaError_t launch_sort_nw(int F, const RowArgs& a, int num_sms, cudaStream_t s)
   const int threads = NW > 1 ? NW * 32 : rows * 32;
   const size_t smem = sort_row_bytes(F) * rows;
   cudaError_t e;
-  if (smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (NW > 1 && sort_row_bytes(512 * NW) > 48 * 1024) {
+    e = allow_shared_memory(kernel, sort_row_bytes(512 * NW));
     if (e != cudaSuccess) return e;
   }
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,

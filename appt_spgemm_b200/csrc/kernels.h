@@ -14,6 +14,16 @@ namespace spg {
 extern thread_local long long g_kernel_launches;
 #define SPG_COUNT_LAUNCH() (++::spg::g_kernel_launches)
 
+// What a kernel may be launched with at most belongs to its function in the
+// process's device context, which the engine contexts of all threads share: a
+// launcher sets it to one value, the most it ever asks for, never to what the
+// launch at hand needs (a thread that lowered it between another's call and launch
+// made that launch fail).
+template <typename K>
+cudaError_t allow_shared_memory(K kernel, size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // ---- validation / pre-pass / binning (k_prepass.cu) --------------------------
 
 // Flags DEV_ERR_BAD_INDEX / sets *bad (device int) when A is not a square CSR

@@ -54,7 +54,7 @@ __device__ __forceinline__ int2 row_panels(const HeavyArgs& h, int row) {
 __device__ __forceinline__ int32_t column_bound(const int32_t* __restrict__ col, int32_t l,
                                                 int32_t u, int64_t c) {
   while (l < u) {
-    const int32_t mid = (l + u) >> 1;
+    const int32_t mid = l + ((u - l) >> 1);  // (l + u may exceed 2^31)
     if (col[mid] < c) l = mid + 1; else u = mid;
   }
   return l;

@@ -609,7 +609,7 @@ __global__ void k_describe(MatView A, const int32_t* __restrict__ colcount, Desc
       // is (j, i) present?  binary search for i in row j
       int32_t lo = A.rowptr[j], hi = A.rowptr[j + 1];
       while (lo < hi) {
-        int32_t mid = (lo + hi) >> 1;
+        const int32_t mid = lo + ((hi - lo) >> 1);  // (lo + hi may exceed 2^31)
         if (A.col[mid] < i) lo = mid + 1; else hi = mid;
       }
       if (lo < A.rowptr[j + 1] && A.col[lo] == i) ++sym;

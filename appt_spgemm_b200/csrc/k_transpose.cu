@@ -66,7 +66,7 @@ __global__ void k_sym_transpose_vals(MatView A, double* __restrict__ t_val, int*
         }
         const int32_t end = hi;
         while (lo < hi) {
-          const int32_t mid = (lo + hi) >> 1;
+          const int32_t mid = lo + ((hi - lo) >> 1);  // (lo + hi may exceed 2^31)
           if (A.col[mid] < k) lo = mid + 1; else hi = mid;
         }
         if (lo < end && A.col[lo] == k) {

@@ -88,3 +88,59 @@ def test_heavy_rows_of_different_shapes_in_several_contexts():
         return run
 
     in_threads(*(body(*j) for j in jobs))
+
+
+def most_entries(total, tail_rows, degree, seed):
+    """A matrix of `total` entries on the device, whose last `tail_rows` rows are a
+    random product of their own and whose other entries point at empty rows; with it
+    those rows as a matrix of their own."""
+    from appt_spgemm_b200.engine import CsrDevice
+    n = 1 << 26
+    tail = csr.uniform(tail_rows, degree, seed)
+    first, end = 40, n - tail_rows           # the empty rows
+    rest = total - tail.nnz
+    counts = np.zeros(n, dtype=np.int64)
+    counts[:rest // (end - first)] = end - first
+    counts[rest // (end - first)] = rest % (end - first)
+    counts[end:] = np.diff(tail.rowptr)
+    rp = np.zeros(n + 1, dtype=np.int32)
+    rp[1:] = np.cumsum(counts)
+    col = torch.empty(total, dtype=torch.int32, device="cuda:0")
+    for r in range(first):
+        if counts[r]:
+            col[rp[r]:rp[r + 1]] = torch.arange(first, first + int(counts[r]), dtype=torch.int32,
+                                                device="cuda:0")
+    col[rest:] = torch.from_numpy(tail.col + np.int32(end)).to("cuda:0")
+    val = torch.zeros(total, dtype=torch.float64, device="cuda:0")
+    val[rest:] = torch.from_numpy(tail.val).to("cuda:0")
+    return CsrDevice(n, torch.from_numpy(rp).to("cuda:0"), col, val), tail
+
+
+def needs_memory(bytes_):
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < bytes_:
+        pytest.skip("not enough device memory")
+
+
+def test_searches_beyond_two_to_the_thirty_entries():
+    # the middle of two positions above 2^30: panels that search for their slices
+    # (the table of their bounds would be as large as C many times), and the
+    # descriptors' look for each entry's mirror
+    from appt_spgemm_b200.engine import Engine
+    needs_memory(90 << 30)
+    A, tail = most_entries((1 << 31) - (1 << 16), 3000, 90, seed=5)
+    with Engine("cuda:0") as e:
+        ref = oracle.multiply(tail, "AA")
+        got = []
+        assert "num/panels" in kernels(e, lambda: got.append(e.multiply(A, "AA")))
+        e.check_device_status()
+        C, end = got[0], A.n - tail.n
+        assert int(C.rowptr[end]) == 0
+        assert_same_csr((C.rowptr[end:].cpu().numpy(), C.col.cpu().numpy() - end,
+                         C.val.cpu().numpy()), ref, "last rows")
+        d = e.describe(A)
+        assert d["products_aa"] == int(np.diff(tail.rowptr)[tail.col].sum())
+        mirrored = len(np.intersect1d(
+            *(lambda r: (r * tail.n + tail.col, tail.col * tail.n + r))(
+                np.repeat(np.arange(tail.n, dtype=np.int64), np.diff(tail.rowptr)))))
+        assert abs(d["pattern_symmetry"] * A.nnz - mirrored) < 0.5

@@ -10,6 +10,10 @@
 namespace spg {
 
 // A matrix as the kernels see it (B is A, or the engine's transpose of A).
+// A position among a matrix's entries, to which a kernel adds a step: a matrix may
+// hold 2^31 − 1 entries, and a position past its end wraps in a signed word.
+using Pos = uint32_t;
+
 struct MatView {
   int32_t n;
   int64_t nnz;

@@ -76,13 +76,13 @@ __global__ void __launch_bounds__(256) k_dense_w32(RowArgs a) {
     const int nwords = (int)(((int64_t)hi - lo + 32) >> 5);  // row_bin keeps it <= W
     for (int i = lane * 4; i < nwords; i += 128) *(uint4*)(bm + i) = make_uint4(0, 0, 0, 0);
     __syncwarp();
-    const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+    const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
 
     // mark: segments in any order (an OR); when every B row of a chunk fits
     // one segment, the columns of kMarkAhead segments are loaded before any
     // of them is marked (their loads overlap)
     constexpr int kMarkAhead = 8;
-    for (int32_t pb = ps; pb < pe; pb += 32) {
+    for (Pos pb = ps; pb < pe; pb += 32) {
       const int cnt = min(32, pe - pb);
       int bs = 0, len = 0;
       if (lane < cnt) {
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256) k_dense_w32(RowArgs a) {
 
     // accumulate in the order of A's row: D segments loaded, then added in turn
     constexpr int D = 4;
-    for (int32_t pb = ps; pb < pe; pb += 32) {
+    for (Pos pb = ps; pb < pe; pb += 32) {
       const int cnt = min(32, pe - pb);
       int bs = 0, len = 0;
       double av = 0.0;

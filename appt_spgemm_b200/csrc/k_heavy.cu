@@ -49,11 +49,11 @@ constexpr int kLongBRow = 256;
 __device__ __forceinline__ void mark_window(const RowArgs& a, int row, long long w0, int nwords,
                                             uint32_t* bm, int* st_bs, int* st_len, int* st_long,
                                             void* scratch) {
-  const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+  const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
   const long long wbits = (long long)nwords * 32;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwarps = blockDim.x >> 5;
   int* nlong_p = (int*)scratch;
-  for (int32_t pb = ps; pb < pe; pb += blockDim.x) {
+  for (Pos pb = ps; pb < pe; pb += blockDim.x) {
     const int cnt = min((int)blockDim.x, pe - pb);
     int bs = 0, len = 0;
     if (tid < cnt) {
@@ -225,9 +225,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num(HeavyArgs h) {
       __syncthreads();
       // k-ordered accumulation in place; the first HT entries of B row t+1 are
       // loaded while row t is accumulated
-      const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+      const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
       const long long wbits = (long long)nwords * 32;
-      for (int32_t pb = ps; pb < pe; pb += HT) {
+      for (Pos pb = ps; pb < pe; pb += HT) {
         const int cnt = min(HT, pe - pb);
         if (tid < cnt) {
           const int32_t k = a.A.col[pb + tid];

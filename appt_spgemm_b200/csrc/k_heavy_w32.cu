@@ -63,15 +63,15 @@ __device__ __forceinline__ int window_end(const uint16_t* cnt, int b, int nb, in
 // One window [c0, c1) of row `row`: accumulate, sort and write its entries at
 // base + written; returns the number of entries written.
 template <int LOG2T>
-__device__ __forceinline__ int heavy_window(const HeavyArgs& h, int row, int ps, int pe, int c0, int c1,
+__device__ __forceinline__ int heavy_window(const HeavyArgs& h, int row, Pos ps, Pos pe, int c0, int c1,
                            int* keys, double* vals, int64_t base, int64_t room) {
   constexpr int T = 1 << LOG2T;
   const RowArgs& a = h.r;
   const int lane = threadIdx.x & 31;
   for (int s = lane * 4; s < T; s += 128) *(int4*)(keys + s) = make_int4(-1, -1, -1, -1);
   __syncwarp();
-  for (int g0 = ps; g0 < pe; g0 += 32) {
-    const int p = g0 + lane;
+  for (Pos g0 = ps; g0 < pe; g0 += 32) {
+    const Pos p = g0 + lane;
     int4 st = make_int4(0, 0, INT_MAX, 0);
     if (p < pe) st = h.hcur[p];
     const bool act = st.z < c1;
@@ -89,8 +89,8 @@ __device__ __forceinline__ int heavy_window(const HeavyArgs& h, int row, int ps,
         jr[d] = INT_MAX;
         br[d] = 0.0;
         if (td[d] >= 0) {
-          const int cur = __shfl_sync(kFull, st.x, td[d]);
-          const int end = __shfl_sync(kFull, st.y, td[d]);
+          const Pos cur = __shfl_sync(kFull, st.x, td[d]);
+          const Pos end = __shfl_sync(kFull, st.y, td[d]);
           if (cur + lane < end) {
             jr[d] = a.B.col[cur + lane];
             br[d] = a.B.val[cur + lane];
@@ -101,9 +101,9 @@ __device__ __forceinline__ int heavy_window(const HeavyArgs& h, int row, int ps,
       for (int d = 0; d < kHeavyD; ++d) {
         const int t = td[d];
         if (t < 0) break;
-        const int end = __shfl_sync(kFull, st.y, t);
+        const Pos end = __shfl_sync(kFull, st.y, t);
         const double at = __shfl_sync(kFull, av, t);
-        int q = __shfl_sync(kFull, st.x, t);
+        Pos q = __shfl_sync(kFull, st.x, t);
         int j = jr[d];
         double bv = br[d];
         int next;
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
 
   for (int r = blockIdx.x * nw + w; r < a.nrows; r += gridDim.x * nw) {
     const int row = a.rows[r];
-    const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+    const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
     const int lo = h.lo[row], hi = h.hi[row];
     const int lo_r = lo;
     const int64_t expect = (int64_t)a.cnt_in[row];
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
     int64_t written = 0;
     if (lo_r <= hi) {
       // cursors at the first B entry >= lo_r of every B row of the row
-      for (int p = ps + lane; p < pe; p += 32) {
+      for (Pos p = ps + lane; p < pe; p += 32) {
         const int32_t k = a.A.col[p];
         int s = a.B.rowptr[k];
         const int e = a.B.rowptr[k + 1];

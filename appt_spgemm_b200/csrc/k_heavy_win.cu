@@ -88,11 +88,11 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
     const long long expect = (long long)a.cnt_in[row];
     const int64_t base = a.rowptr[row];
     const int cb = a.colbase ? a.colbase[row] : 0;
-    const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+    const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
     long long written = 0;
     if (lo_r <= hi) {
       // cursors at the first B entry >= lo_r of every B row of the row
-      for (int32_t p = ps + tid; p < pe; p += HT) {
+      for (Pos p = ps + tid; p < pe; p += HT) {
         const int32_t k = a.A.col[p];
         int s = a.B.rowptr[k];
         const int e = a.B.rowptr[k + 1];
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
         __syncthreads();
 
         // 1. mark the window's columns
-        for (int32_t pb = ps; pb < pe; pb += HT) {
+        for (Pos pb = ps; pb < pe; pb += HT) {
           const int n_here = min(HT, pe - pb);
           int cur = 0, end = 0, nxt = INT_MAX;
           if (tid < n_here) {
@@ -169,9 +169,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
           const int nlong = scratch[43];
           for (int i = 0; i < nlong; ++i) {
             const int t = st_list[i];
-            const int e = st_end[t];
-            for (int q0 = st_cur[t];; q0 += HT) {
-              const int q = q0 + tid;
+            const Pos e = st_end[t];
+            for (Pos q0 = st_cur[t];; q0 += HT) {
+              const Pos q = q0 + tid;
               const int j = q < e ? a.B.col[q] : INT_MAX;
               if (j < c1) {
                 const int d = j - c0;
@@ -183,9 +183,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
           // short runs: a warp each, 32 entries at a time until the window ends
           for (int t = wid; t < n_here; t += nwarps) {
             if (!st_nxt[t]) continue;
-            const int e = st_end[t];
-            for (int q0 = st_cur[t];; q0 += 32) {
-              const int q = q0 + lane;
+            const Pos e = st_end[t];
+            for (Pos q0 = st_cur[t];; q0 += 32) {
+              const Pos q = q0 + lane;
               const int j = q < e ? a.B.col[q] : INT_MAX;
               if (j < c1) {
                 const int d = j - c0;
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
         __syncthreads();
 
         // 3. accumulate in the order of A's row
-        for (int32_t pb = ps; pb < pe; pb += HT) {
+        for (Pos pb = ps; pb < pe; pb += HT) {
           const int n_here = min(HT, pe - pb);
           int cur = 0, end = 0, nxt = INT_MAX;
           double av = 0.0;
@@ -249,11 +249,11 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
           __syncthreads();
           for (int i = 0; i < nact; ++i) {
             const int t = st_list[i];
-            const int s = st_cur[t], e = st_end[t];
+            const Pos s = st_cur[t], e = st_end[t];
             const double at = st_a[t];
             int moved = 0;
-            for (int q0 = s;; q0 += HT) {
-              const int q = q0 + tid;
+            for (Pos q0 = s;; q0 += HT) {
+              const Pos q = q0 + tid;
               const int j = q < e ? a.B.col[q] : INT_MAX;
               const bool in = j < c1;
               if (in) {
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
               if (c < HT) break;
             }
             if (tid == 0) {
-              const int nc = s + moved;
+              const Pos nc = s + moved;
               h.hcur[pb + t] = make_int4(nc, e, nc < e ? a.B.col[nc] : INT_MAX, 0);
             }
           }

@@ -39,10 +39,10 @@ __device__ __forceinline__ void narrow_row(const RowArgs& a, const WarpGroup& g,
                                            double* acc, Segment* segs, int W) {
   const int lo = a.lo[row];
   const int span = min(a.hi[row] - lo + 1, W);
-  const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+  const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
   const int32_t* bcol = a.B.col + g.lane;
   const double* bval = a.B.val + g.lane;
-  for (int32_t pb = ps; pb < pe;) {
+  for (Pos pb = ps; pb < pe;) {
     // the segments of the next entries of A's row, as many whole entries as the
     // list takes (a B row lies within the span: at most 1024 / G segments)
     int start = 0, len = 0;

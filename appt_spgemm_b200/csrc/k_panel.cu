@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h, const int64_t* _
     const int row = a.rows[r];
     const int2 pr = row_panels(h, row);
     const int p = pr.x + (int)(t - off[r]);
-    const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+    const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
     const int cb = a.colbase ? a.colbase[row] : 0;
     const int w0 = p << h.pan_log2;
 
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h, const int64_t* _
       av = a.A.val[ps + lane];
     }
     if (ps + 32 + lane < pe) k = a.A.col[ps + 32 + lane];
-    int32_t pb = ps;                 // next 32 entries
+    Pos pb = ps;                     // next 32 entries
     int run = 0, c0 = 0, first = 0;  // products of the current 32, next one, this lane's first
     auto advance = [&]() -> bool {   // to the next products, if any
       while (c0 >= run) {

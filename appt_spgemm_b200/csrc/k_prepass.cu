@@ -29,10 +29,10 @@ __global__ void k_validate(MatView A, uint32_t* status) {
       continue;
     }
     bool bad = false;
-    for (int32_t p = s + lane; p < e; p += 32) {
+    for (Pos p = s + lane; p < (Pos)e; p += 32) {
       const int32_t j = A.col[p];
       if (j < 0 || j >= A.n) bad = true;
-      if (p > s && A.col[p - 1] >= j) bad = true;
+      if (p > (Pos)s && A.col[p - 1] >= j) bad = true;
     }
     if (__any_sync(0xffffffffu, bad) && lane == 0) report(status, DEV_ERR_INVALID_CSR);
   }
@@ -74,14 +74,14 @@ __global__ void k_prepass(MatView A, MatView B, int64_t* __restrict__ f, int32_t
     bool unsorted = false;
     // four entries per lane at a time, each step's loads issued together (a hub
     // row is a chain of them: R-MAT 2^15 113 -> 53 µs)
-    for (int32_t p0 = s + lane; p0 < e; p0 += 128) {
+    for (Pos p0 = s + lane; p0 < (Pos)e; p0 += 128) {
       int32_t k[4], bs[4], be[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int32_t p = p0 + 32 * u;
-        const bool in = p < e;
+        const Pos p = p0 + 32 * u;
+        const bool in = p < (Pos)e;
         k[u] = in ? A.col[p] : 0;
-        if (in && status && p > s && A.col[p - 1] >= k[u]) unsorted = true;
+        if (in && status && p > (Pos)s && A.col[p - 1] >= k[u]) unsorted = true;
         const bool ok = in && k[u] >= 0 && k[u] < B.n;
         bad = bad || (in && !ok);
         bs[u] = ok ? 0 : -1;
@@ -602,7 +602,7 @@ __global__ void k_describe(MatView A, const int32_t* __restrict__ colcount, Desc
       paat += c * c;
       maxcol = max(maxcol, (int)c);
     }
-    for (int32_t p = s + lane; p < e; p += 32) {
+    for (Pos p = s + lane; p < (Pos)e; p += 32) {
       const int32_t j = A.col[p];
       paa += (unsigned long long)(A.rowptr[j + 1] - A.rowptr[j]);
       band = max(band, (int)(j > i ? j - i : i - j));

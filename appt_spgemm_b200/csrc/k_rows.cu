@@ -121,8 +121,8 @@ __device__ __forceinline__ void hash_row(const Grp& g, const RowArgs& a, const i
                                          uint32_t* rtmp, int* rcnt) {
   constexpr int T = 1 << LOG2T;
   for (int s = g.lane; s < T; s += g.G) keys[s] = kEmptyKey;
-  const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
-  for (int32_t pb = ps; pb < pe; pb += g.G) {
+  const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+  for (Pos pb = ps; pb < pe; pb += g.G) {
     const int cnt = min(g.G, pe - pb);
     g.sync();  // table cleared / previous chunk's staging consumed
     if (g.lane < cnt) {

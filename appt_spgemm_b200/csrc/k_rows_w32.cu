@@ -136,9 +136,9 @@ __device__ __forceinline__ int count_bits(const RowArgs& a, int row, int lo, int
   const int words = ((span + 127) >> 7) << 2;
   for (int s = lane * 4; s < words; s += 128) *(int4*)(bits + s) = make_int4(0, 0, 0, 0);
   __syncwarp();
-  const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+  const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
   int count = 0;  // this lane's products that found their bit clear
-  for (int32_t pb = ps; pb < pe; pb += 32) {
+  for (Pos pb = ps; pb < pe; pb += 32) {
     int bs = 0, len = 0;
     if (pb + lane < pe) {
       const int32_t k = a.A.col[pb + lane];
@@ -253,8 +253,8 @@ __global__ void __launch_bounds__(256, 5) k_hash_w32(RowArgs a) {
     // plain calls of the batch mix 224 / 204 ms against 191 ms)
     for (int s = lane * 4; s < T; s += 128) *(int4*)(keys + s) = make_int4(-1, -1, -1, -1);
     __syncwarp();
-    const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
-    for (int32_t pb = ps; pb < pe; pb += 32) {
+    const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+    for (Pos pb = ps; pb < pe; pb += 32) {
       const int cnt = min(32, pe - pb);
       int bs = 0, len = 0;
       double av = 0.0;

@@ -440,10 +440,10 @@ struct RowSums {
 
   template <bool SHIFT>
   __device__ __forceinline__ bool add(const MatView& A, const int4* __restrict__ info, int32_t n_b,
-                                      int32_t s, int32_t p0, int32_t p1, int step, int32_t back) {
+                                      Pos s, Pos p0, Pos p1, int step, int32_t back) {
     bool shifted = SHIFT;
 #pragma unroll 2
-    for (int32_t p = p0; p < p1; p += step) {
+    for (Pos p = p0; p < p1; p += step) {
       const int32_t k = A.col[p];
       if (p > s && A.col[p - 1] >= k) bad = true;
       if (SHIFT && back > 0 && A.col[p - back] != k - 1) shifted = false;
@@ -711,9 +711,10 @@ __global__ void __launch_bounds__(256) k_prepass_long(MatView A, int32_t n_b,
   if (n < 0 || n > max_pieces) return;  // A is invalid, and some pieces are not listed
   for (int c = blockIdx.x; c < n; c += gridDim.x) {
     const int2 piece = pieces[c];
-    const int32_t s = A.rowptr[piece.x], e = min(A.rowptr[piece.x + 1], piece.y + kLongPiece);
+    const Pos s = A.rowptr[piece.x];
+    const Pos e = min((Pos)A.rowptr[piece.x + 1], (Pos)piece.y + kLongPiece);
     RowSums t;
-    t.add<false>(A, info, n_b, s, piece.y + threadIdx.x, e, blockDim.x, 0);
+    t.add<false>(A, info, n_b, s, (Pos)piece.y + threadIdx.x, e, blockDim.x, 0);
     t.reduce(WarpGroup(32));
     if ((threadIdx.x & 31) == 0) {
       if (t.bad) report(status, DEV_ERR_INVALID_CSR);
@@ -790,17 +791,18 @@ __global__ void __launch_bounds__(256) k_find_runs(
   if (G == kShortLanes) {  // few entries a row: a thread per row
     bool follows = tid > 0 && tid < rows && sflag[tid];
     if (follows)
-      for (int32_t q = ptr[tid]; q < ptr[tid + 1] && follows; q += 4) {
+      for (Pos q = ptr[tid], e = ptr[tid + 1]; q < e && follows; q += 4) {
         int32_t k[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) k[u] = A.col[min(q + u, ptr[tid + 1] - 1)];
+        for (int u = 0; u < 4; ++u) k[u] = A.col[min(q + u, e - 1)];
 #pragma unroll
         for (int u = 0; u < 4; ++u) follows = flag_b[k[u]] && follows;
       }
     const unsigned starts = __ballot_sync(kFull, tid < rows && !follows);
     if ((tid & 31) == 0) firsts[tid >> 5] = starts;
   } else for (int r0 = tid / G; r0 < kRunBlock; r0 += kRunBlock / G * kRowsAhead) {  // whole warps
-    int32_t p[kRowsAhead], e[kRowsAhead], k[kRowsAhead];
+    Pos p[kRowsAhead], e[kRowsAhead];
+    int32_t k[kRowsAhead];
     bool follows[kRowsAhead];
 #pragma unroll
     for (int u = 0; u < kRowsAhead; ++u) {
@@ -816,7 +818,7 @@ __global__ void __launch_bounds__(256) k_find_runs(
       if (k[u] >= 0) follows[u] = follows[u] && flag_b[k[u]];
 #pragma unroll
     for (int u = 0; u < kRowsAhead; ++u) {
-      for (int32_t q = p[u] + G; q < e[u]; q += G) follows[u] = follows[u] && flag_b[A.col[q]];
+      for (Pos q = p[u] + G; q < e[u]; q += G) follows[u] = follows[u] && flag_b[A.col[q]];
       const bool all = g.ballot(!follows[u]) == 0u;
       const int r = r0 + u * (kRunBlock / G);
       if (g.lane == 0 && r < rows && !all) atomicOr(&firsts[r >> 5], 1u << (r & 31));

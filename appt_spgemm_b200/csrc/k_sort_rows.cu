@@ -87,7 +87,7 @@ __device__ __forceinline__ void sort_row(const RowArgs& a, const int row, const 
   const int lane = threadIdx.x & 31;
   const int wid = NW == 1 ? 0 : (int)(threadIdx.x >> 5);
   const int tid = NW == 1 ? lane : (int)threadIdx.x;
-  const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+  const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
   const int lo = a.lo[row], hi = a.hi[row];
   const uint32_t span = (uint32_t)(hi - lo) + 1u;
   const int64_t base = a.rowptr[row];
@@ -100,7 +100,7 @@ __device__ __forceinline__ void sort_row(const RowArgs& a, const int row, const 
   // expand: 32 entries of A's row at a time, their products 32 at a time; with
   // several warps each takes its share of those
   int done = 0;
-  for (int32_t pb = ps; pb < pe; pb += 32) {
+  for (Pos pb = ps; pb < pe; pb += 32) {
     int bs = 0, len = 0;
     double av = 0.0;
     if (pb + lane < pe) {

@@ -25,7 +25,7 @@ __global__ void k_transpose_scatter(MatView A, const int32_t* __restrict__ t_row
     // indices are checked (the one-readback plan runs this before the host has
     // the validation verdict): an invalid input only leaves slots unwritten
     if (s < 0 || e < s || (int64_t)e > A.nnz) s = e = 0;
-    for (int32_t p = s + lane; p < e; p += 32) {
+    for (Pos p = s + lane; p < (Pos)e; p += 32) {
       const int32_t k = A.col[p];
       if (k < 0 || k >= A.n) continue;
       const int32_t d = t_rowptr[k] + atomicAdd(&cursor[k], 1);
@@ -53,7 +53,7 @@ __global__ void k_sym_transpose_vals(MatView A, double* __restrict__ t_val, int*
     if (s < 0 || e < s || (int64_t)e > A.nnz) {
       miss = true;
     } else {
-      for (int32_t p = s + lane; p < e; p += 32) {
+      for (Pos p = s + lane; p < (Pos)e; p += 32) {
         const int32_t i = A.col[p];
         if (i < 0 || i >= A.n) {
           miss = true;

@@ -354,8 +354,8 @@ template <int G>
 __device__ __forceinline__ void narrow_mark(const RowArgs& a, const WarpGroup& g, int row, int lo,
                                             int span, unsigned char* seen) {
   constexpr int kAhead = 8;
-  const int32_t ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
-  for (int32_t pb = ps; pb < pe; pb += G) {
+  const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
+  for (Pos pb = ps; pb < pe; pb += G) {
     const int cnt = min(G, pe - pb);
     int bs = 0, len = 0;
     if (g.lane < cnt) {

@@ -122,6 +122,14 @@ def needs_memory(bytes_):
         pytest.skip("not enough device memory")
 
 
+def check_last_rows(e, A, tail, label):
+    C, end = e.multiply(A, "AA"), A.n - tail.n
+    e.check_device_status()
+    assert int(C.rowptr[end]) == 0
+    assert_same_csr((C.rowptr[end:].cpu().numpy(), C.col.cpu().numpy() - end,
+                     C.val.cpu().numpy()), oracle.multiply(tail, "AA"), label)
+
+
 def test_searches_beyond_two_to_the_thirty_entries():
     # the middle of two positions above 2^30: panels that search for their slices
     # (the table of their bounds would be as large as C many times), and the
@@ -130,17 +138,34 @@ def test_searches_beyond_two_to_the_thirty_entries():
     needs_memory(90 << 30)
     A, tail = most_entries((1 << 31) - (1 << 16), 3000, 90, seed=5)
     with Engine("cuda:0") as e:
-        ref = oracle.multiply(tail, "AA")
-        got = []
-        assert "num/panels" in kernels(e, lambda: got.append(e.multiply(A, "AA")))
-        e.check_device_status()
-        C, end = got[0], A.n - tail.n
-        assert int(C.rowptr[end]) == 0
-        assert_same_csr((C.rowptr[end:].cpu().numpy(), C.col.cpu().numpy() - end,
-                         C.val.cpu().numpy()), ref, "last rows")
+        assert "num/panels" in kernels(e, lambda: check_last_rows(e, A, tail, "last rows"))
         d = e.describe(A)
         assert d["products_aa"] == int(np.diff(tail.rowptr)[tail.col].sum())
         mirrored = len(np.intersect1d(
             *(lambda r: (r * tail.n + tail.col, tail.col * tail.n + r))(
                 np.repeat(np.arange(tail.n, dtype=np.int64), np.diff(tail.rowptr)))))
         assert abs(d["pattern_symmetry"] * A.nnz - mirrored) < 0.5
+
+
+FORCED = dict(force_heavy=1, heavy_split=1)
+
+
+# the last row, up to the last entry that 32-bit row pointers can count, through each
+# row kernel: a step past its end must not wrap round
+@pytest.mark.parametrize("tail_rows,degree,configs", [
+    (12, 5, [{}]), (900, 60, [{}]), (3000, 9, [{}]),
+    (1500, 40, [dict(heavy_split=1 << 30), dict(heavy_split=1 << 30, lanes_per_row=16)]),
+    (3000, 60, [{}, FORCED, dict(FORCED, heavy_split=1 << 30), dict(FORCED, heavy_vcap=8192),
+                dict(heavy_split=1, dense_max_words=2048)]),
+    (3000, 400, [{}])])
+def test_the_last_entries_of_a_full_matrix(tail_rows, degree, configs):
+    from appt_spgemm_b200._capi import SpgemmError
+    from appt_spgemm_b200.engine import Engine
+    needs_memory(90 << 30)
+    A, tail = most_entries((1 << 31) - 1, tail_rows, degree, seed=degree)
+    for cfg in configs:
+        with Engine("cuda:0", **cfg) as e:
+            check_last_rows(e, A, tail, str(cfg))
+    A.col[-1] = A.col[-2]  # not increasing
+    with Engine("cuda:0") as e, pytest.raises(SpgemmError, match="strictly increase"):
+        e.multiply(A, "AA")

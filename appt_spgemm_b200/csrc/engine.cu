@@ -615,12 +615,13 @@ bool small_plan_eligible(const spg_ctx* ctx, spg_task task, const spg_csr_dev* A
          A->nnz <= c.small_max_nnz && A->n <= kSmallMaxN && !c.force_heavy;
 }
 
-// The heavy rows' classes as the one list that they are.
+// The classes of the heavy and of the paneled rows as the one list each that they are.
 void merge_heavy(int64_t* count) {
-  for (int c = 1; c < kHeavyClasses; ++c) {
-    count[kHeavyBin] += count[kHeavyBin + c];
-    count[kHeavyBin + c] = 0;
-  }
+  for (int b : {kHeavyBin, kPanelBin0})
+    for (int c = 1; c < kHeavyClasses; ++c) {
+      count[b] += count[b + c];
+      count[b + c] = 0;
+    }
 }
 
 spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
@@ -736,7 +737,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   BinSource bsym{0, n, p->f, p->lo, p->hi, nullptr, kMaxTableLog2, force,
                  ctx->cfg.sym_load_pct,
                  numeric_heavy_min(num_lg, ctx->cfg.num_load_pct),
-                 p->A.rowptr, split, short_lg,
+                 p->A.rowptr, p->A.col, split, short_lg,
                  numeric_heavy_min(short_lg, ctx->cfg.num_load_pct), dense_lw, 0, panels,
                  pre.lead, pre.runlen, pre.need};
   // column blocks of the heavy rows: 1024 columns (windows are packed from
@@ -844,7 +845,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     ProfScope ps(ctx, "sym/bin", bs, b);
     TRY_CUDA(launch_hash_bin(b, false, r, ctx->num_sms, bs), "symbolic");
   }
-  for (int b = kNarrowBin0; b < kNumBins; ++b) {
+  for (int b = kNarrowBin0; b < kPanelBin0; ++b) {
     if (sym_count[b] == 0) continue;
     RowArgs r = ra;
     r.rows = rows_sym + sym_start[b];
@@ -894,8 +895,8 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   // numeric binning by exact counts, stats; host sync #2 (nnz(C))
   TRY(palloc(p, &p->rows_num, n));
   BinSource bnum{1, n, p->f, p->lo, p->hi, p->rownnz, num_lg, force,
-                 ctx->cfg.num_load_pct, 0, p->A.rowptr, split, short_lg, 0, dense_lw,
-                 1, panels, pre.lead, pre.runlen, pre.need};
+                 ctx->cfg.num_load_pct, 0, p->A.rowptr, p->A.col, split, short_lg, 0, dense_lw,
+                 1, panels && p->pan_log2 > 0 && p->blk_cnt, pre.lead, pre.runlen, pre.need};
   {
     ProfScope ps(ctx, "plan/bin_num", st);
     TRY_CUDA(launch_bin_rows(bnum, bin, work_num, p->rows_num, st),
@@ -918,7 +919,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   p->info.products_computed = (int64_t)sv[0];
   p->info.max_row_products = (int64_t)sv[1];
   p->info.max_row_nnz = (int64_t)sv[2];
-  p->info.heavy_rows = p->num_count[kHeavyBin];
+  p->info.heavy_rows = p->num_count[kHeavyBin] + p->num_count[kPanelBin0];
   p->heavy_windows = p->num_count[kHeavyBin] > 0 && p->blk_cnt;
   for (int b = 1; b < kNumBins; ++b)
     if (p->num_count[b] > 0) ++bins_used;
@@ -927,14 +928,14 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   p->info.workspace_bytes = p->ws_bytes;
   // the panels' slice bounds (an int per row of B and panel) may take an eighth
   // of C's size; beyond that the panels search for them
-  if (p->heavy_windows && p->pan_log2 > 0) {
+  if (p->num_count[kPanelBin0] > 0) {
     p->npan = ((n - 1) >> p->pan_log2) + 1;
     p->pan_table = 4 * (int64_t)n * (p->npan + 1) <=
                    std::max<int64_t>((int64_t)64 << 20, p->info.output_bytes / 8);
   }
   p->info.exec_workspace_bytes =
       (p->heavy_windows ? 16 * Ad->nnz : 0) +
-      (p->npan > 0 ? panel_workspace(n, p->npan, p->num_count[kHeavyBin], p->pan_table) : 0);
+      (p->npan > 0 ? panel_workspace(n, p->npan, p->num_count[kPanelBin0], p->pan_table) : 0);
   return SPG_OK;
 }
 
@@ -1003,12 +1004,12 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
     }
     void* panel_ws = nullptr;
     if (p->npan > 0 &&
-        (result = talloc(&panel_ws, (size_t)panel_workspace(n, p->npan, p->num_count[kHeavyBin],
+        (result = talloc(&panel_ws, (size_t)panel_workspace(n, p->npan, p->num_count[kPanelBin0],
                                                             p->pan_table))) != SPG_OK)
       break;
     int launches = p->small && n > 0 ? 1 : 0;
     for (int b = 1; b < kNumBins; ++b)
-      if (p->num_count[b] > 0) launches += b == kHeavyBin && p->heavy_windows ? 3 : 1;
+      if (p->num_count[b] > 0) launches += b == kHeavyBin && p->heavy_windows ? 2 : 1;
     BinFork fork(ctx, st, launches);
     if (p->small && n > 0) {
       RowArgs r = ra;
@@ -1035,7 +1036,7 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       cudaError_t e = launch_hash_bin(b, true, r, ctx->num_sms, bs);
       if (e != cudaSuccess) result = cuda_status(e, "numeric");
     }
-    for (int b = kNarrowBin0; b < kNumBins && result == SPG_OK; ++b) {
+    for (int b = kNarrowBin0; b < kPanelBin0 && result == SPG_OK; ++b) {
       if (p->num_count[b] == 0) continue;
       RowArgs r = ra;
       r.rows = p->rows_num + p->num_start[b];
@@ -1079,7 +1080,24 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       if (e != cudaSuccess) result = cuda_status(e, "numeric");
     }
     if (result != SPG_OK) break;
-    if (p->num_count[kHeavyBin] > 0) {
+    if (p->num_count[kPanelBin0] > 0 && result == SPG_OK) {
+      HeavyArgs h{};
+      h.r = ra;
+      h.r.rows = p->rows_num + p->num_start[kPanelBin0];
+      h.r.nrows = (int32_t)p->num_count[kPanelBin0];
+      h.lo = p->lo;
+      h.hi = p->hi;
+      h.blk_off = p->blk_off;
+      h.blk_cnt = p->blk_cnt;
+      h.blk_log2 = p->blk_log2;
+      h.pan_log2 = p->pan_log2;
+      h.npan = p->npan;
+      const cudaStream_t bs = fork.next();
+      ProfScope ps(ctx, "num/panels", bs);
+      const cudaError_t e = launch_panels(h, panel_ws, p->pan_table, ctx->num_sms, bs);
+      if (e != cudaSuccess) result = cuda_status(e, "numeric panels");
+    }
+    if (p->num_count[kHeavyBin] > 0 && result == SPG_OK) {
       HeavyArgs h{};
       h.r = ra;
       h.r.rows = p->rows_num + p->num_start[kHeavyBin];
@@ -1109,15 +1127,8 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       const int win_threads = ctx->cfg.heavy_threads > 512 ? 1024 : 512;
       h.vcap = ctx->cfg.heavy_vcap > 0 ? (int32_t)ctx->cfg.heavy_vcap : 8192;
       h.wcap_bits = win_threads > 512 ? (1 << 18) : (1 << 17);
-      h.pan_log2 = p->pan_log2;
-      h.npan = p->npan;
       cudaError_t e = cudaSuccess;
-      if (p->npan > 0) {
-        const cudaStream_t bs = fork.next();
-        ProfScope ps(ctx, "num/panels", bs);
-        e = launch_panels(h, panel_ws, p->pan_table, ctx->num_sms, bs);
-      }
-      if (e == cudaSuccess && windows) {
+      if (windows) {
         const cudaStream_t bs = fork.next();
         ProfScope ps(ctx, "num/heavy_w32", bs);
         e = launch_heavy_w32(h, ctx->num_sms, bs);

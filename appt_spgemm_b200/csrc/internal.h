@@ -53,7 +53,10 @@ constexpr int kRunBin0 = kSortBin0 + kSortBins;  // 30
 constexpr int kNarrowBins = 8;
 constexpr int kNarrowMin = 128;
 constexpr int kNarrowBin0 = kRunBin0 + kRunBins;  // 34
-constexpr int kNumBins = kNarrowBin0 + kNarrowBins;  // 42
+// Rows cut into panels (numeric phase only; heavy rows in the symbolic one), in as
+// many bins and in the same order as the heavy rows.
+constexpr int kPanelBin0 = kNarrowBin0 + kNarrowBins;  // 42
+constexpr int kNumBins = kPanelBin0 + kHeavyClasses;   // 48
 constexpr int kDenseVals = 256;  // entries of a bitmap-path row (numeric)
 
 }  // namespace spg

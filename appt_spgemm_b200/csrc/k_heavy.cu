@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num(HeavyArgs h) {
     const int hi = h.hi[row];
     const int lo = h.lo[row];
     const long long expect = (long long)a.cnt_in[row];
-    if (heavy_row_paneled(h, row) || heavy_row_windowed(h, row)) continue;  // another kernel's row
+    if (heavy_row_windowed(h, row)) continue;  // the windowed warp kernel's row
     const int64_t base = a.rowptr[row];
     const int cb = a.colbase ? a.colbase[row] : 0;
     long long written = 0;

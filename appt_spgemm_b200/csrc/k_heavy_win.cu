@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
     const int r = cta_item(h.queue, a.nrows, it, &s_next);
     if (r >= a.nrows) break;
     const int row = a.rows[r];
-    if (heavy_row_paneled(h, row) || heavy_row_windowed(h, row)) continue;  // the windowed warp kernel's row
+    if (heavy_row_windowed(h, row)) continue;  // the windowed warp kernel's row
     const int lo = h.lo[row], hi = h.hi[row];
     const int lo_r = lo;
     const long long expect = (long long)a.cnt_in[row];

@@ -82,8 +82,8 @@ __global__ void k_panel_bounds(MatView B, int pan_log2, int npan, int32_t* __res
   }
 }
 
-// One CTA: the task offsets of the rows, a task per panel of those that take
-// panels; off[nrows] is the number of tasks.  The rows are listed by product
+// One CTA: the task offsets of the rows, a task per panel; off[nrows] is the number
+// of tasks.  The rows are listed by product
 // count, largest first, so a hub row's tasks start early and none of them is
 // left to the end.
 constexpr int kOffsetThreads = 1024, kOffsetRows = 8;
@@ -96,8 +96,7 @@ __global__ void __launch_bounds__(kOffsetThreads) k_panel_offsets(HeavyArgs h,
   __syncthreads();
   for (int r0 = 0; r0 < nrows; r0 += kOffsetThreads * kOffsetRows) {
     // each step's loads issued together (rows past the end count the last one)
-    int n[kOffsetRows], lo[kOffsetRows], hi[kOffsetRows], len[kOffsetRows], sum = 0;
-    int64_t f[kOffsetRows];
+    int n[kOffsetRows], lo[kOffsetRows], hi[kOffsetRows], sum = 0;
 #pragma unroll
     for (int u = 0; u < kOffsetRows; ++u)
       n[u] = h.r.rows[min(r0 + tid * kOffsetRows + u, nrows - 1)];
@@ -105,13 +104,12 @@ __global__ void __launch_bounds__(kOffsetThreads) k_panel_offsets(HeavyArgs h,
     for (int u = 0; u < kOffsetRows; ++u) {
       lo[u] = h.lo[n[u]];
       hi[u] = h.hi[n[u]];
-      f[u] = h.f[n[u]];
-      len[u] = h.r.A.rowptr[n[u] + 1] - h.r.A.rowptr[n[u]];
     }
 #pragma unroll
     for (int u = 0; u < kOffsetRows; ++u) {
-      const bool takes = r0 + tid * kOffsetRows + u < nrows && paneled_row(f[u], len[u], lo[u], hi[u]);
-      n[u] = takes ? (hi[u] >> h.pan_log2) - (lo[u] >> h.pan_log2) + 1 : 0;
+      n[u] = r0 + tid * kOffsetRows + u < nrows
+                 ? (hi[u] >> h.pan_log2) - (lo[u] >> h.pan_log2) + 1
+                 : 0;
       sum += n[u];
     }
     int tot;

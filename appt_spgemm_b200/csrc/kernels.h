@@ -52,20 +52,40 @@ constexpr int64_t kSortMaxProducts = 4096;
 constexpr int64_t kSortMaxMerge2 = 3;
 constexpr int64_t kSortMaxMerge2Large = 6;  // beyond the warp kernels' largest table
 
-// Paneled rows: the fewest products, the narrowest span, the fewest products per
-// 1024 columns of it and, up to kWarpRowMaxProducts products, the fewest per
-// entry of A's row there (a slice of a B row) for rows within and beyond the
-// sorted rows' range.  Measured per call, 48-matrix batch (Erdős–Rényi rows of
-// 1,000 products, slices of 2 to 4) / R-MAT 2^16 / 2^13: slices of 2 for all
-// rows 10.70 / 5.97 / 0.88 ms, of 5 for all 8.63 / 6.56 / 0.88, as below
-// 8.62 / 5.97 / 0.88; tables and sorted rows up to 5,400 entries as before the
-// panels 8.58 / 6.51 / 1.62.
-constexpr int64_t kPanelMinRow = 256;
-constexpr int64_t kPanelMinWideRow = 800;  // over three panels or more: a 27-point row stays hashed
+// Paneled rows: the narrowest span and the fewest products, in all and per 1024
+// columns (a panel costs its task, its slice bounds and a walk over its columns
+// whatever it holds).
+//
+// Rows beyond the sorted rows' range have heavy kernels as their alternative.  From
+// kPanelManyProducts a panel on, panels win whatever the row looks like; below, where
+// the entries of A have slices worth it (kPanelMinSlice products a panel on average)
+// and, over many panels, there are entries enough (the alternative's cost is a barrier
+// per entry).  Measured per call, panels / heavy kernels, 2,000 rows over 200,000
+// columns: 32 entries of 500 products (82 a panel) 2.40 / 1.25 ms, 32 of 1,000 (163)
+// 2.75 / 2.09, 64 of 1,000 (326) 2.28 / 4.80; hub rows of an R-MAT-like graph, 388
+// entries over 17 panels (358 products, less than one a slice) 0.52 / 3.24 ms; the hub
+// row of an arrowhead of 40,000 went to a single warp, 12.6 -> 4.4 ms.  R-MAT 2^16
+// (64 panels) / 2^17 / 2^18, without the condition on the entries 5.26 / 16.5 / 47.3
+// ms, with it 5.87 / 15.5 / 43.2, beyond 64 panels only (as below) 5.25 / 15.5 / 43.2.
+//
+// Smaller rows could be sorted or hashed.  Panels serve them where B's rows are long
+// (hubs: kPanelMinMean), or where slices are (kPanelMinSliceSmall) and the row keeps
+// kPanelMinEntries entries a panel: a table of few entries is small.  Few are kept
+// where the columns of A's row are neighbours (a mesh with several unknowns per node),
+// which is all that the symbolic phase can see of it.  Per call, panels / tables,
+// 5-point grid of 150 x 150 with six unknowns a node 3.39 / 1.05 ms, four 0.65 / 0.48;
+// 27-point grid 34^3 with two 2.97 / 2.49; Erdos-Renyi 3,000 rows of 40 0.26 / 0.34 ms,
+// 1,100 of 28 0.20 / 0.29; none of these rows in panels: R-MAT 2^12 0.65 -> 0.82 ms.
 constexpr int32_t kPanelMinSpan = 600;
 constexpr int64_t kPanelMinProducts = 64;
-constexpr int64_t kPanelMinSliceSmall = 5;
+constexpr int64_t kPanelManyProducts = 192;
 constexpr int64_t kPanelMinSlice = 2;
+constexpr int64_t kPanelFewPanels = 64;
+constexpr int64_t kPanelMinRow = 256;
+constexpr int64_t kPanelMinWideRow = 800;  // over three panels or more
+constexpr int64_t kPanelMinSliceSmall = 5;
+constexpr int64_t kPanelMinMean = 64;
+constexpr int64_t kPanelMinEntries = 48;
 // one warp walks a windowed heavy row alone: a larger row would set its tail
 constexpr int64_t kWarpRowMaxProducts = (int64_t)1 << 17;
 
@@ -103,7 +123,7 @@ struct BinSource {
   // min(products, span) >= short_min (symbolic): the windowed warp kernel
   // serves them better than the CTA-per-row tables, whose per-k barrier idles
   // most of the CTA on short B rows
-  const int32_t* arowptr;
+  const int32_t *arowptr, *acol;
   int64_t short_split;
   int short_max_log2;
   int64_t short_min;
@@ -115,7 +135,7 @@ struct BinSource {
   // numeric: rows of up to kSortMaxProducts products of which few
   // merge take the sorted-row kernels
   int sort_rows;
-  // rows for the panel kernel go heavy whatever their table (0: no such rule)
+  // rows for the panel kernel, whatever their table (0: none)
   int panels;
   // runs of shifted rows (nullptr: none): rows back to the run's first row, and
   // at that row the run's length and the doubles 32 of its rows need
@@ -204,17 +224,35 @@ __host__ __device__ __forceinline__ int heavy_class(int64_t f) {
   return c;
 }
 
-// A row of f products from `len` entries of A over columns [lo, hi]: cut into
-// panels?  By its products and span alone, so that the symbolic and the numeric
-// binning agree.
-__host__ __device__ __forceinline__ bool paneled_row(int64_t f, int32_t len, int32_t lo,
-                                                     int32_t hi) {
+// Are the row's columns (len of them, sorted) mostly runs of neighbours?  By eight
+// of its entries.  Neighbouring rows of B then hold much the same columns: the
+// unknowns of a mesh's node, or the neighbours of a grid point.
+__host__ __device__ __forceinline__ bool clumped_columns(const int32_t* cols, int32_t len) {
+  int next = 0;
+  for (int t = 0; t < 8; ++t) {
+    const int32_t p = (int32_t)((int64_t)(len - 1) * t >> 3);
+    next += p + 1 < len && cols[p + 1] == cols[p] + 1;
+  }
+  return next >= 4;
+}
+
+// A row of f products from `len` entries of A (their columns: cols) over columns
+// [lo, hi]: cut into panels?  `entries`: its entries, -1 while they are not known
+// (symbolic phase: a row that is heavy there for its panels may be hashed in the
+// numeric phase, but not the reverse, for want of its column counts).
+__host__ __device__ __forceinline__ bool paneled_row(int64_t f, int32_t len, const int32_t* cols,
+                                                     int32_t lo, int32_t hi, int64_t entries) {
   if (f < kPanelMinRow || hi - lo < kPanelMinSpan) return false;
   const int64_t panels = (hi >> 10) - (lo >> 10) + 1;
-  if (panels > 2 && f < kPanelMinWideRow) return false;
-  return f >= kPanelMinProducts * panels &&
-         (f > kWarpRowMaxProducts ||
-          f >= (f > kSortMaxProducts ? kPanelMinSlice : kPanelMinSliceSmall) * panels * len);
+  if (f < kPanelMinProducts * panels) return false;
+  if (f > kSortMaxProducts)
+    return f >= kPanelManyProducts * panels ||
+           (f >= kPanelMinSlice * panels * len &&
+            (panels <= kPanelFewPanels || 2 * (int64_t)len >= panels));
+  if (f < kPanelMinSliceSmall * panels * len || (panels > 2 && f < kPanelMinWideRow)) return false;
+  if (f >= kPanelMinMean * len) return true;
+  if (entries >= 0 && entries < kPanelMinEntries * panels) return false;
+  return !clumped_columns(cols, len);
 }
 
 // Table size rule: symbolic tables hold keys only and are sized for the load
@@ -242,9 +280,10 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
   }
   if (s.mode == 1 && s.lead && s.runlen[i])
     return kRunBin0 + run_team(size, s.need[i], s.f[i], (int64_t)s.hi[i] - s.lo[i] + 1);
-  if (s.force_heavy ||
-      (s.panels && paneled_row(s.f[i], s.arowptr[i + 1] - s.arowptr[i], s.lo[i], s.hi[i])))
-    return kHeavyBin;
+  if (s.panels && paneled_row(s.f[i], s.arowptr[i + 1] - s.arowptr[i], s.acol + s.arowptr[i],
+                              s.lo[i], s.hi[i], s.mode == 1 ? size : -1))
+    return s.mode == 1 ? kPanelBin0 : kHeavyBin;
+  if (s.force_heavy) return kHeavyBin;
   int lg = table_log2(size, s.load_pct);
   if (s.mode == 1 && s.sort_rows && lg <= s.max_log2 &&
       sorted_row(s.f[i], size, (int64_t)s.hi[i] - s.lo[i] + 1,
@@ -281,8 +320,8 @@ constexpr int kBinRowsPerBlock = 256;  // rows per block of the binning kernels
 // Binning: the rows of each bin listed one bin after another (in row order within
 // blocks of kBinRowsPerBlock rows).
 //   bin: a byte per row; work: kBinWork int64 on the device, of which the first
-//   kNumBins + 1 come back: the rows of each bin, and (symbolic) the blocks of
-//   1024 columns that the heavy rows span
+//   kNumBins + 1 come back: the rows of each bin, and the blocks of 1024 columns
+//   that the heavy (symbolic phase) or the paneled rows (numeric) span
 constexpr int kBinWork = 2 * kNumBins + 1;
 // `skip` (device, may be null): where it is not 0 nothing is done (work stays 0).
 cudaError_t launch_bin_rows(const BinSource& src, uint8_t* bin, int64_t* work, int32_t* rows_out,
@@ -474,21 +513,15 @@ struct HeavyArgs {
   int32_t* queue;
   // panel kernel (k_panel.cu): panels of 2^pan_log2 columns, npan of them over
   // n columns; slice bounds (nullptr: searched for) and task counter set by
-  // launch_panels (npan 0: no row takes it)
+  // launch_panels
   int32_t pan_log2, npan;
   const int32_t* ptr;
   int64_t* task_queue;
 };
 
-__device__ __forceinline__ bool heavy_row_paneled(const HeavyArgs& h, int row) {
-  return h.npan > 0 && paneled_row(h.f[row], h.r.A.rowptr[row + 1] - h.r.A.rowptr[row],
-                                   h.lo[row], h.hi[row]);
-}
-
 // The heavy row goes to the windowed warp kernel: mean B-row length
 // f / nnz(A row) below split, and at most kWarpRowMaxProducts products.
 __device__ __forceinline__ bool heavy_row_windowed(const HeavyArgs& h, int row) {
-  if (heavy_row_paneled(h, row)) return false;
   if (h.split <= 0 || h.f[row] > kWarpRowMaxProducts) return false;
   const int64_t len = (int64_t)h.r.A.rowptr[row + 1] - h.r.A.rowptr[row];
   return h.f[row] < h.split * len;

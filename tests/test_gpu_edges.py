@@ -169,3 +169,65 @@ def test_the_last_entries_of_a_full_matrix(tail_rows, degree, configs):
     A.col[-1] = A.col[-2]  # not increasing
     with Engine("cuda:0") as e, pytest.raises(SpgemmError, match="strictly increase"):
         e.multiply(A, "AA")
+
+
+def from_rows(n, rows, seed):
+    rows = [np.unique(np.asarray(r, dtype=np.int64)) for r in rows]
+    rp = np.zeros(n + 1, dtype=np.int32)
+    rp[1:len(rows) + 1] = np.cumsum([len(r) for r in rows])
+    rp[len(rows) + 1:] = rp[len(rows)]
+    col = np.concatenate(rows).astype(np.int32)
+    return csr.CsrHost(n, rp, col, np.random.default_rng(seed).uniform(-1, 1, len(col)))
+
+
+def unknowns(A, k):
+    """k unknowns per node of A's mesh: every entry a k x k block."""
+    rows = []
+    for i in range(A.n):
+        c = A.col[A.rowptr[i]:A.rowptr[i + 1]].astype(np.int64)
+        rows += [(c[:, None] * k + np.arange(k)).ravel()] * k
+    return from_rows(A.n * k, rows, k)
+
+
+def long_b_rows(n, rows, entries, length):
+    """`rows` rows of `entries` entries, which point at 400 rows of `length`."""
+    rng = np.random.default_rng(n + entries)
+    lists = [rng.integers(400, n, length) for _ in range(400)]
+    lists += [rng.choice(400, entries, replace=False) for _ in range(rows)]
+    return from_rows(n, lists, 3)
+
+
+def arrowhead(n, width):
+    rows = [np.concatenate([[0], np.arange(max(0, i - width), min(n, i + width + 1))])
+            for i in range(n)]
+    rows[0] = np.arange(0, n, 7)
+    return from_rows(n, rows, 5)
+
+
+# which rows are worth a panel: meshes with several unknowns per node keep their tables
+# (one panel's products merge into few entries), as do long rows with few products per
+# panel; random rows and hubs take panels, all of an arrowhead's
+@pytest.mark.parametrize("A,panels,windows", [
+    (lambda: unknowns(csr.laplace2d(60), 6), False, False),
+    (lambda: unknowns(csr.laplace2d(40), 8), False, False),
+    (lambda: unknowns(csr.stencil27(20, 1), 2), False, False),
+    (lambda: unknowns(csr.stencil27(14, 1), 3), True, None),
+    (lambda: csr.erdos_renyi(3000, 40.0, 1), True, None),
+    (lambda: long_b_rows(200000, 500, 32, 500), False, None),
+    (lambda: long_b_rows(200000, 500, 64, 800), True, None),
+    (lambda: long_b_rows(50000, 500, 64, 100), True, None),
+    (lambda: arrowhead(6000, 3), True, False)],
+    ids=["grid6", "grid8", "cube2", "cube3", "random", "few-products", "many-products",
+         "many-entries", "arrowhead"])
+def test_rows_worth_a_panel(A, panels, windows):
+    from appt_spgemm_b200.engine import Engine
+    A = A()
+    with Engine("cuda:0", small_max_nnz=-1) as e:
+        for task in ("AA", "AAt"):
+            got = []
+            ran = kernels(e, lambda: got.append(e.multiply(dev(A), task)))
+            e.check_device_status()
+            assert_same_csr(got[0].to_host(), oracle.multiply(A, task), task)
+            if task == "AA":
+                assert ("num/panels" in ran) == panels, ran
+                assert windows is None or ("num/heavy_w32" in ran) == windows, ran

@@ -876,6 +876,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     h.blk_cnt = p->blk_cnt;
     h.blk_log2 = p->blk_log2;
     h.queue = p->hqueue + kHeavyBin;
+    h.f = p->f;
     const cudaStream_t bs = fork.next();
     ProfScope ps(ctx, "sym/heavy", bs);
     TRY_CUDA(launch_heavy(false, h, p->heavy_threads, ctx->num_sms, bs),

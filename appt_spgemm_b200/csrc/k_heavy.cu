@@ -40,12 +40,30 @@ size_t heavy_smem_bytes(bool numeric, int threads, int window_bits) {
 // warp each.
 constexpr int kLongBRow = 256;
 
+// Marks bit d of a bitmap of wbits.  MERGING: most bits are set already, so they are
+// looked at first (the atomics of neighbouring columns are one after another on
+// their word: dense 2,000 x 2,000, symbolic 33 -> 10 ms; random rows of
+// 32 products a column 1.78 against 1.71 ms).
+template <bool MERGING>
+__device__ __forceinline__ void mark_bit(uint32_t* bm, long long d, long long wbits) {
+  if (d < 0 || d >= wbits) return;
+  const uint32_t bit = 1u << (d & 31);
+  if (MERGING && (*(volatile uint32_t*)&bm[d >> 5] & bit)) return;
+  atomicOr(&bm[d >> 5], bit);
+}
+
+constexpr int64_t kMarkMerging = 64;  // products per column spanned
+__device__ __forceinline__ bool row_merges(const HeavyArgs& h, int row) {
+  return h.f[row] >= kMarkMerging * ((int64_t)h.hi[row] - h.lo[row] + 1);
+}
+
 // Mark the columns of row `row` that fall in [w0, w0 + 32·nwords) in the shared
 // bitmap.  Marking is an OR, so
 // the B rows need no order: per chunk of blockDim entries of A's row, the
 // long B rows (listed in st_long) are swept by the whole CTA one after another
 // and the short ones are dealt out to the warps, a B row per warp — no search
 // for the B row of a product.
+template <bool MERGING>
 __device__ __forceinline__ void mark_window(const RowArgs& a, int row, long long w0, int nwords,
                                             uint32_t* bm, int* st_bs, int* st_len, int* st_long,
                                             void* scratch) {
@@ -72,16 +90,14 @@ __device__ __forceinline__ void mark_window(const RowArgs& a, int row, long long
       const int t = st_long[i];
       const int32_t b = st_bs[t], l = st_len[t];
       for (int q = tid; q < l; q += blockDim.x) {
-        const long long d = (long long)a.B.col[b + q] - w0;
-        if (d >= 0 && d < wbits) atomicOr(&bm[d >> 5], 1u << (d & 31));
+        mark_bit<MERGING>(bm, (long long)a.B.col[b + q] - w0, wbits);
       }
     }
     for (int t = wid; t < cnt; t += nwarps) {
       const int32_t b = st_bs[t], l = st_len[t];
       if (l >= kLongBRow) continue;
       for (int q = lane; q < l; q += 32) {
-        const long long d = (long long)a.B.col[b + q] - w0;
-        if (d >= 0 && d < wbits) atomicOr(&bm[d >> 5], 1u << (d & 31));
+        mark_bit<MERGING>(bm, (long long)a.B.col[b + q] - w0, wbits);
       }
     }
     __syncthreads();  // staging and the long-row count are reused by the next chunk
@@ -106,6 +122,7 @@ __global__ void __launch_bounds__(1024, 2) k_heavy_sym(HeavyArgs h) {
     if (r >= a.nrows) break;
     const int row = a.rows[r];
     const int lo = h.lo[row], hi = h.hi[row];
+    const bool merging = row_merges(h, row);
     long long c = 0;
     // windows start on a column block's first column
     const int lo_blk = lo >> h.blk_log2 << h.blk_log2;
@@ -113,7 +130,8 @@ __global__ void __launch_bounds__(1024, 2) k_heavy_sym(HeavyArgs h) {
       const int nwords = (int)min((long long)nw_max, (hi - w0) / 32 + 1);
       for (int i = threadIdx.x; i < nwords; i += blockDim.x) bm[i] = 0u;
       __syncthreads();
-      mark_window(a, row, w0, nwords, bm, st_bs, st_ex, st_long, scratch);
+      if (merging) mark_window<true>(a, row, w0, nwords, bm, st_bs, st_ex, st_long, scratch);
+      else mark_window<false>(a, row, w0, nwords, bm, st_bs, st_ex, st_long, scratch);
       // a warp per column block of the window (32 or more words): the bit
       // counts are the row totals and, when asked for, the block counts
       int lc = 0;
@@ -179,6 +197,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num(HeavyArgs h) {
     const int row = a.rows[r];
     const int hi = h.hi[row];
     const int lo = h.lo[row];
+    const bool merging = row_merges(h, row);
     const long long expect = (long long)a.cnt_in[row];
     if (heavy_row_windowed(h, row)) continue;  // the windowed warp kernel's row
     const int64_t base = a.rowptr[row];
@@ -189,7 +208,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num(HeavyArgs h) {
       const int ngroups = (nwords + 3) >> 2;
       for (int i = tid; i < ngroups * 4; i += HT) bm[i] = 0u;
       __syncthreads();
-      mark_window(a, row, w0, nwords, bm, st_bs, st_ex, st_long, scratch);
+      if (merging) mark_window<true>(a, row, w0, nwords, bm, st_bs, st_ex, st_long, scratch);
+      else mark_window<false>(a, row, w0, nwords, bm, st_bs, st_ex, st_long, scratch);
       // exclusive prefix of the bit counts per group of 4 words
       const int per = (ngroups + HT - 1) / HT;
       const int gb = min(ngroups, tid * per), ge = min(ngroups, gb + per);

@@ -231,3 +231,29 @@ def test_rows_worth_a_panel(A, panels, windows):
             if task == "AA":
                 assert ("num/panels" in ran) == panels, ran
                 assert windows is None or ("num/heavy_w32" in ran) == windows, ran
+
+
+def dense(n):
+    return csr.CsrHost(n, (np.arange(n + 1) * n).astype(np.int32),
+                       np.tile(np.arange(n, dtype=np.int32), n),
+                       np.random.default_rng(n).uniform(-1, 1, n * n))
+
+
+def test_marking_rows_that_merge():
+    # rows whose products fall on a few columns time after time are marked with a look
+    # before the atomic: no slower than their sums; rows either side of that line
+    from appt_spgemm_b200.engine import Engine
+    with Engine("cuda:0") as e:
+        A = dev(dense(2000))
+        for _ in range(2):
+            e.profile_enable(True)
+            e.profile_reset()
+            e.multiply(A, "AA")
+            torch.cuda.synchronize()
+            ms = {k: v["ms"] for k, v in e.profile_read()["kernels"].items()}
+        assert ms["sym/heavy"] < ms["num/panels"], ms
+    with Engine("cuda:0", force_heavy=1) as e:
+        for B in (dense(63), dense(64), dense(65), dense(300), csr.erdos_renyi(300, 140.0, 3)):
+            C = e.multiply(dev(B), "AA")
+            e.check_device_status()
+            assert_same_csr(C.to_host(), oracle.multiply(B, "AA"), str(B.n))

@@ -412,7 +412,7 @@ int64_t plan_workspace_bound(const spg_config& cfg, spg_task task, int64_t n, in
          + scan + 4 * nz + 8 * nz + 4 * nn + 4;   // scan, staging copy, long list
   }
   b += 8 * nn + 4 * nn + 4 * nn + 4;                              // f, lo, hi, queue
-  b += 16 * nn + 8 * prepass_pieces(nz) + 8 + 7 * nn;                             // pre-pass, runs
+  b += 16 * nn + 8 * prepass_pieces(nz) + 12 + 7 * nn;                             // pre-pass, runs
   b += nn + 8 * (2 * kBinWork + kRowStats) + 4 * nn;              // binning, statistics
   b += 4 * nn + 8 * (nn + 1) + scan;                              // heavy block offsets
   const int64_t per_row_blocks = (nn + 1023) / 1024 + 1;
@@ -725,7 +725,8 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   pre.hi = p->hi;
   TRY(palloc(p, &pre.info, n));
   TRY(palloc(p, &pre.pieces, prepass_pieces(Ad->nnz)));
-  TRY(palloc(p, &pre.marks, 2));
+  TRY(palloc(p, &pre.marks, 3));
+  pre.mid = rows_sym;  // (listed later)
   TRY(palloc(p, &pre.flag_a, n));
   TRY(palloc(p, &pre.need, n));
   if (runs) {

@@ -492,7 +492,7 @@ constexpr int kRowsAhead = 4;      // rows whose loads a group has in flight tog
 // CTA; every index is checked before it is used, and a row that meets one out
 // of range gets f = −1.  Rows of more than kLongRow entries are listed, a piece
 // {row, first entry} at a time, for k_prepass_long.  marks: {pieces listed,
-// rows flagged}.  Bound by the latency of entry -> row of B, hence four rows of
+// rows flagged, rows listed}.  Bound by the latency of entry -> row of B, hence four rows of
 // a group at a time where none is longer than the group.
 constexpr int kRunBlock = 256;
 constexpr int kShortLanes = 8;  // lanes per row of the matrices that take k_prepass_short
@@ -616,13 +616,15 @@ __global__ void __launch_bounds__(256) k_prepass_rows(
 // The same with a thread per row, for matrices of few entries a row: a group of
 // eight lanes spends its instructions on the reductions (5-point grid 1009²:
 // 94 -> 20 µs with the row's entries in turn, four loads in flight).  Rows of
-// more than kThreadRow entries are taken by whole warps afterwards.
+// more than kThreadRow entries are listed for the warps of k_prepass_long (a warp
+// that took its own 32 rows' one after another: 120 against 24 µs where 2,000 rows
+// of 64 entries lie together among 100,000).
 constexpr int kThreadRow = 16;
 __global__ void __launch_bounds__(256) k_prepass_short(
     MatView A, int32_t n_b, const int4* __restrict__ info, int64_t* __restrict__ f,
     int32_t* __restrict__ lo, int32_t* __restrict__ hi, uint8_t* __restrict__ flag,
     int2* __restrict__ pieces, int64_t max_pieces, int32_t* __restrict__ marks,
-    uint32_t* status, const int* skip) {
+    int32_t* __restrict__ mid, uint32_t* status, const int* skip) {
   if (skip && *skip) return;
   const int lane = threadIdx.x & 31;
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -665,19 +667,13 @@ __global__ void __launch_bounds__(256) k_prepass_short(
       }
     }
   }
-  for (unsigned more = __ballot_sync(kFull, len > kThreadRow && len <= kLongRow); more;
-       more &= more - 1u) {
-    const int src = __ffs((int)more) - 1;
-    const int32_t ws = __shfl_sync(kFull, s, src), we = __shfl_sync(kFull, e, src);
-    const bool wc = __shfl_sync(kFull, (int)candidate, src);
-    RowSums w;
-    const bool ws_same = w.add<true>(A, info, n_b, ws, ws + lane, we, 32, wc ? we - ws : 0);
-    const bool all = __all_sync(kFull, ws_same);
-    w.reduce(WarpGroup(32));
-    if (lane == src) {
-      t = w;
-      same = all && wc;
-    }
+  const bool is_mid = len > kThreadRow && len <= kLongRow;
+  const unsigned mids = __ballot_sync(kFull, is_mid);
+  if (mids) {
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&marks[2], __popc(mids));
+    at = __shfl_sync(kFull, at, 0) + __popc(mids & lanemask_lt());
+    if (is_mid) mid[at] = (int32_t)i;
   }
   if (len > kLongRow) {
     const int pc = (len + kLongPiece - 1) / kLongPiece;
@@ -688,27 +684,25 @@ __global__ void __launch_bounds__(256) k_prepass_short(
       for (int c = 0; c < pc; ++c) pieces[at + c] = make_int2((int)i, s + c * kLongPiece);
   }
   const bool bad = t.bad || wrong;
-  if (on) {
+  if (on && !is_mid) {
     if (bad) report(status, DEV_ERR_INVALID_CSR);
     f[i] = bad ? -1 : t.products();
     lo[i] = bad ? INT_MAX : t.mn;
     hi[i] = bad ? -1 : t.mx;
     flag[i] = same && !bad;
   }
-  const int flagged = __syncthreads_count(on && same && !bad);
+  const int flagged = __syncthreads_count(on && !is_mid && same && !bad);
   if (threadIdx.x == 0 && flagged) atomicAdd(&marks[1], flagged);
 }
 
-// The listed pieces.
-__global__ void __launch_bounds__(256) k_prepass_long(MatView A, int32_t n_b,
-                                                      const int4* __restrict__ info,
-                                                      int64_t* f, int32_t* lo, int32_t* hi,
-                                                      const int2* __restrict__ pieces,
-                                                      int64_t max_pieces,
-                                                      const int32_t* __restrict__ marks,
-                                                      uint32_t* status) {
-  const int n = marks[0];
-  if (n < 0 || n > max_pieces) return;  // A is invalid, and some pieces are not listed
+// The listed pieces, a CTA each, and the listed rows, a warp each.
+__global__ void __launch_bounds__(256) k_prepass_long(
+    MatView A, int32_t n_b, const int4* __restrict__ info, int64_t* f, int32_t* lo, int32_t* hi,
+    uint8_t* __restrict__ flag, const int2* __restrict__ pieces, int64_t max_pieces,
+    const int32_t* __restrict__ mid, int32_t* marks, uint32_t* status) {
+  const int lane = threadIdx.x & 31;
+  int n = marks[0];
+  if (n < 0 || n > max_pieces) n = 0;  // A is invalid, and some pieces are not listed
   for (int c = blockIdx.x; c < n; c += gridDim.x) {
     const int2 piece = pieces[c];
     const Pos s = A.rowptr[piece.x];
@@ -716,13 +710,33 @@ __global__ void __launch_bounds__(256) k_prepass_long(MatView A, int32_t n_b,
     RowSums t;
     t.add<false>(A, info, n_b, s, (Pos)piece.y + threadIdx.x, e, blockDim.x, 0);
     t.reduce(WarpGroup(32));
-    if ((threadIdx.x & 31) == 0) {
+    if (lane == 0) {
       if (t.bad) report(status, DEV_ERR_INVALID_CSR);
       atomicAdd((unsigned long long*)&f[piece.x], (unsigned long long)t.products());
       atomicMin(&lo[piece.x], t.mn);
       atomicMax(&hi[piece.x], t.mx);
     }
   }
+  const int rows = marks[2];
+  int flagged = 0;
+  for (int r = (blockIdx.x * 256 + threadIdx.x) >> 5; r < rows; r += gridDim.x * 8) {
+    const int32_t i = mid[r];  // (its row pointers were checked)
+    const int32_t s = A.rowptr[i], e = A.rowptr[i + 1], s1 = i > 0 ? A.rowptr[i - 1] : -1;
+    const bool candidate = e - s <= kMaxLen && s1 >= 0 && s - s1 == e - s;
+    RowSums t;
+    bool same = t.add<true>(A, info, n_b, s, (Pos)s + lane, e, 32, candidate ? e - s : 0);
+    same = __all_sync(kFull, same) && candidate;
+    t.reduce(WarpGroup(32));
+    if (lane == 0) {
+      if (t.bad) report(status, DEV_ERR_INVALID_CSR);
+      f[i] = t.bad ? -1 : t.products();
+      lo[i] = t.bad ? INT_MAX : t.mn;
+      hi[i] = t.bad ? -1 : t.mx;
+      flag[i] = same && !t.bad;
+      flagged += same && !t.bad;
+    }
+  }
+  if (flagged) atomicAdd(&marks[1], flagged);
 }
 
 // Too few rows of A are their predecessor shifted for runs to matter.
@@ -899,7 +913,7 @@ cudaError_t launch_runs(int team, const RowArgs& a, int num_sms, cudaStream_t s)
 cudaError_t launch_prepass_rows(const MatView& A, const MatView& B, const PrepassArrays& w,
                                 int num_sms, uint32_t* status, cudaStream_t s, const int* skip) {
   if (A.n == 0) return launch_validate(A, status, s);
-  cudaError_t e = cudaMemsetAsync(w.marks, 0, 2 * sizeof(int32_t), s);
+  cudaError_t e = cudaMemsetAsync(w.marks, 0, 3 * sizeof(int32_t), s);
   if (e != cudaSuccess) return e;
   const int G = lanes_for(A);
   const unsigned blocks = (unsigned)(((int64_t)A.n + kRunBlock - 1) / kRunBlock);
@@ -910,15 +924,17 @@ cudaError_t launch_prepass_rows(const MatView& A, const MatView& B, const Prepas
   while (rows > kRowsAhead * (256 / G) && rows > 32 && A.n / rows < num_sms * 8) rows >>= 1;
   if (G == kShortLanes)
     k_prepass_short<<<blocks, 256, 0, s>>>(A, B.n, w.info, w.f, w.lo, w.hi, w.flag_a, w.pieces,
-                                           prepass_pieces(A.nnz), w.marks, status, skip);
+                                           prepass_pieces(A.nnz), w.marks, w.mid, status,
+                                           skip);
   else
     k_prepass_rows<<<(unsigned)((A.n + rows - 1) / rows), 256, 0, s>>>(
         A, B.n, w.info, G, rows, w.f, w.lo, w.hi, w.flag_a, w.pieces, prepass_pieces(A.nnz),
         w.marks, status, skip);
   SPG_COUNT_LAUNCH();
-  if (A.nnz > kLongRow) {
-    k_prepass_long<<<num_sms * 4, 256, 0, s>>>(A, B.n, w.info, w.f, w.lo, w.hi, w.pieces,
-                                               prepass_pieces(A.nnz), w.marks, status);
+  if (A.nnz > kThreadRow) {
+    k_prepass_long<<<num_sms * 4, 256, 0, s>>>(A, B.n, w.info, w.f, w.lo, w.hi, w.flag_a,
+                                               w.pieces, prepass_pieces(A.nnz), w.mid, w.marks,
+                                               status);
     SPG_COUNT_LAUNCH();
   }
   if (!w.lead) return cudaGetLastError();

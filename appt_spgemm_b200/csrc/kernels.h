@@ -461,14 +461,14 @@ cudaError_t launch_narrow(bool numeric, int W, int lanes, const RowArgs& a, int 
                           cudaStream_t s);
 // The pre-pass of the regular plans (k_runs.cu): products and column span per
 // row, the validation of A and, with `lead`, the runs of shifted rows.  Per row
-// of B: info; per row of A: the others; marks: two ints; pieces:
+// of B: info; per row of A: the others (mid: scratch); marks: three ints; pieces:
 // prepass_pieces(nnz).
 // (rows of more than 256 entries, in pieces of 1024: at most 1.25 nnz / 256)
 constexpr int64_t prepass_pieces(int64_t nnz) { return nnz / 200 + 1; }
 struct PrepassArrays {
   int4* info;
   int64_t* f;
-  int32_t *lo, *hi, *marks;
+  int32_t *lo, *hi, *marks, *mid;
   int2* pieces;
   uint8_t *flag_a, *flag_b, *lead;
   uint16_t *need, *runlen;

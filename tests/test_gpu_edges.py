@@ -257,3 +257,33 @@ def test_marking_rows_that_merge():
             C = e.multiply(dev(B), "AA")
             e.check_device_status()
             assert_same_csr(C.to_host(), oracle.multiply(B, "AA"), str(B.n))
+
+
+def test_prepass_of_longer_rows_together():
+    # 2,000 rows of 64 entries next to one another among rows of two: the pre-pass takes
+    # no longer than with the same rows spread over the matrix
+    from appt_spgemm_b200.engine import Engine
+    n, step = 100000, 47
+    rng = np.random.default_rng(1)
+    longer = [np.unique(rng.integers(0, n, 64)) for _ in range(2000)]
+    took = {}
+    with Engine("cuda:0", small_max_nnz=-1) as e:
+        for name, at in (("together", np.arange(400, 2400)), ("spread", np.arange(2000) * step)):
+            rows = [[i, (i * 7) % n] for i in range(n)]
+            for i, r in zip(at, longer):
+                rows[i] = r
+            A = from_rows(n, rows, 2)
+            C = e.multiply(dev(A), "AA")
+            assert_same_csr(C.to_host(), oracle.multiply(A, "AA"), name)
+            d = dev(A)
+            e.profile_enable(True)
+            times = []
+            for _ in range(9):
+                e.profile_reset()
+                e.multiply(d, "AA")
+                torch.cuda.synchronize()
+                times.append(e.profile_read()["kernels"]["plan/prepass"]["ms"])
+            e.profile_enable(False)
+            took[name] = np.median(times)
+        e.check_device_status()
+    assert took["together"] < 1.7 * took["spread"], took

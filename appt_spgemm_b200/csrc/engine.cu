@@ -577,7 +577,9 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   p->info.max_row_nnz = (int64_t)sv[2];
   p->info.heavy_rows = 0;
   p->info.bins_used = 1;
-  p->info.symmetric_pattern = p->task == SPG_TASK_AATS && words[1] == 0;
+  // (Aᵀ of a symmetric pattern is A's with other values: later executes gather them)
+  p->symmetric = p->task == SPG_TASK_AATS && words[1] == 0;
+  p->info.symmetric_pattern = p->symmetric;
   // numeric table: the exact largest row at the numeric load, 16 to 2048
   // slots; tables below 2048 slots run rows on lane groups sized to B's mean
   // row length (several rows per warp), 2048 a warp per row

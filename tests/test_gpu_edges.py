@@ -287,3 +287,27 @@ def test_prepass_of_longer_rows_together():
             took[name] = np.median(times)
         e.check_device_status()
     assert took["together"] < 1.7 * took["spread"], took
+
+
+def test_symmetric_small_plan_gathers_its_transpose():
+    # a plan of the symmetric variant executed again: the values of A^T by one launch
+    # (its pattern is A's), then the product; an unsymmetric one transposes
+    from appt_spgemm_b200.engine import Engine
+    sym, unsym = csr.laplace2d(50), csr.erdos_renyi(900, 5.0, 3)
+    with Engine("cuda:0") as e:
+        launches = {}
+        for name, A in (("sym", sym), ("unsym", unsym)):
+            A.val = np.random.default_rng(4).uniform(-1, 1, A.nnz)
+            d = dev(A)
+            p = e.plan(d, "AAtS")
+            assert p.info["symmetric_pattern"] == (name == "sym")
+            C = p.execute()
+            d.val.copy_(torch.from_numpy(A.val[::-1].copy()))  # other values, same pattern
+            e.profile_reset()
+            p.execute(C)
+            launches[name] = e.profile_read()["launches"]
+            e.check_device_status()
+            B = csr.CsrHost(A.n, A.rowptr, A.col, A.val[::-1].copy())
+            assert_same_csr(C.to_host(), oracle.multiply(B, "AAtS"), name)
+            p.close()
+    assert launches["sym"] == 2 < launches["unsym"], launches

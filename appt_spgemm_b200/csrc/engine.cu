@@ -762,19 +762,19 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
       ProfScope ps(ctx, "plan/bin_sym", st);
       TRY_CUDA(launch_bin_rows(bsym, bin, work, rows_sym, st, skip), "symbolic binning");
     }
-    TRY_CUDA(cudaMemcpyAsync(hp, work, sizeof(int64_t) * (kNumBins + 1), cudaMemcpyDeviceToHost,
+    TRY_CUDA(cudaMemcpyAsync(hp, work, sizeof(int64_t) * kBinBack, cudaMemcpyDeviceToHost,
                              st), "bin readback");
-    TRY_CUDA(cudaMemcpyAsync(hp + kNumBins + 1, ctx->d_status, 2 * sizeof(uint32_t),
+    TRY_CUDA(cudaMemcpyAsync(hp + kBinBack, ctx->d_status, 2 * sizeof(uint32_t),
                              cudaMemcpyDeviceToHost, st), "status readback");
     TRY_CUDA(cudaStreamSynchronize(st), "bin sync");
-    const uint32_t* words = (const uint32_t*)(hp + kNumBins + 1);
+    const uint32_t* words = (const uint32_t*)(hp + kBinBack);
     if (words[0] & DEV_ERR_INVALID_CSR) return status_from_bits(DEV_ERR_INVALID_CSR);
     return SPG_OK;
   };
   // (a pattern found not to be symmetric by now is binned once, transposed; A is
   // then validated in that pass)
   TRY(bin_pass(p->symmetric ? (const int*)(ctx->d_status + 1) : nullptr));
-  if (p->symmetric && ((const uint32_t*)(hp + kNumBins + 1))[1] != 0) {
+  if (p->symmetric && ((const uint32_t*)(hp + kBinBack))[1] != 0) {
     // A·Aᵀ of a pattern that is not symmetric: transpose and bin again
     TRY(build_transpose());
     TRY(bin_pass(nullptr));
@@ -930,12 +930,15 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   p->info.bins_used = bins_used;
   p->info.output_bytes = 8 * ((int64_t)n + 1) + 12 * p->nnz_c;
   p->info.workspace_bytes = p->ws_bytes;
-  // the panels' slice bounds (an int per row of B and panel) may take an eighth
-  // of C's size; beyond that the panels search for them
+  // the panels' slice bounds (an int per row of B and panel), where they are used
+  // often enough, may take an eighth of C's size; else the panels search for them
   if (p->num_count[kPanelBin0] > 0) {
     p->npan = ((n - 1) >> p->pan_log2) + 1;
-    p->pan_table = 4 * (int64_t)n * (p->npan + 1) <=
-                   std::max<int64_t>((int64_t)64 << 20, p->info.output_bytes / 8);
+    const int64_t entries = (int64_t)n * (p->npan + 1);
+    const int64_t slices = (p->pan_log2 > 10 ? hp[kNumBins + 1] >> (p->pan_log2 - 10)
+                                             : hp[kNumBins + 1] << (10 - p->pan_log2));
+    p->pan_table = entries <= kPanelTableEntries * slices &&
+                   4 * entries <= std::max<int64_t>((int64_t)64 << 20, p->info.output_bytes / 8);
   }
   p->info.exec_workspace_bytes =
       (p->heavy_windows ? 16 * Ad->nnz : 0) +

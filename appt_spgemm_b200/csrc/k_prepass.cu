@@ -151,22 +151,28 @@ __global__ void __launch_bounds__(256) k_bin_count(BinSource src, uint8_t* __res
                                                    const int* skip) {
   if (skip && *skip) return;
   __shared__ int cnt[kNumBins];
-  __shared__ unsigned long long blocks;
+  __shared__ unsigned long long blocks, slices;
   if (threadIdx.x < kNumBins) cnt[threadIdx.x] = 0;
-  if (threadIdx.x == 0) blocks = 0;
+  if (threadIdx.x == 0) blocks = slices = 0;
   __syncthreads();
   const int64_t base = (int64_t)blockIdx.x * kBinRowsPerBlock;
   for (int t = threadIdx.x; t < kBinRowsPerBlock; t += blockDim.x) {
     const int64_t i = base + t;
     int b = i < src.n ? row_bin(src, (int)i) : -1;
     unsigned nb = 0;
+    unsigned long long ns = 0;
     if (b == kHeavyBin || b == kPanelBin0) {
       if (src.mode == 0 || b == kPanelBin0) nb = (src.hi[i] >> 10) - (src.lo[i] >> 10) + 1;
+      if (b == kPanelBin0) ns = (unsigned long long)nb * (src.arowptr[i + 1] - src.arowptr[i]);
       b += heavy_class(src.f[i]);
     }
     if (__any_sync(0xffffffffu, nb > 0)) {  // (an atomic per row: 30 µs on 2,000 heavy rows)
       nb = __reduce_add_sync(0xffffffffu, nb);
-      if ((threadIdx.x & 31) == 0) atomicAdd(&blocks, (unsigned long long)nb);
+      for (int o = 16; o > 0; o >>= 1) ns += __shfl_xor_sync(0xffffffffu, ns, o);
+      if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&blocks, (unsigned long long)nb);
+        if (ns) atomicAdd(&slices, ns);
+      }
     }
     const unsigned same = __match_any_sync(0xffffffffu, b);
     if (b < 0) continue;
@@ -177,6 +183,7 @@ __global__ void __launch_bounds__(256) k_bin_count(BinSource src, uint8_t* __res
   if (threadIdx.x < kNumBins && cnt[threadIdx.x])
     atomicAdd(&work[threadIdx.x], (unsigned long long)cnt[threadIdx.x]);
   if (threadIdx.x == 0 && blocks) atomicAdd(&work[kNumBins], blocks);
+  if (threadIdx.x == 0 && slices) atomicAdd(&work[kNumBins + 1], slices);
 }
 
 __global__ void __launch_bounds__(256) k_bin_scatter(int64_t n, const uint8_t* __restrict__ bin,
@@ -204,7 +211,7 @@ __global__ void __launch_bounds__(256) k_bin_scatter(int64_t n, const uint8_t* _
   if (tid < kNumBins) {
     unsigned long long start = 0;
     for (int k = 0; k < tid; ++k) start += work[k];
-    place[tid] = cnt[tid] ? (int)(start + atomicAdd(&work[kNumBins + 1 + tid],
+    place[tid] = cnt[tid] ? (int)(start + atomicAdd(&work[kBinBack + tid],
                                                     (unsigned long long)cnt[tid]))
                           : 0;
   }

@@ -86,6 +86,12 @@ constexpr int64_t kPanelMinWideRow = 800;  // over three panels or more
 constexpr int64_t kPanelMinSliceSmall = 5;
 constexpr int64_t kPanelMinMean = 64;
 constexpr int64_t kPanelMinEntries = 48;
+// Slice bounds are tabulated for every row of B and panel where that is at most so
+// many bounds per slice that the paneled rows read (each saves its two searches).  Per
+// call with / without the table at 0.08 bounds a slice (R-MAT 2^16) 5.25 / 8.71 ms,
+// 1.6 (long rows over 100,000 columns) 1.43 / 2.06, 3.2 1.22 / 1.32, 7.6 10.54 / 10.62,
+// 30 and 600 (a few hub rows) no difference beyond 10 µs, for 57 MB.
+constexpr int64_t kPanelTableEntries = 8;
 // one warp walks a windowed heavy row alone: a larger row would set its tail
 constexpr int64_t kWarpRowMaxProducts = (int64_t)1 << 17;
 
@@ -320,9 +326,11 @@ constexpr int kBinRowsPerBlock = 256;  // rows per block of the binning kernels
 // Binning: the rows of each bin listed one bin after another (in row order within
 // blocks of kBinRowsPerBlock rows).
 //   bin: a byte per row; work: kBinWork int64 on the device, of which the first
-//   kNumBins + 1 come back: the rows of each bin, and the blocks of 1024 columns
-//   that the heavy (symbolic phase) or the paneled rows (numeric) span
-constexpr int kBinWork = 2 * kNumBins + 1;
+//   kBinBack come back: the rows of each bin; the blocks of 1024 columns that the
+//   heavy (symbolic phase) or the paneled rows (numeric) span, and the slices of B
+//   rows that the latter read there (blocks times entries of A)
+constexpr int kBinBack = kNumBins + 2;
+constexpr int kBinWork = kBinBack + kNumBins;
 // `skip` (device, may be null): where it is not 0 nothing is done (work stays 0).
 cudaError_t launch_bin_rows(const BinSource& src, uint8_t* bin, int64_t* work, int32_t* rows_out,
                             cudaStream_t s, const int* skip = nullptr);

@@ -311,3 +311,23 @@ def test_symmetric_small_plan_gathers_its_transpose():
             assert_same_csr(C.to_host(), oracle.multiply(B, "AAtS"), name)
             p.close()
     assert launches["sym"] == 2 < launches["unsym"], launches
+
+
+def table_bytes(n):
+    return 4 * n * (((n - 1) >> 10) + 2)
+
+
+# the table of the panels' slice bounds, an int per row of B and panel of 1024 columns:
+# taken where its bounds are read often, not for a few rows among many
+@pytest.mark.parametrize("n,rows,table", [(60000, 2, False), (60000, 2000, True)])
+def test_panel_table_only_where_it_is_used(n, rows, table):
+    from appt_spgemm_b200.engine import Engine
+    A = long_b_rows(n, rows, 40, 800)
+    with Engine("cuda:0", small_max_nnz=-1) as e:
+        p = e.plan(dev(A), "AA")
+        assert (p.info["exec_workspace_bytes"] >= table_bytes(n)) == table, p.info
+        got = []
+        assert "num/panels" in kernels(e, lambda: got.append(p.execute()))
+        e.check_device_status()
+        assert_same_csr(got[0].to_host(), oracle.multiply(A, "AA"), str(rows))
+        p.close()

@@ -626,6 +626,12 @@ void merge_heavy(int64_t* count) {
     }
 }
 
+void set_exec_workspace(spg_plan* p) {
+  p->info.exec_workspace_bytes =
+      (p->heavy_windows ? 16 * p->A.nnz : 0) +
+      (p->npan > 0 ? panel_workspace(p->n, p->npan, p->num_count[kPanelBin0], p->pan_table) : 0);
+}
+
 spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   spg_ctx* ctx = p->ctx;
   cudaStream_t st = p->stream;
@@ -940,9 +946,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
     p->pan_table = entries <= kPanelTableEntries * slices &&
                    4 * entries <= std::max<int64_t>((int64_t)64 << 20, p->info.output_bytes / 8);
   }
-  p->info.exec_workspace_bytes =
-      (p->heavy_windows ? 16 * Ad->nnz : 0) +
-      (p->npan > 0 ? panel_workspace(n, p->npan, p->num_count[kPanelBin0], p->pan_table) : 0);
+  set_exec_workspace(p);
   return SPG_OK;
 }
 
@@ -1010,10 +1014,17 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       hcur = (int4*)hc;
     }
     void* panel_ws = nullptr;
-    if (p->npan > 0 &&
-        (result = talloc(&panel_ws, (size_t)panel_workspace(n, p->npan, p->num_count[kPanelBin0],
-                                                            p->pan_table))) != SPG_OK)
-      break;
+    bool pan_table = p->pan_table;
+    if (p->npan > 0) {
+      const int64_t rows = p->num_count[kPanelBin0];
+      result = talloc(&panel_ws, (size_t)panel_workspace(n, p->npan, rows, pan_table));
+      if (result == SPG_ERR_OOM && pan_table) {  // the table is a convenience: search instead
+        clear_error();
+        pan_table = false;
+        result = talloc(&panel_ws, (size_t)panel_workspace(n, p->npan, rows, false));
+      }
+      if (result != SPG_OK) break;
+    }
     int launches = p->small && n > 0 ? 1 : 0;
     for (int b = 1; b < kNumBins; ++b)
       if (p->num_count[b] > 0) launches += b == kHeavyBin && p->heavy_windows ? 2 : 1;
@@ -1101,7 +1112,7 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       h.npan = p->npan;
       const cudaStream_t bs = fork.next();
       ProfScope ps(ctx, "num/panels", bs);
-      const cudaError_t e = launch_panels(h, panel_ws, p->pan_table, ctx->num_sms, bs);
+      const cudaError_t e = launch_panels(h, panel_ws, pan_table, ctx->num_sms, bs);
       if (e != cudaSuccess) result = cuda_status(e, "numeric panels");
     }
     if (p->num_count[kHeavyBin] > 0 && result == SPG_OK) {
@@ -1177,6 +1188,11 @@ spg_task parse_task(const char* t, bool* ok) {
 }
 
 }  // namespace
+
+void spg::plan_spare_workspace(spg_plan* p) {
+  p->pan_table = false;
+  set_exec_workspace(p);
+}
 
 extern "C" {
 

@@ -15,6 +15,10 @@ spg_status set_error(spg_status st, const char* fmt, ...)
     ;
 void clear_error();
 
+// Executes of `plan` do without the workspace that only makes them faster (its info
+// says what they then take).
+void plan_spare_workspace(spg_plan* plan);
+
 // ---- device status word bits (kernels atomicOr these; host maps to status) ----
 enum DeviceErrorBits : uint32_t {
   DEV_ERR_HASH_FULL = 1u << 0,  // bounded probe exhausted

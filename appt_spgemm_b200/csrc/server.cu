@@ -150,6 +150,16 @@ void split_into_requests(const Job& j, std::vector<Job>& split) {
   }
 }
 
+// A planned job that exceeds the whole budget only by workspace that it can do without
+// does without it.
+void spare_workspace(const spg_server* s, Job& j) {
+  if (j.need() <= s->cfg.memory_budget_bytes) return;
+  j.temp -= j.info.exec_workspace_bytes;
+  spg::plan_spare_workspace(j.p);
+  spg_plan_get_info(j.p, &j.info);
+  j.temp += j.info.exec_workspace_bytes;
+}
+
 // Plan `j` (one request or a batch).  Returns false when the job is gone: a
 // single request that failed to plan is finished with the error; a batch
 // that failed to plan is split into single-request jobs appended to `split`.
@@ -165,6 +175,7 @@ bool plan_job(spg_server* s, spg_ctx* ctx, cudaStream_t st, Job& j, std::vector<
     spg_plan_get_info(j.p, &j.info);
     j.outs = output_bytes(r->A.n, j.info.nnz_c);
     j.temp = j.info.workspace_bytes + j.info.exec_workspace_bytes;
+    spare_workspace(s, j);
     std::lock_guard<std::mutex> lk(s->mu);
     hold(s, j.info.workspace_bytes);
     r->products = j.info.products;
@@ -193,6 +204,7 @@ bool plan_job(spg_server* s, spg_ctx* ctx, cudaStream_t st, Job& j, std::vector<
   }
   j.temp = output_bytes(j.info.n, j.info.nnz_c) + j.info.workspace_bytes +
            j.info.exec_workspace_bytes;
+  spare_workspace(s, j);
   std::lock_guard<std::mutex> lk(s->mu);
   hold(s, j.info.workspace_bytes);
   const double t = s->now_ms();

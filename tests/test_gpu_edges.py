@@ -331,3 +331,53 @@ def test_panel_table_only_where_it_is_used(n, rows, table):
         e.check_device_status()
         assert_same_csr(got[0].to_host(), oracle.multiply(A, "AA"), str(rows))
         p.close()
+
+
+def test_panels_without_memory_for_their_table():
+    # the table is taken for speed alone: an execute that cannot have it searches
+    from appt_spgemm_b200.engine import Engine
+    A = long_b_rows(120000, 1000, 60, 800)
+    ref = oracle.multiply(A, "AA")
+    torch.cuda.empty_cache()
+    with Engine("cuda:0", small_max_nnz=-1, pool_release_bytes=1) as e:
+        p = e.plan(dev(A), "AA")
+        nnz = int(p.info["nnz_c"])
+        assert p.info["exec_workspace_bytes"] >= table_bytes(A.n) > 50 << 20
+        from appt_spgemm_b200.engine import CsrResult
+        C = CsrResult(A.n, nnz, torch.zeros(A.n + 1, dtype=torch.int64, device="cuda:0"),
+                      torch.zeros(nnz, dtype=torch.int32, device="cuda:0"),
+                      torch.zeros(nnz, dtype=torch.float64, device="cuda:0"))
+        torch.cuda.synchronize()
+        hog, chunk = [], 1 << 34
+        while chunk >= 1 << 21:  # the rest of the memory, down to a few MB
+            try:
+                hog.append(torch.empty(chunk, dtype=torch.uint8, device="cuda:0"))
+            except torch.OutOfMemoryError:
+                chunk >>= 1
+        try:
+            p.execute(C)
+            torch.cuda.synchronize()
+        finally:
+            hog.clear()
+            torch.cuda.empty_cache()
+        e.check_device_status()
+        assert_same_csr(C.to_host(), ref, "without the table")
+        p.close()
+
+
+def test_server_runs_what_fits_without_the_table():
+    from appt_spgemm_b200.engine import Engine, Server
+    A = long_b_rows(60000, 2000, 40, 800)
+    d = dev(A)
+    with Engine("cuda:0") as e:
+        p = e.plan(d, "AA")
+        need = sum(p.info[k] for k in ("workspace_bytes", "exec_workspace_bytes", "output_bytes"))
+        p.close()
+    with Server(workers=1, memory_budget_bytes=need - table_bytes(A.n) // 2, batch_rows=1) as srv:
+        rid = srv.submit(d, "AA")
+        info = srv.wait(rid)
+        assert info["status"] == 0
+        assert_same_csr(srv.result(rid).to_host(), oracle.multiply(A, "AA"), "served")
+        srv.release(rid)
+        st = srv.stats()
+        assert st["rejected"] == 0 and st["peak_held_bytes"] <= st["budget_bytes"]

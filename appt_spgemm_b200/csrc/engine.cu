@@ -198,6 +198,7 @@ struct spg_plan {
                               // (zeroed before each launch; bins may run at once)
   int pan_log2 = 0;           // heavy rows in panels of 2^pan_log2 columns (0: none)
   int npan = 0;
+  int64_t pan_tasks = 0;      // at most so many panels over all rows
   bool pan_table = false;     // their slice bounds are tabulated at each execute
   int window_bits = 1 << 20;  // heavy-path shape (heavy_shape)
   int heavy_threads = 1024;
@@ -940,9 +941,13 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   // often enough, may take an eighth of C's size; else the panels search for them
   if (p->num_count[kPanelBin0] > 0) {
     p->npan = ((n - 1) >> p->pan_log2) + 1;
-    const int64_t entries = (int64_t)n * (p->npan + 1);
-    const int64_t slices = (p->pan_log2 > 10 ? hp[kNumBins + 1] >> (p->pan_log2 - 10)
-                                             : hp[kNumBins + 1] << (10 - p->pan_log2));
+    // (as for the blocks: from 1024 columns to the panels' width)
+    auto scaled = [&](int64_t blocks, int64_t rows) {
+      return p->pan_log2 <= 10 ? blocks << (10 - p->pan_log2)
+                               : (blocks >> (p->pan_log2 - 10)) + 2 * rows;
+    };
+    p->pan_tasks = scaled(hp[kNumBins], p->num_count[kPanelBin0]);
+    const int64_t entries = (int64_t)n * (p->npan + 1), slices = scaled(hp[kNumBins + 1], 0);
     p->pan_table = entries <= kPanelTableEntries * slices &&
                    4 * entries <= std::max<int64_t>((int64_t)64 << 20, p->info.output_bytes / 8);
   }
@@ -1110,6 +1115,8 @@ spg_status execute_impl(spg_plan* p, spg_csr_out* C, cudaStream_t st) {
       h.blk_log2 = p->blk_log2;
       h.pan_log2 = p->pan_log2;
       h.npan = p->npan;
+      h.tasks = p->pan_tasks;
+      h.retire = ctx->num_sms > ctx->device_sms;
       const cudaStream_t bs = fork.next();
       ProfScope ps(ctx, "num/panels", bs);
       const cudaError_t e = launch_panels(h, panel_ws, pan_table, ctx->num_sms, bs);

@@ -20,6 +20,9 @@
 //    first (−0.0 becomes +0.0; nothing else changes), so the first addition
 //    gives 0.0 + product and the places still holding −0.0 at the end are the
 //    columns without an entry;
+//  - warps draw panels until none is left; in launches that are to leave their SMs to
+//    others now and then (grid_sms) there are as many warps as panels, up to the
+//    grid's limit, and each leaves after its share;
 //  - the symbolic phase's distinct-column counts per block give the panel's
 //    first slot in C, and the panel is written in column order.
 // R-MAT 2^16: the launches of the rows that were in CTAs 2.7 ms against 6.8
@@ -149,10 +152,16 @@ __global__ void __launch_bounds__(512) k_panel_num(HeavyArgs h, const int64_t* _
   double* acc = (double*)(smem + (size_t)wid * panel_warp_bytes(h.pan_log2));
   double2* slice = (double2*)(acc + W);  // 32 of {a_ik, B position of the run's product 0}
   const int64_t total = off[a.nrows];
+  int64_t share = total;
+  if (h.retire) {
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    if ((int64_t)blockIdx.x * (blockDim.x >> 5) + wid >= total) return;
+    share = (total + warps - 1) / warps;
+  }
   for (int x = lane; x < W; x += 32) acc[x] = __longlong_as_double(kAbsent);
   __syncwarp();
 
-  for (;;) {
+  for (; share > 0; --share) {
     int64_t t = 0;
     if (lane == 0) t = (int64_t)atomicAdd((unsigned long long*)h.task_queue, 1ull);
     t = __shfl_sync(kFull, t, 0);
@@ -358,8 +367,8 @@ cudaError_t launch_panels(HeavyArgs& h, void* workspace, bool table, int num_sms
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, bytes);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
-  const int64_t most = (int64_t)h.r.nrows * h.npan;  // tasks
-  const int64_t grid = std::min<int64_t>((int64_t)per_sm * num_sms, (most + warps - 1) / warps);
+  const int64_t grid =
+      std::max<int64_t>(1, std::min<int64_t>((int64_t)per_sm * num_sms, (h.tasks + warps - 1) / warps));
   kernel<<<(unsigned)grid, warps * 32, bytes, s>>>(h, off);
   SPG_COUNT_LAUNCH();
   return cudaGetLastError();

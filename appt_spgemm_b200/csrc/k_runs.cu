@@ -28,6 +28,7 @@
 // those runs): two entries' sums at a time 1.16, entries drawn by list length 1.16,
 // neighbouring runs to one CTA 1.16 ms;
 // the entries shared out by list length, or 16 warps a team (32 per SM): no change.
+#include <algorithm>
 #include <climits>
 
 #include "kernels.h"
@@ -932,7 +933,8 @@ cudaError_t launch_prepass_rows(const MatView& A, const MatView& B, const Prepas
         w.marks, status, skip);
   SPG_COUNT_LAUNCH();
   if (A.nnz > kThreadRow) {
-    k_prepass_long<<<num_sms * 4, 256, 0, s>>>(A, B.n, w.info, w.f, w.lo, w.hi, w.flag_a,
+    // (grid_sms asks for many CTAs, and few have anything to do)
+    k_prepass_long<<<std::min(num_sms * 4, 148 * 64), 256, 0, s>>>(A, B.n, w.info, w.f, w.lo, w.hi, w.flag_a,
                                                w.pieces, prepass_pieces(A.nnz), w.mid, w.marks,
                                                status);
     SPG_COUNT_LAUNCH();

@@ -525,6 +525,8 @@ struct HeavyArgs {
   int32_t pan_log2, npan;
   const int32_t* ptr;
   int64_t* task_queue;
+  int64_t tasks;            // at most so many panels
+  bool retire;              // a warp leaves after its share of them (grid_sms)
 };
 
 // The heavy row goes to the windowed warp kernel: mean B-row length

@@ -381,3 +381,34 @@ def test_server_runs_what_fits_without_the_table():
         srv.release(rid)
         st = srv.stats()
         assert st["rejected"] == 0 and st["peak_held_bytes"] <= st["budget_bytes"]
+
+
+def test_panels_leave_their_sms():
+    # grid_sms: CTAs leave after their share of the work, so that a small product on a
+    # stream of higher priority is done long before a large one that started first
+    from appt_spgemm_b200.engine import Engine
+    small, large = dev(csr.laplace2d(64)), dev(csr.erdos_renyi(40000, 150.0, 1))
+    low, high = torch.cuda.Stream(priority=0), torch.cuda.Stream(priority=-5)
+    with Engine("cuda:0", grid_sms=1 << 16) as el, Engine("cuda:0") as es:
+        A = csr.erdos_renyi(6000, 80.0, 2)
+        C = el.multiply(dev(A), "AA")  # the same values with a warp per panel
+        assert_same_csr(C.to_host(), oracle.multiply(A, "AA"), "retiring")
+        p = el.plan(large, "AA", stream=low)
+        C = p.execute(stream=low)
+        es.multiply(small, "AA", stream=high)
+        torch.cuda.synchronize()
+        start, mid, end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+        start.record(low)
+        assert "num/panels" in kernels(el, lambda: p.execute(C, stream=low))
+        torch.cuda.synchronize()
+        start.record(low)
+        p.execute(C, stream=low)
+        end.record(low)
+        es.multiply(small, "AA", stream=high)
+        mid.record(high)
+        torch.cuda.synchronize()
+        el.check_device_status()
+        es.check_device_status()
+        p.close()
+        assert start.elapsed_time(mid) < 0.5 * start.elapsed_time(end), (
+            start.elapsed_time(mid), start.elapsed_time(end))

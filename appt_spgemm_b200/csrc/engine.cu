@@ -718,7 +718,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
                                                  : kHeavySplitDefault;
   const int short_lg = std::min(num_lg, 11);
   // panels, unless the configuration shapes the heavy path itself
-  const int panels = ctx->cfg.heavy_split == 0 && ctx->cfg.heavy_vcap < 0;
+  const int panels = split == kHeavySplitDefault && ctx->cfg.heavy_vcap < 0;
   // bitmap bins: the largest bitmap the config allows
   int dense_lw = -1;
   if (ctx->cfg.dense_max_words >= (1 << kDenseMinLog2W)) {

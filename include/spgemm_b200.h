@@ -102,13 +102,13 @@ typedef struct spg_config {
                                  min(products, span), percent 20..90; 0 → 75     */
   int32_t num_load_pct;       /* numeric tables sized for at most this load of
                                  the exact row count, percent 20..90; 0 → 66     */
-  int32_t heavy_split;        /* 0 → heavy rows of enough products per 1024
-                                 columns are cut into panels, the others split
-                                 at 128; set: no panels, heavy rows of at most
-                                 2^17 products whose B rows average fewer
-                                 entries than this take the warp-per-row
-                                 windowed kernel, the others the CTA-per-row
-                                 kernel (1: all CTA)                           */
+  int32_t heavy_split;        /* heavy rows of at most 2^17 products whose B
+                                 rows average fewer entries than this take the
+                                 warp-per-row windowed kernel, the others the
+                                 CTA-per-row kernel (1: all CTA); 0 → 128.  At
+                                 0 and 128 rows of enough products per 1024
+                                 columns are cut into panels first, at other
+                                 values none are                               */
   int64_t pool_release_bytes; /* memory-pool release threshold; 0 → keep all    */
   int64_t heavy_block_budget; /* most per-block column counts kept for heavy
                                  rows (2 bytes each; blocks widen from 1024

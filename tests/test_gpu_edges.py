@@ -412,3 +412,14 @@ def test_panels_leave_their_sms():
         p.close()
         assert start.elapsed_time(mid) < 0.5 * start.elapsed_time(end), (
             start.elapsed_time(mid), start.elapsed_time(end))
+
+
+@pytest.mark.parametrize("split,panels", [(0, True), (128, True), (127, False), (1 << 30, False)])
+def test_the_default_split_written_out(split, panels):
+    from appt_spgemm_b200.engine import Engine
+    A = csr.rmat(12, 16, seed=2)
+    with Engine("cuda:0", heavy_split=split) as e:
+        got = []
+        ran = kernels(e, lambda: got.append(e.multiply(dev(A), "AA")))
+        assert ("num/panels" in ran) == panels, ran
+        assert_same_csr(got[0].to_host(), oracle.multiply(A, "AA"), str(split))

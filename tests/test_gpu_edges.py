@@ -423,3 +423,45 @@ def test_the_default_split_written_out(split, panels):
         ran = kernels(e, lambda: got.append(e.multiply(dev(A), "AA")))
         assert ("num/panels" in ran) == panels, ran
         assert_same_csr(got[0].to_host(), oracle.multiply(A, "AA"), str(split))
+
+
+# infinities, NaN and both zeros through each row kernel: what a place or a slot holds
+# to say that it has no entry must not be taken for a value, nor the reverse
+@pytest.mark.parametrize("A,kernel", [
+    (lambda: csr.erdos_renyi(3000, 45.0, 1), "num/panels"),
+    (lambda: csr.banded(3000, 40, 0.4, 2), "num/narrow"),
+    (lambda: csr.uniform(20011, 20, 3), "num/sort"),
+    (lambda: csr.stencil27(14, 4), "num/runs"),
+    (lambda: csr.uniform(3000, 2, 5), "num/bin")],
+    ids=["panels", "narrow", "sorted", "runs", "tables"])
+def test_special_values(A, kernel):
+    from appt_spgemm_b200.engine import Engine
+    A = A()
+    A.val = np.random.default_rng(6).choice(
+        [0.0, -0.0, 1.0, -1.0, 1e308, -1e308, 5e-324, np.inf, -np.inf, np.nan], A.nnz,
+        p=[0.2, 0.2, 0.2, 0.2, 0.05, 0.05, 0.05, 0.02, 0.02, 0.01])
+    with Engine("cuda:0", small_max_nnz=-1) as e:
+        for task in ("AA", "AAt", "AAtS"):
+            got = []
+            ran = kernels(e, lambda: got.append(e.multiply(dev(A), task)))
+            assert task != "AA" or any(x.startswith(kernel) for x in ran), ran
+            e.check_device_status()
+            rp, ci, cx = got[0].to_host()
+            orp, oci, ocx = oracle.multiply(A, task)
+            assert np.array_equal(rp, orp) and np.array_equal(ci, oci), task
+            nan = np.isnan(ocx)  # (which NaN is the hardware's choice)
+            assert nan.any() and np.isinf(ocx).any() and np.array_equal(np.isnan(cx), nan), task
+            assert np.array_equal(cx[~nan].view(np.int64), ocx[~nan].view(np.int64)), task
+
+
+def test_knobs_with_many_runs_per_bin():
+    # concurrent bins and retiring CTAs over thousands of runs, and panels beside them
+    from appt_spgemm_b200.engine import Engine
+    grid, side = csr.laplace2d(220), csr.stencil27(26, 2)
+    for cfg in (dict(bin_streams=4), dict(grid_sms=1 << 16), dict(bin_streams=4, grid_sms=1 << 16)):
+        with Engine("cuda:0", small_max_nnz=-1, **cfg) as e:
+            for A in (grid, side, csr.rmat(12, 16, seed=4)):
+                for task in ("AA", "AAt"):
+                    C = e.multiply(dev(A), task)
+                    e.check_device_status()
+                    assert_same_csr(C.to_host(), oracle.multiply(A, task), str(cfg))

@@ -614,8 +614,13 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
 
 bool small_plan_eligible(const spg_ctx* ctx, spg_task task, const spg_csr_dev* A) {
   const spg_config& c = ctx->cfg;
-  return c.small_max_nnz > 0 &&
-         A->nnz <= c.small_max_nnz && A->n <= kSmallMaxN && !c.force_heavy;
+  if (c.small_max_nnz <= 0 || A->nnz > c.small_max_nnz || A->n > kSmallMaxN || c.force_heavy)
+    return false;
+  // A row of A·Aᵀ has (nnz / n)² products on average at least (the squares of the
+  // column counts): beyond the table's rows the transpose would be for nothing.
+  // (small_max_nnz may exceed its default: in floating point)
+  const double mean = A->n > 0 ? (double)A->nnz / A->n : 0.0;
+  return task == SPG_TASK_AA || mean * mean <= (double)kSmallCap;
 }
 
 // The classes of the heavy and of the paneled rows as the one list each that they are.

@@ -465,3 +465,18 @@ def test_knobs_with_many_runs_per_bin():
                     C = e.multiply(dev(A), task)
                     e.check_device_status()
                     assert_same_csr(C.to_host(), oracle.multiply(A, task), str(cfg))
+
+
+# A·Aᵀ plans that cannot be small (a row of it has the squared mean degree of products or
+# more, against 1536) are not tried as such; either side of the line
+@pytest.mark.parametrize("degree,tried", [(39, True), (40, False), (60, False)])
+def test_hopeless_small_plans_are_not_tried(degree, tried):
+    from appt_spgemm_b200.engine import Engine
+    A = csr.uniform(2000, degree, degree)
+    with Engine("cuda:0") as e:
+        for task in ("AAt", "AAtS"):
+            got = []
+            ran = kernels(e, lambda: got.append(e.multiply(dev(A), task)))
+            assert ("sym/small" in ran) == tried, ran
+            e.check_device_status()
+            assert_same_csr(got[0].to_host(), oracle.multiply(A, task), task)

@@ -437,17 +437,17 @@ void plan_free(spg_plan* p) {
 }
 
 // The plan of a small A·A or A·Aᵀ with one host synchronisation.  The regular
-// plan waits three times (validation verdict, bin sizes, nnz(C)); on a
+// plan waits twice (the validation verdict with the bin sizes, then nnz(C)); on a
 // matrix of a few thousand rows those round trips and the per-bin launches
 // are most of the call.  Here every kernel runs before the verdict is known
 // (the pre-pass and the transpose check every index they use; a row with an
 // invalid index gets f = −1 and is skipped), every row takes one
-// warp-per-row symbolic launch with a 2048-slot table, and one readback
-// brings the verdict, nnz(C) and the row statistics together.  A·Aᵀ always
-// uses the counting-sort transpose (no symmetric-pattern shortcut, which would
-// need the verdict first).  A row of more than kSmallCap products reports
-// DEV_ERR_SMALL_CAP, and the caller plans again on the regular path
-// (*fallback).  Execute then runs one numeric launch over all rows.
+// warp-per-row symbolic launch with a table sized by n, and one readback
+// brings the verdict, nnz(C) and the row statistics together.  A·Aᵀ is planned
+// over the counting-sort transpose (the symmetric-pattern shortcut would need the
+// verdict first; the symmetric variant's later executes take it).  A row of more
+// than kSmallCap products reports DEV_ERR_SMALL_CAP, and the caller plans again on
+// the regular path (*fallback).  Execute then runs one numeric launch over all rows.
 spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) {
   *fallback = false;
   spg_ctx* ctx = p->ctx;
@@ -586,7 +586,6 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   // row length (several rows per warp), 2048 a warp per row
   int lg = ceil_log2_64((int64_t)sv[2] * 100 / ctx->cfg.num_load_pct + 1);
   p->small_log2 = lg < kMinTableLog2 ? kMinTableLog2 : (lg > 11 ? 11 : lg);
-  // products that hardly merge: sorted rows, sized from the largest row
   // narrow rows: by the widest row and the means over all rows
   if (n > 0 && sv[0] > 0 && sv[1] <= (unsigned long long)kNarrowMaxProducts &&
       (int64_t)sv[0] >= kNarrowMinProducts * n &&
@@ -595,6 +594,7 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
     while (p->small_narrow < (int64_t)sv[3]) p->small_narrow <<= 1;
     p->small_lanes = (int64_t)sv[0] > kNarrowHalfMean * nnz ? 32 : 16;
   }
+  // products that hardly merge: sorted rows, sized from the largest row
   if ((int64_t)sv[0] >= kSortMinProducts * n && sorted_row((int64_t)sv[1], kSortMaxProducts, n) &&
       2 * (int64_t)sv[0] <= kSortMaxMerge2 * p->nnz_c)
     p->small_sort = (int)sv[1];

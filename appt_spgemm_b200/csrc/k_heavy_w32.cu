@@ -181,13 +181,12 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
     const int row = a.rows[r];
     const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
     const int lo = h.lo[row], hi = h.hi[row];
-    const int lo_r = lo;
     const int64_t expect = (int64_t)a.cnt_in[row];
     if (!heavy_row_windowed(h, row)) continue;  // the CTA kernel's row
     const int64_t base = a.rowptr[row];
     int64_t written = 0;
-    if (lo_r <= hi) {
-      // cursors at the first B entry >= lo_r of every B row of the row
+    if (lo <= hi) {
+      // cursors at the first entry of every B row of the row
       for (Pos p = ps + lane; p < pe; p += 32) {
         const int32_t k = a.A.col[p];
         int s = a.B.rowptr[k];
@@ -198,14 +197,14 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
       const int64_t b0 = h.blk_off[row];
       const int nb = (int)(h.blk_off[row + 1] - b0);
       const uint16_t* cnt = h.blk_cnt + b0;
-      int b = (lo_r >> h.blk_log2) - (lo >> h.blk_log2);
+      int b = 0;
       const int lo_blk = lo >> h.blk_log2 << h.blk_log2;
       while (b < nb) {
         const int bstart = lo_blk + (b << h.blk_log2);
         if ((int)cnt[b] > h.cap) {
           // a dense block: fixed windows of sw columns
           const int bend = (int)min((int64_t)bstart + bw, (int64_t)hi + 1);
-          for (int c0 = max(bstart, lo_r); c0 < bend;) {
+          for (int c0 = max(bstart, lo); c0 < bend;) {
             const int c1 = min(bend, bstart + ((c0 - bstart) / sw + 1) * sw);
             written += heavy_window<LOG2T>(h, row, ps, pe, c0, c1, keys, vals,
                                                  base + written, expect - written);
@@ -214,7 +213,7 @@ __global__ void __launch_bounds__(64, 4) k_heavy_w32(HeavyArgs h) {
           ++b;
         } else {
           const int e = window_end(cnt, b, nb, h.cap, max_blocks);
-          const int c0 = max(bstart, lo_r);
+          const int c0 = max(bstart, lo);
           const int c1 = (int)min((int64_t)lo_blk + ((int64_t)e << h.blk_log2), (int64_t)hi + 1);
           written += heavy_window<LOG2T>(h, row, ps, pe, c0, c1, keys, vals, base + written,
                                                expect - written);

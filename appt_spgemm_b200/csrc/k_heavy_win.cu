@@ -84,14 +84,13 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
     const int row = a.rows[r];
     if (heavy_row_windowed(h, row)) continue;  // the windowed warp kernel's row
     const int lo = h.lo[row], hi = h.hi[row];
-    const int lo_r = lo;
     const long long expect = (long long)a.cnt_in[row];
     const int64_t base = a.rowptr[row];
     const int cb = a.colbase ? a.colbase[row] : 0;
     const Pos ps = a.A.rowptr[row], pe = a.A.rowptr[row + 1];
     long long written = 0;
-    if (lo_r <= hi) {
-      // cursors at the first B entry >= lo_r of every B row of the row
+    if (lo <= hi) {
+      // cursors at the first entry of every B row of the row
       for (Pos p = ps + tid; p < pe; p += HT) {
         const int32_t k = a.A.col[p];
         int s = a.B.rowptr[k];
@@ -102,7 +101,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
       const int nb = (int)(h.blk_off[row + 1] - b0);
       const uint16_t* cnt = h.blk_cnt + b0;
       // window walk state (thread 0): next block, next column inside a cut block
-      int wb = (lo_r >> bw_log2) - (lo >> bw_log2);
+      int wb = 0;
       const int lo_blk = lo >> bw_log2 << bw_log2;
       long long wsub = -1;
       for (;;) {
@@ -114,7 +113,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
             const long long bstart = (long long)lo_blk + ((long long)wb << bw_log2);
             const long long bend = min(bstart + bwidth, (long long)hi + 1);
             if ((int)cnt[wb] > vcap || bwidth > wcap) {
-              const long long s0 = wsub >= 0 ? wsub : max(bstart, (long long)lo_r);
+              const long long s0 = wsub >= 0 ? wsub : max(bstart, (long long)lo);
               const long long s1 = min(bend, bstart + ((s0 - bstart) / sub + 1) * sub);
               c0 = (int)s0;
               c1 = (int)s1;
@@ -130,7 +129,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_heavy_num_win(HeavyArgs h) {
                 tot += cnt[e];
                 ++e;
               }
-              c0 = (int)max(bstart, (long long)lo_r);
+              c0 = (int)max(bstart, (long long)lo);
               c1 = (int)min((long long)lo_blk + ((long long)e << bw_log2), (long long)hi + 1);
               wb = e;
             }

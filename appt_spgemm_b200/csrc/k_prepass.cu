@@ -54,15 +54,14 @@ cudaError_t launch_validate(const MatView& A, uint32_t* status, cudaStream_t s) 
 // Every index is checked before it is used, so the kernel may run before the
 // host has seen the validation verdict: a row that meets a row pointer or
 // column outside its range gets f = −1, and the later kernels of the
-// one-readback plan skip it.  With `status` set it is also the validation of
-// A (k_validate's checks, in the same read of A's rows): a violation sets
-// DEV_ERR_INVALID_CSR there.
+// one-readback plan skip it.  It is also the validation of A (k_validate's checks,
+// in the same read of A's rows): a violation sets DEV_ERR_INVALID_CSR in `status`.
 __global__ void k_prepass(MatView A, MatView B, int64_t* __restrict__ f, int32_t* __restrict__ lo,
                           int32_t* __restrict__ hi, uint32_t* status, int64_t fcap) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  if (status && warp == 0 && lane == 0 &&
+  if (warp == 0 && lane == 0 &&
       (A.rowptr[0] != 0 || (int64_t)A.rowptr[A.n] != A.nnz))
     report(status, DEV_ERR_INVALID_CSR);
   for (int64_t i = warp; i < A.n; i += nwarps) {
@@ -81,7 +80,7 @@ __global__ void k_prepass(MatView A, MatView B, int64_t* __restrict__ f, int32_t
         const Pos p = p0 + 32 * u;
         const bool in = p < (Pos)e;
         k[u] = in ? A.col[p] : 0;
-        if (in && status && p > (Pos)s && A.col[p - 1] >= k[u]) unsorted = true;
+        if (in && p > (Pos)s && A.col[p - 1] >= k[u]) unsorted = true;
         const bool ok = in && k[u] >= 0 && k[u] < B.n;
         bad = bad || (in && !ok);
         bs[u] = ok ? 0 : -1;
@@ -112,8 +111,8 @@ __global__ void k_prepass(MatView A, MatView B, int64_t* __restrict__ f, int32_t
     }
     bad = __any_sync(0xffffffffu, bad);
     unsorted = __any_sync(0xffffffffu, unsorted);
-    if (status && lane == 0 && (bad || unsorted)) report(status, DEV_ERR_INVALID_CSR);
-    if (status && lane == 0 && !bad && prod > fcap) report(status, DEV_ERR_SMALL_CAP);
+    if (lane == 0 && (bad || unsorted)) report(status, DEV_ERR_INVALID_CSR);
+    if (lane == 0 && !bad && prod > fcap) report(status, DEV_ERR_SMALL_CAP);
     if (lane == 0) {
       f[i] = bad ? -1 : prod;
       lo[i] = bad ? INT_MAX : mn;
@@ -124,11 +123,8 @@ __global__ void k_prepass(MatView A, MatView B, int64_t* __restrict__ f, int32_t
 
 cudaError_t launch_prepass(const MatView& A, const MatView& B, int64_t* f, int32_t* lo,
                            int32_t* hi, cudaStream_t s, uint32_t* status, int64_t fcap) {
-  if (A.n == 0) {
-    if (!status) return cudaSuccess;
-    // no rows: the validation is rowptr[0] == 0 and nnz == 0 alone
-    return launch_validate(A, status, s);
-  }
+  // no rows: the validation is rowptr[0] == 0 and nnz == 0 alone
+  if (A.n == 0) return launch_validate(A, status, s);
   const int threads = 256;
   int64_t blocks = ((int64_t)A.n * 32 + threads - 1) / threads;
   if (blocks > 148 * 64) blocks = 148 * 64;

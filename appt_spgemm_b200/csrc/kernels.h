@@ -33,12 +33,11 @@ cudaError_t launch_validate(const MatView& A, uint32_t* status, cudaStream_t s);
 
 // Per row i of C = A·B: products f_i = Σ_{k∈A_i} nnz(B_k) and the column span
 // [lo_i, hi_i] of the output row (B rows sorted).  Rows with f_i = 0 get
-// lo = INT_MAX, hi = -1; rows that meet an index out of range f_i = −1.  With
-// `status`, A is validated in the same pass (launch_validate's checks), and a row
-// of more than fcap products reports DEV_ERR_SMALL_CAP.
+// lo = INT_MAX, hi = -1; rows that meet an index out of range f_i = −1.  A is
+// validated in the same pass (launch_validate's checks), and a row of more than
+// fcap products reports DEV_ERR_SMALL_CAP.
 cudaError_t launch_prepass(const MatView& A, const MatView& B, int64_t* f, int32_t* lo,
-                           int32_t* hi, cudaStream_t s, uint32_t* status = nullptr,
-                           int64_t fcap = INT64_MAX);
+                           int32_t* hi, cudaStream_t s, uint32_t* status, int64_t fcap);
 
 // Sorted rows: the fewest and the most products, the most products per two entries.
 // Measured per call, Erdős–Rényi 262,147 (81 products a row) A·Aᵀ / R-MAT 2^14 A·A:
@@ -165,9 +164,8 @@ __host__ __device__ __forceinline__ int narrow_bin(int64_t f, int32_t len, int64
 
 // Runs: the fewest rows, and the limits of a row (products, columns spanned) and
 // of its operands for 32 rows (doubles), split over the teams of a CTA: two CTAs
-// share an SM's 227 KB.  Runs from 32 rows on only: 96³ stencil 2.04 ms against 1.88
-//, 47³ 617 against 599 µs; from 4 on: no faster (597
-// against 587 µs), so 8.
+// share an SM's 227 KB.  Runs from 32 rows on only: 96³ stencil 2.04 ms against 1.88,
+// 47³ 617 against 599 µs; from 4 on: no faster (597 against 587 µs), so 8.
 constexpr int kRunMinRows = 8;
 constexpr int kRunMaxProducts = 768;
 constexpr int kRunMaxSpan = 1 << 18;

@@ -75,6 +75,11 @@ constexpr int64_t kSortMaxMerge2Large = 6;  // beyond the warp kernels' largest 
 // 5-point grid of 150 x 150 with six unknowns a node 3.39 / 1.05 ms, four 0.65 / 0.48;
 // 27-point grid 34^3 with two 2.97 / 2.49; Erdos-Renyi 3,000 rows of 40 0.26 / 0.34 ms,
 // 1,100 of 28 0.20 / 0.29; none of these rows in panels: R-MAT 2^12 0.65 -> 0.82 ms.
+// Over three panels or more from kPanelMinWideRow products on: from 256 / 400 / 800 /
+// 1600, R-MAT 2^12 0.46 / 0.50 / 0.59 / 0.70 ms and Erdos-Renyi 4,000 rows of 30 0.25 /
+// 0.28 / 0.32 / 0.29, but the rows of a 27-point mesh with its nodes renumbered (24^3)
+// 0.43 / 0.45 / 0.35 / 0.35 and a thin band of 20,000 (half width 1,300) 0.51 / 0.49 /
+// 0.43 / 0.43.
 constexpr int32_t kPanelMinSpan = 600;
 constexpr int64_t kPanelMinProducts = 64;
 constexpr int64_t kPanelManyProducts = 192;
@@ -165,7 +170,9 @@ __host__ __device__ __forceinline__ int narrow_bin(int64_t f, int32_t len, int64
 // Runs: the fewest rows, and the limits of a row (products, columns spanned) and
 // of its operands for 32 rows (doubles), split over the teams of a CTA: two CTAs
 // share an SM's 227 KB.  Runs from 32 rows on only: 96³ stencil 2.04 ms against 1.88,
-// 47³ 617 against 599 µs; from 4 on: no faster (597 against 587 µs), so 8.
+// 47³ 617 against 599 µs; from 4 on: no faster (597 against 587 µs), so 8.  Rows of
+// more products were not tried; the lists of 1,024 are the most that leave room for
+// the second CTA.
 constexpr int kRunMinRows = 8;
 constexpr int kRunMaxProducts = 768;
 constexpr int kRunMaxSpan = 1 << 18;

@@ -75,18 +75,23 @@ constexpr int64_t kSortMaxMerge2Large = 6;  // beyond the warp kernels' largest 
 // 5-point grid of 150 x 150 with six unknowns a node 3.39 / 1.05 ms, four 0.65 / 0.48;
 // 27-point grid 34^3 with two 2.97 / 2.49; Erdos-Renyi 3,000 rows of 40 0.26 / 0.34 ms,
 // 1,100 of 28 0.20 / 0.29; none of these rows in panels: R-MAT 2^12 0.65 -> 0.82 ms.
-// Over three panels or more from kPanelMinWideRow products on: from 256 / 400 / 800 /
+// Over three panels or more from kPanelMinMidRow products on: from 256 / 400 / 800 /
 // 1600, R-MAT 2^12 0.46 / 0.50 / 0.59 / 0.70 ms and Erdos-Renyi 4,000 rows of 30 0.25 /
 // 0.28 / 0.32 / 0.29, but the rows of a 27-point mesh with its nodes renumbered (24^3)
 // 0.43 / 0.45 / 0.35 / 0.35 and a thin band of 20,000 (half width 1,300) 0.51 / 0.49 /
-// 0.43 / 0.43.
+// 0.43 / 0.43.  With short rows of B also over one or two panels (a CTA per row in the
+// symbolic phase): 40 such meshes of 16^3 in a batch 2.29 -> 1.18 ms, 50 Erdos-Renyi
+// matrices of 1,500 rows of 25 1.37 -> 1.19; but not where the matrix has too few rows
+// to fill the GPU and launches count: R-MAT 2^11 0.40 -> 0.51 ms, Erdos-Renyi 1,100
+// rows of 28 0.22 -> 0.27.
 constexpr int32_t kPanelMinSpan = 600;
 constexpr int64_t kPanelMinProducts = 64;
 constexpr int64_t kPanelManyProducts = 192;
 constexpr int64_t kPanelMinSlice = 2;
 constexpr int64_t kPanelFewPanels = 64;
 constexpr int64_t kPanelMinRow = 256;
-constexpr int64_t kPanelMinWideRow = 800;  // over three panels or more
+constexpr int64_t kPanelMinMidRow = 800;
+constexpr int32_t kPanelFewRows = 8192;
 constexpr int64_t kPanelMinSliceSmall = 5;
 constexpr int64_t kPanelMinMean = 64;
 constexpr int64_t kPanelMinEntries = 48;
@@ -248,11 +253,12 @@ __host__ __device__ __forceinline__ bool clumped_columns(const int32_t* cols, in
 }
 
 // A row of f products from `len` entries of A (their columns: cols) over columns
-// [lo, hi]: cut into panels?  `entries`: its entries, -1 while they are not known
+// [lo, hi] of a matrix of n rows: cut into panels?  `entries`: its entries, -1 while they are not known
 // (symbolic phase: a row that is heavy there for its panels may be hashed in the
 // numeric phase, but not the reverse, for want of its column counts).
 __host__ __device__ __forceinline__ bool paneled_row(int64_t f, int32_t len, const int32_t* cols,
-                                                     int32_t lo, int32_t hi, int64_t entries) {
+                                                     int32_t lo, int32_t hi, int64_t entries,
+                                                     int32_t n) {
   if (f < kPanelMinRow || hi - lo < kPanelMinSpan) return false;
   const int64_t panels = (hi >> 10) - (lo >> 10) + 1;
   if (f < kPanelMinProducts * panels) return false;
@@ -260,8 +266,10 @@ __host__ __device__ __forceinline__ bool paneled_row(int64_t f, int32_t len, con
     return f >= kPanelManyProducts * panels ||
            (f >= kPanelMinSlice * panels * len &&
             (panels <= kPanelFewPanels || 2 * (int64_t)len >= panels));
-  if (f < kPanelMinSliceSmall * panels * len || (panels > 2 && f < kPanelMinWideRow)) return false;
-  if (f >= kPanelMinMean * len) return true;
+  const bool long_b = f >= kPanelMinMean * len;
+  if (f < kPanelMinSliceSmall * panels * len) return false;
+  if (f < kPanelMinMidRow && (panels > 2 || (!long_b && n > kPanelFewRows))) return false;
+  if (long_b) return true;
   if (entries >= 0 && entries < kPanelMinEntries * panels) return false;
   return !clumped_columns(cols, len);
 }
@@ -292,7 +300,7 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
   if (s.mode == 1 && s.lead && s.runlen[i])
     return kRunBin0 + run_team(size, s.need[i], s.f[i], (int64_t)s.hi[i] - s.lo[i] + 1);
   if (s.panels && paneled_row(s.f[i], s.arowptr[i + 1] - s.arowptr[i], s.acol + s.arowptr[i],
-                              s.lo[i], s.hi[i], s.mode == 1 ? size : -1))
+                              s.lo[i], s.hi[i], s.mode == 1 ? size : -1, s.n))
     return s.mode == 1 ? kPanelBin0 : kHeavyBin;
   if (s.force_heavy) return kHeavyBin;
   int lg = table_log2(size, s.load_pct);

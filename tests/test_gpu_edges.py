@@ -197,6 +197,18 @@ def long_b_rows(n, rows, entries, length):
     return from_rows(n, lists, 3)
 
 
+def renumbered(A, window, seed):
+    """A's nodes shuffled within windows of the order: an unstructured mesh's rows."""
+    rng = np.random.default_rng(seed)
+    q = np.lexsort((rng.random(A.n), np.arange(A.n) // window))
+    to = np.empty(A.n, dtype=np.int64)
+    to[q] = np.arange(A.n)
+    rows = [None] * A.n
+    for i in range(A.n):
+        rows[to[i]] = to[A.col[A.rowptr[i]:A.rowptr[i + 1]]]
+    return from_rows(A.n, rows, seed)
+
+
 def arrowhead(n, width):
     rows = [np.concatenate([[0], np.arange(max(0, i - width), min(n, i + width + 1))])
             for i in range(n)]
@@ -216,9 +228,11 @@ def arrowhead(n, width):
     (lambda: long_b_rows(200000, 500, 32, 500), False, None),
     (lambda: long_b_rows(200000, 500, 64, 800), True, None),
     (lambda: long_b_rows(50000, 500, 64, 100), True, None),
+    (lambda: renumbered(csr.stencil27(24, 1), 64, 2), False, None),
+    (lambda: csr.erdos_renyi(1100, 28.0, 1), True, None),
     (lambda: arrowhead(6000, 3), True, False)],
     ids=["grid6", "grid8", "cube2", "cube3", "random", "few-products", "many-products",
-         "many-entries", "arrowhead"])
+         "many-entries", "mesh", "random-small", "arrowhead"])
 def test_rows_worth_a_panel(A, panels, windows):
     from appt_spgemm_b200.engine import Engine
     A = A()
@@ -480,3 +494,18 @@ def test_hopeless_small_plans_are_not_tried(degree, tried):
             assert ("sym/small" in ran) == tried, ran
             e.check_device_status()
             assert_same_csr(got[0].to_host(), oracle.multiply(A, task), task)
+
+
+def test_meshes_of_a_batch_keep_their_tables():
+    # rows of one or two panels: in a batch there are enough of them to fill the GPU, and
+    # tables serve a renumbered mesh's rows better
+    from appt_spgemm_b200.engine import Engine
+    As = [renumbered(csr.stencil27(16, 1), 64, i) for i in range(4)]
+    with Engine("cuda:0") as e:
+        got = []
+        ran = kernels(e, lambda: got.append(e.multiply_batched([dev(A) for A in As], "AA")))
+        assert "sym/heavy" not in ran and "num/panels" not in ran, ran
+        for b, A in enumerate(As):
+            rp, col, val = got[0].instance(b)
+            assert_same_csr((rp.cpu().numpy(), col.cpu().numpy(), val.cpu().numpy()),
+                            oracle.multiply(A, "AA"), f"instance {b}")

@@ -856,7 +856,10 @@ __global__ void __launch_bounds__(256) k_find_runs(
         break;
       }
     }
-    if (tid == first && next - first >= kRunMinRows) list[atomicAdd(&s_count, 1)] = (uint8_t)tid;
+    const int least = first == 0 || next == rows ? kRunMinRows
+                      : G == kShortLanes         ? kRunMinWholeShort
+                                                 : kRunMinWhole;
+    if (tid == first && next - first >= least) list[atomicAdd(&s_count, 1)] = (uint8_t)tid;
   }
   __syncthreads();
   // what 32 rows of each run take, a group of lanes per run

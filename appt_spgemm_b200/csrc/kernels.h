@@ -178,7 +178,15 @@ __host__ __device__ __forceinline__ int narrow_bin(int64_t f, int32_t len, int64
 // 47³ 617 against 599 µs; from 4 on: no faster (597 against 587 µs), so 8.  Rows of
 // more products were not tried; the lists of 1,024 are the most that leave room for
 // the second CTA.
+// A run that is whole (not cut at a block of rows, where its other part reuses what
+// was found for it) has to be longer: its own steps and idle lanes cost more than they
+// save.  Numeric phase of batches of 27-point grids of side 12 / 14 / 16 / 18 / 20 / 24
+// (runs of the side less four), runs against tables: 1086 / 452, 1237 / 665, 1269 /
+// 958, 1595 / 2480, 1417 / 1424, 990 / 1047 µs; 5-point grids (few entries a row) of 12
+// / 16 / 20 / 24 / 30: 201 / 101, 159 / 119, 201 / 170, 200 / 180, 179 / 174.
 constexpr int kRunMinRows = 8;
+constexpr int kRunMinWhole = 14;
+constexpr int kRunMinWholeShort = 24;
 constexpr int kRunMaxProducts = 768;
 constexpr int kRunMaxSpan = 1 << 18;
 constexpr int kRunBuffer = 9216;

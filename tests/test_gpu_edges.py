@@ -509,3 +509,28 @@ def test_meshes_of_a_batch_keep_their_tables():
             rp, col, val = got[0].instance(b)
             assert_same_csr((rp.cpu().numpy(), col.cpu().numpy(), val.cpu().numpy()),
                             oracle.multiply(A, "AA"), f"instance {b}")
+
+
+# whole runs of shifted rows: shorter ones are hashed.  (Grid lines of a power of two
+# lie whole in the blocks of 256 rows that runs are looked for in; of a line that a
+# block cuts, parts of 8 rows are runs too.)
+@pytest.mark.parametrize("grid,count,taken", [
+    (lambda i: csr.stencil27(16, i), 8, False), (lambda i: csr.stencil27(32, i), 2, True),
+    (lambda i: csr.laplace2d(16), 90, False), (lambda i: csr.laplace2d(32), 30, True),
+    (lambda i: csr.laplace2d(27), 30, True)],
+    ids=["12", "28", "12-short", "28-short", "cut"])
+def test_whole_runs_worth_their_setup(grid, count, taken):
+    from appt_spgemm_b200.engine import Engine
+    As = [grid(i) for i in range(count)]
+    for i, A in enumerate(As):
+        A.val = np.random.default_rng(i).uniform(-1, 1, A.nnz)
+    with Engine("cuda:0") as e:
+        for task in ("AA", "AAt"):
+            got = []
+            ran = kernels(e, lambda: got.append(e.multiply_batched([dev(A) for A in As], task)))
+            e.check_device_status()
+            for b, A in enumerate(As):
+                rp, col, val = got[0].instance(b)
+                assert_same_csr((rp.cpu().numpy(), col.cpu().numpy(), val.cpu().numpy()),
+                                oracle.multiply(A, task), f"instance {b}")
+            assert any(x.startswith("num/runs") for x in ran) == taken, ran

@@ -116,6 +116,11 @@ constexpr int64_t kNarrowMinMean = 6;
 constexpr int64_t kNarrowHalfMean = 10;
 constexpr int64_t kNarrowFill = 4;
 constexpr int64_t kNarrowMinProducts = 48;
+// Rows of up to kNarrowTinySpan columns have small tables, of which a warp takes
+// several: summed densely only where B's rows fill more than half of the lanes.
+// Numeric phase, dense blocks of 7 / 8 / 10 / 12 / 16 / 20 on the diagonal, narrow
+// against tables: 232 / 162, 266 / 169, 322 / 336, 363 / 332, 335 / 300, 313 / 525 µs.
+constexpr int64_t kNarrowTinySpan = 16;
 constexpr int64_t kNarrowMaxProducts = 1 << 16;
 
 // What a row's bin is computed from.
@@ -162,7 +167,9 @@ struct BinSource {
 // A row of f products from `len` entries of A over `span` columns: summed densely?
 // (The same answer for the symbolic and the numeric binning.)
 __host__ __device__ __forceinline__ bool narrow_row_rule(int64_t f, int32_t len, int64_t span) {
-  return span <= kNarrowMin << (kNarrowBins / 2 - 1) && f >= kNarrowMinMean * len &&
+  const int64_t lanes = f > kNarrowHalfMean * len ? 32 : 16;
+  return (span > kNarrowTinySpan || 2 * f > lanes * len) &&
+         span <= kNarrowMin << (kNarrowBins / 2 - 1) && f >= kNarrowMinMean * len &&
          f * kNarrowFill >= span && f >= kNarrowMinProducts &&
          f <= (span > kPanelMinSpan ? kSortMaxProducts : kNarrowMaxProducts);  // (else panels)
 }

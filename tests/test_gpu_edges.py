@@ -534,3 +534,28 @@ def test_whole_runs_worth_their_setup(grid, count, taken):
                 assert_same_csr((rp.cpu().numpy(), col.cpu().numpy(), val.cpu().numpy()),
                                 oracle.multiply(A, task), f"instance {b}")
             assert any(x.startswith("num/runs") for x in ran) == taken, ran
+
+
+def blocks(n, b):
+    """Dense blocks of b on the diagonal."""
+    k = n // b
+    col = np.repeat(np.arange(k) * b, b * b).reshape(k, b, b) + np.arange(b)
+    return csr.CsrHost(k * b, (np.arange(k * b + 1) * b).astype(np.int32),
+                       col.ravel().astype(np.int32),
+                       np.random.default_rng(b).uniform(-1, 1, col.size))
+
+
+# rows of a few columns: tables unless B's rows fill the lanes that would sum them
+@pytest.mark.parametrize("b,narrow", [(7, False), (8, False), (9, True), (10, True), (11, False),
+                                      (16, False), (17, True), (33, True)])
+def test_narrow_rows_of_few_columns(b, narrow):
+    from appt_spgemm_b200.engine import Engine
+    A = blocks(3000, b)
+    for cfg in (dict(), dict(small_max_nnz=-1)):
+        with Engine("cuda:0", **cfg) as e:
+            for task in ("AA", "AAt"):
+                got = []
+                ran = kernels(e, lambda: got.append(e.multiply(dev(A), task)))
+                assert not cfg or any(x.startswith("num/narrow") for x in ran) == narrow, ran
+                e.check_device_status()
+                assert_same_csr(got[0].to_host(), oracle.multiply(A, task), task)

@@ -554,8 +554,9 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   }
   {
     ProfScope ps(ctx, "plan/scan", st);
-    TRY_CUDA(launch_row_pointers(p->rownnz, nullptr, p->f, p->lo, p->hi, n, p->rowptr, stats,
-                                 ctx->d_status, w + o_scan, st), "row pointer scan");
+    TRY_CUDA(launch_row_pointers(p->A, p->B, p->rownnz, nullptr, p->f, p->lo, p->hi, n,
+                                 p->rowptr, stats, ctx->d_status, w + o_scan, st),
+             "row pointer scan");
   }
   int64_t* hp = ctx->h_pin;
   TRY_CUDA(cudaMemcpyAsync(hp, stats, sizeof(int64_t) * kRowStats, cudaMemcpyDeviceToHost, st),
@@ -596,7 +597,7 @@ spg_status plan_build_small(spg_plan* p, const spg_csr_dev* Ad, bool* fallback) 
   }
   // products that hardly merge: sorted rows, sized from the largest row
   if ((int64_t)sv[0] >= kSortMinProducts * n && sorted_row((int64_t)sv[1], kSortMaxProducts, n) &&
-      2 * (int64_t)sv[0] <= kSortMaxMerge2 * p->nnz_c)
+      2 * (int64_t)sv[0] <= kSortMaxMerge2 * p->nnz_c && !crowded(sv[6]))
     p->small_sort = (int)sv[1];
   if (ctx->cfg.lanes_per_row > 0) {
     p->G = ctx->cfg.lanes_per_row;
@@ -752,7 +753,7 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   BinSource bsym{0, n, p->f, p->lo, p->hi, nullptr, kMaxTableLog2, force,
                  ctx->cfg.sym_load_pct,
                  numeric_heavy_min(num_lg, ctx->cfg.num_load_pct),
-                 p->A.rowptr, p->A.col, split, short_lg,
+                 p->A.rowptr, p->A.col, nullptr, split, short_lg,
                  numeric_heavy_min(short_lg, ctx->cfg.num_load_pct), dense_lw, 0, panels,
                  pre.lead, pre.runlen, pre.need};
   // column blocks of the heavy rows: 1024 columns (windows are packed from
@@ -905,14 +906,15 @@ spg_status plan_build(spg_plan* p, const spg_csr_dev* Ad) {
   TRY(palloc(p, &p->rowptr, (int64_t)n + 1));
   {
     ProfScope ps(ctx, "plan/scan", st);
-    TRY_CUDA(launch_row_pointers(p->rownnz, pre.lead, p->f, p->lo, p->hi, n, p->rowptr, stats,
-                                 ctx->d_status, scan_tmp, st), "row pointer scan");
+    TRY_CUDA(launch_row_pointers(p->A, p->B, p->rownnz, pre.lead, p->f, p->lo, p->hi, n,
+                                 p->rowptr, stats, ctx->d_status, scan_tmp, st),
+             "row pointer scan");
   }
   // numeric binning by exact counts, stats; host sync #2 (nnz(C))
   TRY(palloc(p, &p->rows_num, n));
   BinSource bnum{1, n, p->f, p->lo, p->hi, p->rownnz, num_lg, force,
-                 ctx->cfg.num_load_pct, 0, p->A.rowptr, p->A.col, split, short_lg, 0, dense_lw,
-                 1, panels && p->pan_log2 > 0 && p->blk_cnt, pre.lead, pre.runlen, pre.need};
+                 ctx->cfg.num_load_pct, 0, p->A.rowptr, p->A.col, stats + 6, split, short_lg, 0,
+                 dense_lw, 1, panels && p->pan_log2 > 0 && p->blk_cnt, pre.lead, pre.runlen, pre.need};
   {
     ProfScope ps(ctx, "plan/bin_num", st);
     TRY_CUDA(launch_bin_rows(bnum, bin, work_num, p->rows_num, st),

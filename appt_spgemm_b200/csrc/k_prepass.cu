@@ -356,10 +356,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_single(const int32_t* __r
 // gathers the statistics; in the second each tile sums the tiles before it.
 // (A scan of three launches, the run counts and the statistics as launches of
 // their own took 58 against 19 µs on a million rows.)
-//   stats: Σ products, max products, max row count, max span, Σ row counts, and
-//     the two device status words, so that one copy brings a plan's verdict
+//   stats: Σ products, max products, max row count, max span, Σ row counts, the
+//     two device status words, so that one copy brings a plan's verdict, and the
+//     rows looked at for crowding
 struct RowStats {
   unsigned long long sf = 0, mf = 0, mc = 0, ms = 0;
+  unsigned long long crowd = 0;  // rows looked at, and 2^32 times those found crowded
   __device__ __forceinline__ void add(unsigned long long f, int c, int lo, int hi) {
     sf += f;
     mf = f > mf ? f : mf;
@@ -369,9 +371,10 @@ struct RowStats {
   }
   // per warp, then one atomic each per CTA (of one CTA: plain stores)
   __device__ __forceinline__ void store(unsigned long long* stats, bool single) {
-    __shared__ unsigned long long acc[4];
-    if (threadIdx.x < 4) acc[threadIdx.x] = 0;
+    __shared__ unsigned long long acc[5];
+    if (threadIdx.x < 5) acc[threadIdx.x] = 0;
     __syncthreads();
+    if (crowd) atomicAdd(&acc[4], crowd);
     for (int o = 16; o > 0; o >>= 1) {
       sf += __shfl_xor_sync(0xffffffffu, sf, o);
       const unsigned long long a = __shfl_xor_sync(0xffffffffu, mf, o);
@@ -390,7 +393,9 @@ struct RowStats {
     __syncthreads();
     if (single) {
       if (threadIdx.x < 4) stats[threadIdx.x] = acc[threadIdx.x];
+      if (threadIdx.x == 4) stats[6] = acc[4];
     } else if (threadIdx.x == 0) {
+      if (acc[4]) atomicAdd(&stats[6], acc[4]);
       atomicAdd(&stats[0], acc[0]);
       atomicMax(&stats[1], acc[1]);
       atomicMax(&stats[2], acc[2]);
@@ -399,9 +404,30 @@ struct RowStats {
   }
 };
 
+// A sorted row looked at: 1, and 2^32 more when six of eight of its
+// columns lie within 2^-kCrowdLog2 of its span.  (Up to kCrowdMin products fit a bucket.)
+__device__ __noinline__ unsigned long long crowd_look(const MatView& A, const MatView& B,
+                                                      int64_t i, int64_t f, int cnt, int32_t lo,
+                                                      int32_t hi) {
+  if (f <= kCrowdMin || f > kSortMaxProducts || 2 * f > kSortMaxMerge2 * cnt) return 0;
+  const int32_t ps = A.rowptr[i], len = A.rowptr[i + 1] - ps, window = (hi - lo) >> kCrowdLog2;
+  int32_t c[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) c[u] = crowd_column(A.col + ps, len, B.rowptr, B.col, u);
+  int most = 0;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    int near = 0;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) near += c[v] >= c[u] && c[v] - c[u] <= window;
+    most = max(most, c[u] < 0 ? 0 : near);
+  }
+  return most >= 6 ? 1ull << 32 | 1ull : 1ull;
+}
+
 template <bool SINGLE>
 __global__ void __launch_bounds__(kScanThreads) k_count_tiles(
-    int32_t* cnt, const uint8_t* __restrict__ lead, const int64_t* __restrict__ f,
+    MatView A, MatView B, int32_t* cnt, const uint8_t* __restrict__ lead, const int64_t* __restrict__ f,
     const int32_t* __restrict__ lo, const int32_t* __restrict__ hi, int64_t n,
     int64_t* __restrict__ rowptr, long long* __restrict__ tile_sums,
     unsigned long long* __restrict__ stats, const uint32_t* __restrict__ status) {
@@ -463,6 +489,10 @@ __global__ void __launch_bounds__(kScanThreads) k_count_tiles(
       if (d) cnt[i] = c;
       s += c;
       st.add((unsigned long long)f[i], c, lo[i], hi[i]);
+      // (eight threads of the tile look at one row each, so that it costs them one chain
+      // of loads; a single tile's rows are not looked at)
+      if ((threadIdx.x & 63) == 32 && (threadIdx.x >> 6) == k)
+        st.crowd = crowd_look(A, B, i, f[i], c, lo[i], hi[i]);
     }
     s = block_sum64(s, scratch);
     if (threadIdx.x == 0) tile_sums[blockIdx.x] = s;
@@ -506,14 +536,15 @@ __global__ void __launch_bounds__(kScanThreads) k_count_apply(const int32_t* __r
 // the three-launch scan)
 constexpr int64_t kMaxCountTiles = 4096;
 
-cudaError_t launch_row_pointers(int32_t* cnt, const uint8_t* lead, const int64_t* f,
+cudaError_t launch_row_pointers(const MatView& A, const MatView& B, int32_t* cnt,
+                                const uint8_t* lead, const int64_t* f,
                                 const int32_t* lo, const int32_t* hi, int64_t n, int64_t* rowptr,
                                 unsigned long long* stats, const uint32_t* status, void* tmp,
                                 cudaStream_t s) {
   long long* tiles = (long long*)tmp;
   const int64_t ntiles = (n + kScanTile - 1) / kScanTile;
   if (ntiles == 1) {
-    k_count_tiles<true><<<1, kScanThreads, 0, s>>>(cnt, lead, f, lo, hi, n, rowptr, tiles, stats,
+    k_count_tiles<true><<<1, kScanThreads, 0, s>>>(A, B, cnt, lead, f, lo, hi, n, rowptr, tiles, stats,
                                                    status);
     SPG_COUNT_LAUNCH();
     return cudaGetLastError();
@@ -524,7 +555,7 @@ cudaError_t launch_row_pointers(int32_t* cnt, const uint8_t* lead, const int64_t
     e = cudaMemcpyAsync(stats + 5, status, 2 * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
     return e != cudaSuccess ? e : cudaMemsetAsync(rowptr, 0, sizeof(int64_t), s);
   }
-  k_count_tiles<false><<<(unsigned)ntiles, kScanThreads, 0, s>>>(cnt, lead, f, lo, hi, n, rowptr,
+  k_count_tiles<false><<<(unsigned)ntiles, kScanThreads, 0, s>>>(A, B, cnt, lead, f, lo, hi, n, rowptr,
                                                                  tiles, stats, status);
   SPG_COUNT_LAUNCH();
   if ((e = cudaGetLastError()) != cudaSuccess) return e;

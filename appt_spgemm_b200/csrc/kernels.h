@@ -144,6 +144,7 @@ struct BinSource {
   // serves them better than the CTA-per-row tables, whose per-k barrier idles
   // most of the CTA on short B rows
   const int32_t *arowptr, *acol;
+  const unsigned long long* crowd;  // rows looked at, and 2^32 times those found crowded
   int64_t short_split;
   int short_max_log2;
   int64_t short_min;
@@ -255,6 +256,29 @@ __host__ __device__ __forceinline__ int heavy_class(int64_t f) {
   return c;
 }
 
+// Sorted rows most of whose columns crowd into a small part of their span (a community
+// of a graph, with a few links to elsewhere) fill single buckets, and the radix sort
+// that takes over is slower than the tables: communities of 400 among 200,000 columns
+// 1.71 against 1.48 ms, of 1,000 among 100,000 2.15 against 1.81, of 100 among 60,000
+// 194 against 124 µs; with communities of 2,000 among 100,000 sorting is still faster
+// (4.4 against 5.8 ms).  One row in 512 is looked at (k_count_tiles; with 64 of them the
+// plan of Erdos-Renyi 40,009 took 15 µs more), and where most of those have six of eight
+// columns within 2^-kCrowdLog2 of the span none of the matrix's rows are sorted.
+constexpr int kCrowdLog2 = 7;
+constexpr int kCrowdMin = 48;
+__host__ __device__ __forceinline__ bool crowded(unsigned long long crowd) {
+  return 2 * (crowd >> 32) > (crowd & 0xffffffffull);
+}
+// Column t of eight that are spread over a row's products: from the B row of an entry
+// at t / 8 of A's row, the entry at t / 8 of it (-1: none).
+__device__ __forceinline__ int32_t crowd_column(const int32_t* cols, int32_t len,
+                                                const int32_t* browptr, const int32_t* bcol,
+                                                int t) {
+  const int32_t k = cols[(int64_t)len * (2 * t + 1) >> 4];
+  const int32_t bs = browptr[k], m = browptr[k + 1] - bs;
+  return m > 0 ? bcol[bs + ((int64_t)m * (2 * t + 1) >> 4)] : -1;
+}
+
 // Are the row's columns (len of them, sorted) mostly runs of neighbours?  By eight
 // of its entries.  Neighbouring rows of B then hold much the same columns: the
 // unknowns of a mesh's node, or the neighbours of a grid point.
@@ -319,7 +343,7 @@ __host__ __device__ __forceinline__ int row_bin(const BinSource& s, int i) {
     return s.mode == 1 ? kPanelBin0 : kHeavyBin;
   if (s.force_heavy) return kHeavyBin;
   int lg = table_log2(size, s.load_pct);
-  if (s.mode == 1 && s.sort_rows && lg <= s.max_log2 &&
+  if (s.mode == 1 && s.sort_rows && lg <= s.max_log2 && !crowded(*s.crowd) &&
       sorted_row(s.f[i], size, (int64_t)s.hi[i] - s.lo[i] + 1,
                  lg > s.short_max_log2 ? kSortMaxMerge2Large : kSortMaxMerge2)) {
     int b = 0;
@@ -671,10 +695,11 @@ cudaError_t launch_describe(const MatView& A, const int32_t* colcount, DescAccum
 // Row pointers of C from the row counts (with `lead`, a run's rows take its
 // first row's count first), and kRowStats statistics: Σ products, max products,
 // max row count, max column span, nnz(C), and the device status words as they are
-// then.  cnt, f, lo, hi: 16-byte aligned.  tmp: scan_tmp_bytes(n).
-constexpr int kRowStats = 6;
-cudaError_t launch_row_pointers(int32_t* cnt, const uint8_t* lead, const int64_t* f,
-                                const int32_t* lo, const int32_t* hi, int64_t n, int64_t* rowptr,
+// then, and the rows looked at for crowding with 2^32 times those found so.  cnt, f, lo, hi: 16-byte aligned.  tmp: scan_tmp_bytes(n).
+constexpr int kRowStats = 7;
+cudaError_t launch_row_pointers(const MatView& A, const MatView& B, int32_t* cnt,
+                                const uint8_t* lead, const int64_t* f, const int32_t* lo,
+                                const int32_t* hi, int64_t n, int64_t* rowptr,
                                 unsigned long long* stats, const uint32_t* status, void* tmp,
                                 cudaStream_t s);
 cudaError_t launch_col_count(const MatView& A, int32_t* cnt, cudaStream_t s);

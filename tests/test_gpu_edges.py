@@ -559,3 +559,31 @@ def test_narrow_rows_of_few_columns(b, narrow):
                 assert not cfg or any(x.startswith("num/narrow") for x in ran) == narrow, ran
                 e.check_device_status()
                 assert_same_csr(got[0].to_host(), oracle.multiply(A, task), task)
+
+
+def communities(n, size, inside, seed):
+    """Rows of `inside` columns of their own community and one of anywhere."""
+    rng = np.random.default_rng(seed)
+    return from_rows(n, [np.concatenate([i // size * size + rng.integers(0, size, inside),
+                                         rng.integers(0, n, 1)]) for i in range(n)], seed)
+
+
+# sorted rows are hashed where their columns crowd together: communities of a hundredth of
+# the columns and less, one readback or two; not those of a tenth, nor a random graph
+@pytest.mark.parametrize("A,crowded", [
+    (lambda: communities(40000, 200, 12, 1), True), (lambda: communities(40000, 400, 20, 2), True),
+    (lambda: communities(40000, 4000, 20, 3), False),
+    (lambda: csr.erdos_renyi(40000, 16.0, 4), False)],
+    ids=["200", "400", "4000", "random"])
+def test_crowded_rows_are_not_sorted(A, crowded):
+    from appt_spgemm_b200.engine import Engine
+    A = A()
+    for cfg in (dict(small_max_nnz=-1), dict()):
+        with Engine("cuda:0", **cfg) as e:
+            for task in ("AA", "AAt", "AAtS"):
+                got = []
+                ran = kernels(e, lambda: got.append(e.multiply(dev(A), task)))
+                if cfg:
+                    assert any(x.startswith("num/sort") for x in ran) != crowded, (task, ran)
+                e.check_device_status()
+                assert_same_csr(got[0].to_host(), oracle.multiply(A, task), task)
